@@ -22,6 +22,8 @@ struct StepConsts {
     // diagnostics summed by synchronous FP64 launches: cell volume, core
     // radius^2 of Q_core, plaquette-energy prefactor 1/(g^2 dx^4)
     double dV, R2, bpre;
+    // products the gauged site function uses: eta/(2dx), eta dx/2, g/dx
+    double ei, cross, gi;
 };
 
 // Work decomposition of the persistent step kernels: the grid is cut into
@@ -29,6 +31,7 @@ struct StepConsts {
 struct TileGrid {
     int ntx, nty, nseg, seg;
     int nitems;
+    int tw, th;   // sites of a tile along k and j
 };
 
 // A run of planes [i0, i1) of column (kt, jt).

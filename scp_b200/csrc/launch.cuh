@@ -25,6 +25,8 @@ constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 
 // one-site kernels: g gauged, f first step, s synchronous momenta, d damping
 StepFnT<F64> step_fn_f64(int shape, bool g, bool f, bool s, bool d, size_t *smem);
+// FP64 synchronous launch that also sums the first diagnostics pass
+StepFnT<F64> step_diag_fn(int shape, bool g, bool d, size_t *smem);
 StepFnT<F32C> step_fn_f32c(int shape, bool g, bool f, bool s, bool d, size_t *smem);
 // multi-request kernels: g gauged, d damping
 MultiFn<F64> multi_fn_f64(int shape, bool g, bool d, size_t *smem);

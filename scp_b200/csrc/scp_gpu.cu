@@ -171,10 +171,12 @@ struct scp_gpu {
     int shape;
     int pairs = 0;               // 1: two-site packed FP32C kernel
     int threads = 0;
-    TileGrid tg;                 // item plan (the server's tables)
+    TileGrid tg{};               // item plan (the server's tables)
     int grid;
-    TileGrid tg_run;             // plan of the single-grid launches (balanced when large enough)
+    TileGrid tg_run{};           // plan of the single-grid launches
     int grid_run = 0;
+    TileGrid tg_diag{};          // plan of the synchronous launch that sums the diagnostics
+    int grid_diag = 0;
     int64_t steps = 0;
     double G_offset = 0.0;
     int cg_iters = 0;
@@ -236,48 +238,64 @@ static void fill_consts(scp_gpu *h) {
     c.dV = p.dx * p.dx * p.dx;
     c.R2 = p.qdiag_radius * p.qdiag_radius;
     c.bpre = gauged ? 1.0 / (p.g_gauge * p.g_gauge * p.dx * p.dx * p.dx * p.dx) : 0.0;
+    c.ei = c.eta * c.idx1;
+    c.cross = 0.5 * c.eta * c.dx;
+    c.gi = c.g * c.inva;
 }
 
 static bool damping_on(const scp_gpu *h) {
     return h->p.bc_type == 0 && h->p.damp_width > 0 && h->p.damp_rate > 0;
 }
 
-// Choose the i-segment length that minimises (waves x planes per item),
-// planes per item counting the two halo planes a segment re-reads.
-static void plan_tiles(scp_gpu *h, int tx, int ty, int slots) {
-    const int N = h->N;
+// Cut a grid of edge N into tiles of tw x th sites and segments along i, for
+// `slots` resident CTAs: the segment length minimises (waves x planes per
+// item), planes per item counting the two halo planes a segment re-reads.
+// All CTAs start their items on the same plane and walk i in step, so
+// neighbouring columns read each other's halo rows while they are in L2.
+// (Equal shares of all (column, plane) pairs, which leave no slot idle, were
+// measured slower: neighbours drift apart in i and the halo rows come from
+// DRAM again, 837 against 470 MB read per 128^3 step.)
+static void plan_tiles(int N, int tw, int th, int slots, TileGrid *out, int *grid) {
     TileGrid tg;
-    tg.ntx = (N + tx - 1) / tx;
-    tg.nty = (N + ty - 1) / ty;
+    tg.tw = tw;
+    tg.th = th;
+    tg.ntx = (N + tw - 1) / tw;
+    tg.nty = (N + th - 1) / th;
     const int ntiles = tg.ntx * tg.nty;
-
     double best = 1e300;
-    int best_seg = N;
-    const int cands[] = {4, 6, 8, 10, 12, 16, 20, 24, 32, 48, 64, 96, 128, 192, 256, 384, 512, 1024, 2048};
-    for (int s : cands) {
-        if (s > N) break;
-        const long long items = (long long)ntiles * ((N + s - 1) / s);
-        const long long waves = (items + slots - 1) / slots;
-        const double cost = (double)waves * (s + 2);
-        if (cost < best - 1e-9 || (cost < best + 1e-9 && s > best_seg)) { best = cost; best_seg = s; }
+    int best_nseg = 1;
+    for (int ns = 1; ns <= N; ns++) {
+        const int seg = (N + ns - 1) / ns;
+        if (ns > 1 && (N + seg - 1) / seg != ns) continue;   // the same cut as a smaller ns
+        const long long waves = ((long long)ntiles * ns + slots - 1) / slots;
+        const double cost = (double)waves * (seg + 2);
+        if (cost < best - 1e-9) { best = cost; best_nseg = ns; }
     }
-    {   // whole column as one segment
-        const long long waves = (ntiles + slots - 1) / slots;
-        const double cost = (double)waves * (N + 2);
-        if (cost < best - 1e-9) { best = cost; best_seg = N; }
-    }
-    tg.seg = best_seg;
-    tg.nseg = (N + best_seg - 1) / best_seg;
+    tg.seg = (N + best_nseg - 1) / best_nseg;
+    tg.nseg = (N + tg.seg - 1) / tg.seg;
     tg.nitems = ntiles * tg.nseg;
-    h->tg = tg;
-    h->grid = tg.nitems < slots ? tg.nitems : slots;
-    // All CTAs start their items on the same plane and walk i in step, so
-    // neighbouring columns read each other's halo rows while they are in L2.
-    // (Equal shares of all (column, plane) pairs, which leave no slot idle,
-    // were measured slower: neighbours drift apart in i and the halo rows come
-    // from DRAM again, 837 against 470 MB read per 128^3 step.)
-    h->tg_run = tg;
-    h->grid_run = h->grid;
+    *out = tg;
+    *grid = tg.nitems < slots ? tg.nitems : slots;
+}
+
+// Tile of the one-site cp.async kernels for a grid of edge N: up to nt sites
+// whose staged rows (halo included) fit `area` ring elements, least
+// (padded sites) x (cost of the width).  Rows of 32 sites move whole 128-byte
+// lines: width 32 costs 1.  Gauged FP64 measured against it: 16-site rows
+// 192 against 184 us at 128^3 (counted 1.08), rows that start inside a line
+// 362 against 320 us at 150^3 with 7 % fewer padded sites (1.22; 1.12 where an
+// odd N leaves every row unaligned anyway).  So 32-site rows stay except where
+// they pad: 16 x 16 takes 54 us at 80^3 against 62, 25 x 10 takes 107 us at
+// 97^3 (whose fourth column of 32-site tiles holds one site) against 123.
+static void fit_tile(int N, int nt, int area, int *tw, int *th) {
+    double best = 1e300;
+    for (int w = 32; w >= 16; w--) {
+        int h = nt / w;
+        while (h > 1 && (w + 2) * (h + 2) > area) h--;
+        const double pad = (double)((N + w - 1) / w) * w * ((N + h - 1) / h) * h;
+        const double cost = pad * (w == 32 ? 1.0 : w == 16 ? 1.08 : (N & 1) ? 1.12 : 1.22);
+        if (cost < best - 1e-9) { best = cost; *tw = w; *th = h; }
+    }
 }
 
 template <class P>
@@ -420,14 +438,22 @@ static int setup_launch(scp_gpu *h) {
     const bool pairs = h->prec == SCP_PREC_FP32C && h->N % 2 == 0;
     int shape = h->p.tile_variant;
     if (shape == 0) shape = pairs ? 2 : 1;
-    h->shape = shape;
     h->pairs = pairs ? 1 : 0;
+    h->tma = staging_mode(h, shape);
+    // the gauged FP64 ring runs 256-site tiles (one CTA per SM) from 80^3: a
+    // tile of 32 x 8 stages 1.33 sites per site against 1.59 of 32 x 4 (two
+    // CTAs per SM), 184 against 200 us at 128^3 and 1.41 against 1.49 ms at
+    // 256^3; smaller grids have too few tiles for it (28.7 against 27.9 us at
+    // 64^3), and the ungauged ring is faster on 32 x 4 (1.12 against 1.20 ms
+    // at 256^3)
+    if (h->p.tile_variant == 0 && !pairs && h->tma == 0 && h->prec == SCP_PREC_FP64 && h->gauged && h->N >= 80)
+        shape = 2;
+    h->shape = shape;
     int nsm = 0;
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
     const TileShape ts = kShapes[shape];
     h->threads = ts.tx * ts.ty / (pairs ? 2 : 1);
     int occ = 0, rc;
-    h->tma = staging_mode(h, shape);
     if (h->tma == 3) {
         h->threads = 2 * ts.tx * ts.ty;
         rc = setup_duo(h, &occ);
@@ -437,7 +463,22 @@ static int setup_launch(scp_gpu *h) {
     else rc = occupancy_of<F32C>(h, shape, &occ);
     if (rc) return rc;
     if (occ < 1) return SCP_EUNSUPPORTED;
-    plan_tiles(h, ts.tx, ts.ty, nsm * occ);
+    int tw = ts.tx, th = ts.ty;
+    if (h->p.tile_variant == 0 && !pairs && h->tma == 0)
+        fit_tile(h->N, ts.tx * ts.ty, (ts.tx + 2) * (ts.ty + 2), &tw, &th);
+    plan_tiles(h->N, tw, th, nsm * occ, &h->tg, &h->grid);
+    h->tg_run = h->tg;
+    h->grid_run = h->grid;
+    if (h->prec == SCP_PREC_FP64 && h->tma == 0) {
+        size_t smem = 0;
+        for (int d = 0; d < 2; d++) {
+            const void *fn = (const void *)step_diag_fn(shape, h->gauged, d, &smem);
+            CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, h->threads, smem));
+        }
+        if (occ < 1) return SCP_EUNSUPPORTED;
+        plan_tiles(h->N, tw, th, nsm * occ, &h->tg_diag, &h->grid_diag);
+    }
     return SCP_OK;
 }
 
@@ -469,6 +510,9 @@ static int launch_step(scp_gpu *h, bool first, bool sync) {
         } else if (h->tma == 3) {
             StepFnT<F64> fn = step_duo_fn(first, sync, damping_on(h), &smem);
             fn<<<h->grid_run, h->threads, smem, h->stream>>>(io, h->c, h->tg_run);
+        } else if (dg) {
+            StepFnT<F64> fn = step_diag_fn(h->shape, h->gauged, damping_on(h), &smem);
+            fn<<<h->grid_diag, ts.tx * ts.ty, smem, h->stream>>>(io, h->c, h->tg_diag);
         } else {
             StepFnT<F64> fn = step_fn<F64>(h->shape, h->gauged, first, sync, damping_on(h), &smem);
             fn<<<h->grid_run, ts.tx * ts.ty, smem, h->stream>>>(io, h->c, h->tg_run);
@@ -728,8 +772,8 @@ static int init_body(scp_gpu *h, const double *const *cols, bool on_device) {
     // SCP_FUSED_DIAG=0 in the environment keeps the separate pass
     const char *fd = getenv("SCP_FUSED_DIAG");
     if (h->prec == SCP_PREC_FP64 && h->tma == 0 && (h->gauged || !h->links) && !(fd && fd[0] == '0')) {
-        CK(cudaMallocAsync(&h->dpart, sizeof(double) * kDiag1Q * (size_t)h->grid_run, h->stream));
-        h->dev_bytes += sizeof(double) * kDiag1Q * (size_t)h->grid_run;
+        CK(cudaMallocAsync(&h->dpart, sizeof(double) * kDiag1Q * (size_t)h->grid_diag, h->stream));
+        h->dev_bytes += sizeof(double) * kDiag1Q * (size_t)h->grid_diag;
         if (h->gauged) {
             CK(cudaMallocAsync(&h->drho, sizeof(double) * n3, h->stream));
             h->dev_bytes += sizeof(double) * n3;
@@ -1376,7 +1420,7 @@ static int diag_with(scp_gpu *h, const View &V, scp_gpu_diag_out *out) {
     const bool fused = std::is_same<View, ViewF64>::value && h->dvalid;
     if constexpr (std::is_same<View, ViewF64>::value) {
         if (fused) {
-            nb1 = h->grid_run;
+            nb1 = h->grid_diag;
             part1 = h->dpart;
         } else {
             const size_t th = (size_t)FTH * h->N3;
@@ -1619,8 +1663,8 @@ int scp_gpu_get_info(const scp_gpu *h, scp_gpu_info *info) {
     // three fabrics: C with the links (30), L (24), Q (24) unless it is C
     if (h->mfab) info->state_bytes_per_site = 8.0 * (30.0 + 24.0 + (h->fab_lock ? 0.0 : 24.0));
     info->step_bytes_per_site = 2.0 * info->state_bytes_per_site;
-    info->tile_x = kShapes[h->shape].tx;
-    info->tile_y = kShapes[h->shape].ty;
+    info->tile_x = h->tg_run.tw > 0 ? h->tg_run.tw : kShapes[h->shape].tx;
+    info->tile_y = h->tg_run.th > 0 ? h->tg_run.th : kShapes[h->shape].ty;
     info->seg_len = h->tg_run.seg;
     info->sites_per_thread = h->pairs ? 2 : 1;
     info->tma_staging = h->tma;

@@ -25,18 +25,30 @@
 // of w and skips the stage-4 kick; a SYNC launch also stores v_{n+1} and
 // E_{n+1} for diagnostics and snapshots.
 //
-// Data movement.  Persistent CTAs walk work items = (TX x TY) columns in
-// (k, j) times segments of `seg` planes in i.  A CTA streams its column plane
-// by plane through a 3-slot shared-memory ring (plane i, plane i+1, and plane
-// i+2 in flight via cp.async), holding the x(i-1) centre values of its own
-// sites in registers.  Every thread copies its own site; the halo rows and
-// columns (periodic wrap) are spread over the CTA's threads so each thread
-// issues the same copies with no per-field branches.  In gauged mode every
+// Data movement.  Persistent CTAs walk work items = tile columns (tw x th
+// sites in k and j, chosen per grid) times segments of `seg` planes in i.  A
+// CTA streams its column plane by plane through a 3-slot shared-memory ring
+// (plane i, plane i+1, and plane i+2 in flight via cp.async).  Every thread
+// copies its own site; the halo rows and columns (periodic wrap) are spread
+// over the CTA's threads so each thread issues the same copies with no
+// per-field branches.  What a site needs of plane i-1 is carried in registers
+// (FP64: the backward transports along i, or x(i-1) without links; F32C:
+// x(i-1)), and so are the momenta, read one plane ahead.  In gauged mode every
 // thread evaluates the link cos/sin and plaquette sines it needs itself: its
 // own site, the j-1 and k-1 neighbours (recomputed from the ring), and the
-// i-1 values carried in registers from the previous plane -- more sines than
-// sharing them through shared memory, but no extra barrier per plane and no
-// shared array, which leaves room for more resident CTAs.
+// i-1 values carried from the previous plane -- more sines than sharing them
+// through shared memory, but no extra barrier per plane.
+//
+// FP64, what bounds it: DRAM.  A gauged step moves 480 B per site (every state
+// word read and written once) and ran at 0.69 of a plain copy's rate while its
+// momenta were loaded at the top of the plane that uses them: with 8 warps an
+// SM, the warps sat on those loads (2 of 5.4 cycles per issue) whatever the
+// arithmetic cost.  Loading them one plane ahead (gauged.cuh frees the
+// registers that takes), and 256-site tiles with their smaller halo, bring it
+// to 0.85 at 128^3 (182 us against 227) and 0.88 at 256^3 (1.41 ms against
+// 1.78).  Three CTAs of 168 registers were slower (278 us at 128^3): the ring
+// of three leaves the L1 too few lines for the copies in flight.  So were
+// 16-byte copies past L1 (206 against 198 us on 32 x 4 tiles).
 #pragma once
 #include <cuda_bf16.h>
 
@@ -44,6 +56,7 @@
 
 #include "common.cuh"
 #include "diag.cuh"
+#include "gauged.cuh"
 #include "trig.cuh"
 
 namespace scp {
@@ -94,6 +107,14 @@ struct StepLayout {
 __device__ __forceinline__ void cp_async_elem(double *s, const double *g) { cp_async8(s, g); }
 __device__ __forceinline__ void cp_async_elem(float *s, const float *g) { cp_async4(s, g); }
 
+// A load that stays where it is written: the compiler does not move it down to
+// its first use, so its latency passes under what follows.
+__device__ __forceinline__ double ld_early(const double *p) {
+    double v;
+    asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
 __device__ __forceinline__ double ldg_t(const double *p) { return __ldg(p); }
 __device__ __forceinline__ float ldg_t(const float *p) { return __ldg(p); }
 
@@ -135,19 +156,26 @@ struct CpStage {
     int N;
     long long N3;
     bool act;
+    int tx, ty, pitch;
     int oc, c_s;
     int h_s[LY::HPT], h_g[LY::HPT], h_nf[LY::HPT];
 
-    __device__ __forceinline__ explicit CpStage(unsigned char *smem) : xs(reinterpret_cast<T *>(smem)) {}
+    // tw x th sites of a tile, one thread each: at most TX * TY of them, and
+    // a ring field of (tw + 2) x (th + 2) fits the layout's PY * PX
+    __device__ __forceinline__ CpStage(unsigned char *smem, int tw) : xs(reinterpret_cast<T *>(smem)) {
+        ty = (int)threadIdx.x / tw;
+        tx = (int)threadIdx.x - ty * tw;
+        pitch = tw + 2;
+    }
 
     // per-item set-up: this thread's own site and its halo copies
     __device__ __forceinline__ void begin(const StepConsts &c, int k0, int j0, int nk, int nj) {
         N = c.N;
         N3 = c.N3;
-        const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+        const int tid = threadIdx.x;
         act = (tx < nk) && (ty < nj);
         oc = (j0 + ty) * N + k0 + tx;
-        c_s = (ty + 1) * PX + tx + 1;
+        c_s = (ty + 1) * pitch + tx + 1;
         const int jlo = wrapi(j0 - 1, N), jhi = wrapi(j0 + nj, N);
         const int klo = wrapi(k0 - 1, N), khi = wrapi(k0 + nk, N);
 #pragma unroll
@@ -160,7 +188,7 @@ struct CpStage {
             else if (h < 2 * nk + 2 * nj) { r = h - 2 * nk - nj + 1; col = nk + 1; gj = j0 + h - 2 * nk - nj; gk = khi; nf = NF; }
             else if (GAUGED && h == 2 * nk + 2 * nj) { r = nj + 1; col = 0; gj = jhi; gk = klo; nf = 3; }
             else if (GAUGED && h == 2 * nk + 2 * nj + 1) { r = 0; col = nk + 1; gj = jlo; gk = khi; nf = 3; }
-            h_s[q] = r * PX + col;
+            h_s[q] = r * pitch + col;
             h_g[q] = gj * N + gk;
             h_nf[q] = nf;
         }
@@ -200,146 +228,362 @@ struct CpStage {
     template <int PENDING>
     __device__ __forceinline__ void wait(int) { cp_async_wait<PENDING>(); }
     __device__ __forceinline__ bool failed() const { return false; }
-    __device__ __forceinline__ T at(int slot, int f, int r, int col) const {
-        return xs[((slot * NR + f) * PY + r) * PX + col];
+    // the values around this thread's site in one slot
+    struct View {
+        const T *p;
+        int pitch;
+        __device__ __forceinline__ T get(int f, int dj, int dk) const { return p[f * (PY * PX) + dj * pitch + dk]; }
+        // the own value, read again instead of kept in a register
+        __device__ __forceinline__ T again(int f) const { return get(f, 0, 0); }
+    };
+    __device__ __forceinline__ View view(int slot) const { return View{xs + slot * LY::PLANE + c_s, pitch}; }
+};
+
+// ---------------------------------------------------------------- FP64
+
+// Per-thread sums of the first diagnostics pass (energies, charges, core and
+// centroid moments, the per-site terms of diag_ring.cuh) over the sites a
+// synchronous launch advances, without the constant factors, which step_sums
+// applies once per thread.
+enum : int {
+    SS_EPK = 0, SS_ETK, SS_EG, SS_ETG, SS_EP, SS_EC, SS_EE, SS_BB, SS_PINT, SS_TRS, SS_M0, SS_CX, SS_CY, SS_CZ,
+    SS_QP0, SS_QP1, SS_QP2, SS_QT, SS_QC, SS_N
+};
+struct StepSums {
+    double s[SS_N];
+    double pm, smax;   // largest |Phi_a|^2 and their product
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int q = 0; q < SS_N; q++) s[q] = 0.0;
+        pm = smax = 0.0;
     }
 };
 
-// One work item (a TX x TY column over one segment of planes) of one grid.
-// sync and damp are uniform per call; the single-grid kernel passes them as
-// constants, the multi-request kernel per request.  Stage stages the planes.
-// Per-site gradient, coupling and plaquette terms of the gauged diagnostics
-// (the energy's covariant gradients, eta (Phi . curl Theta), 1 - cos of the
-// three plaquettes; compute_energy_complex_gauge, sfa/sim/scp_sim.c:1930-2036)
-// for a synchronous FP64 launch that sums the first diagnostics pass: the
-// covariant differences are formed again from the ring (planes i, i+1) and
-// the thread's x(i-1).  Every input passes through an opaque copy first, so
-// that none of this arithmetic can merge with the force's (which would change
-// how the force's multiply-adds are fused): the launch advances the state bit
-// for bit as one that sums nothing.
-struct DiagGrad {
-    double eg, etg, ec, bb;
-};
-struct Plane12 {
-    double v[12];
-};
-
-__device__ __forceinline__ double opaque(double x) {
-    asm("" : "+d"(x));
-    return x;
+// The slots of the first pass from one thread's sums (the Gauss-law slots are
+// left to the pass that reads E of the neighbouring sites).
+__device__ __forceinline__ void step_sums(const StepSums &t, const StepConsts &c, DiagSums &o) {
+    o.clear();
+    const double hV = 0.5 * c.dV, g2 = c.idx1 * c.idx1;
+    o.S[DS_EPK] = hV * t.s[SS_EPK];
+    o.S[DS_ETK] = hV * t.s[SS_ETK];
+    o.S[DS_EG] = hV * g2 * t.s[SS_EG];
+    o.S[DS_ETG] = hV * g2 * t.s[SS_ETG];
+    o.S[DS_EM] = hV * c.m2 * t.s[SS_M0];
+    o.S[DS_ETM] = hV * c.mtheta2 * t.s[SS_TRS];
+    o.S[DS_EP] = hV * c.mu * t.s[SS_EP];
+    o.S[DS_EC] = -c.ei * c.dV * t.s[SS_EC];
+    o.S[DS_EEM] = c.dV * (0.5 * t.s[SS_EE] + c.bpre * t.s[SS_BB]);
+    o.S[DS_PINT] = c.dV * t.s[SS_PINT];
+    o.S[DS_TRS] = t.s[SS_TRS];
+    o.S[DS_QP] = t.s[SS_QP0] + t.s[SS_QP1] + t.s[SS_QP2];
+    o.S[DS_QT] = t.s[SS_QT];
+    o.S[DS_M0] = t.s[SS_M0];
+    o.S[DS_CX] = t.s[SS_CX];
+    o.S[DS_CY] = t.s[SS_CY];
+    o.S[DS_CZ] = t.s[SS_CZ];
+    o.S[DS_QC] = t.s[SS_QC];
+    o.S[DS_QP0] = t.s[SS_QP0];
+    o.S[DS_QP1] = t.s[SS_QP1];
+    o.S[DS_QP2] = t.s[SS_QP2];
+    o.M[DM_PM] = sqrt(t.pm);
+    o.M[DM_PMAX] = sqrt(t.smax);
+    o.M[DM_SMAX] = t.smax;
 }
 
-template <int TX, int TY>
-__device__ __forceinline__ DiagGrad diag_grad_gauged(const double *xs, int sc, int sp, int r, int col,
-                                                     const Plane12 &xm_in, double c0m_in, double s0m_in,
-                                                     double idx1_in) {
-    constexpr int NR = 15, PX = TX + 2, PY = TY + 2;
-    auto X = [&](int slot, int f, int rr, int cc) -> double {
-        return opaque(xs[((slot * NR + f) * PY + rr) * PX + cc]);
-    };
-    Plane12 xm;
+// The site's momenta w_n, read one plane ahead: each is replaced by the next
+// plane's as soon as its kick has used it, so a load has a whole plane of
+// arithmetic to pass under.
+template <bool GAUGED>
+struct Momenta {
+    double v[GAUGED ? 15 : 12];
+};
+
+// Kick, damping and drift of one site (scp_sim.c:1591-1715, fused) as the
+// accelerations come in; with DIAG also the per-site terms of the sums.
+template <bool GAUGED, bool FIRST, bool DIAG, class Stage>
+struct SiteUpdate {
+    const StepIO<F64> &io;
+    const StepConsts &c;
+    const Stage &stg;
+    StepSums *sums;
+    const long long site;
+    const int mslot;       // momentum slot of the staging (Stage::MOM)
+    const bool SYNC, DAMP;
+    Momenta<GAUGED> &w;
+    const long long next;   // elements to the next plane's site, 0 on a segment's last plane
+    double dmp = 1.0;
+    bool bad = false;
+    double rho = 0.0, rho2 = 0.0;   // charge density and sum of |Phi_a|^2 of the site (DIAG)
+
+    __device__ __forceinline__ double mom(int f) const {
+        if constexpr (Stage::MOM) return stg.mom(mslot, f);
+        else return w.v[f];
+    }
+    // the momentum of the next plane, once this plane's is used
+    __device__ __forceinline__ void ahead(int f) const {
+        if constexpr (!Stage::MOM)
+            if (next) w.v[f] = ld_early(io.win + f * c.N3 + site + next);
+    }
+    __device__ __forceinline__ double kick(double w, double a, double *wn) const {
+        double v = FIRST ? w : rfma(c.hdt, a, w);
+        if (DAMP && !FIRST) v = rmul(v, dmp);
+        *wn = rfma(c.hdt, a, v);
+        return v;
+    }
+    __device__ __forceinline__ double put(int f, double x, double a) {
+        double wn;
+        const double v = kick(mom(f), a, &wn);
+        ahead(f);
+        const double xn = rfma(c.dt, wn, x);
+        st_cs(io.xout + f * c.N3 + site, xn);
+        io.wout[f * c.N3 + site] = wn;
+        if (SYNC && !FIRST) {
+            st_cs(io.sout + f * c.N3 + site, v);
+            bad |= !isfinite(xn) || !isfinite(v);
+        }
+        return v;
+    }
+    __device__ __forceinline__ void theta(int a, double u, double v, double au, double av) {
+        const double pu = put(FTU + a, u, au), pv = put(FTV + a, v, av);
+        if constexpr (DIAG) {
+            sums->s[SS_ETK] += pu * pu + pv * pv;
+            sums->s[SS_TRS] += u * u + v * v;
+            const double q = u * pv - v * pu;
+            sums->s[SS_QT] += q;
+            rho += q;
+        }
+    }
+    __device__ __forceinline__ void phi(int a, double u, double v, double au, double av) {
+        const double pu = put(FU + a, u, au), pv = put(FV + a, v, av);
+        if constexpr (DIAG) {
+            sums->s[SS_EPK] += pu * pu + pv * pv;
+            const double q = u * pv - v * pu;
+            sums->s[SS_QP0 + a] += q;
+            rho += q;
+        }
+    }
+    // potential terms: squared moduli of Phi, den = 1 + kappa s
+    __device__ __forceinline__ void moduli(const double (&s)[3], double den) {
+        if constexpr (DIAG) {
+            const double s3 = s[0] * s[1] * s[2];
+            rho2 = s[0] + s[1] + s[2];
+            sums->s[SS_M0] += rho2;
+            sums->s[SS_EP] += s3 / den;
+            sums->s[SS_PINT] += sqrt(s3);
+            sums->pm = fmax(sums->pm, fmax(s[0], fmax(s[1], s[2])));
+            sums->smax = fmax(sums->smax, s3);
+        }
+    }
+    __device__ __forceinline__ void angles(double p0, double p1, double p2) {
+        if constexpr (DIAG) {   // 1 - cos of the site's own plaquettes, as 2 sin^2 of the half angle
+            double h[3] = {0.5 * p0, 0.5 * p1, 0.5 * p2};
+            sin_batch(h);
+            sums->s[SS_BB] += 2.0 * (h[0] * h[0] + h[1] * h[1] + h[2] * h[2]);
+        }
+    }
+    __device__ __forceinline__ void link(int d, double th0, double K) {
+        double Eh;
+        const double E = kick(mom(FTH + d), K, &Eh);
+        ahead(FTH + d);
+        const double th = link_wrap(rfma(c.gad, Eh, th0));
+        st_cs(io.xout + (FTH + d) * c.N3 + site, th);
+        io.wout[(FTH + d) * c.N3 + site] = Eh;
+        if (SYNC && !FIRST) {
+            st_cs(io.sout + (FTH + d) * c.N3 + site, E);
+            bad |= !isfinite(E) || !isfinite(th);
+        }
+        if constexpr (DIAG) sums->s[SS_EE] += E * E;
+    }
+};
+
+// compute_forces_complex (scp_sim.c:931-994) at one site, explicitly rounded
+// and visited field by field like gauged_site (Phi's neighbours, then Theta's,
+// each Theta field finished at once); xm: x(i-1) of the 12 fields, left
+// holding x(i)
+template <bool SUMS, class V, class Out>
+__device__ __forceinline__ void free_site(const V &cv, const V &pv, double (&xm)[12], const StepConsts &k, Out &out,
+                                          GaugedSums &sums) {
+    double crP[6], crT[6], lap[6];   // curls of Phi and Theta: real part [0..2], imaginary [3..5]
+    double eg = 0.0, etg = 0.0;
+    // one real field (part 0: real, 3: imaginary) of component a: its sum of
+    // neighbours, and its central differences (undivided) into the curl
+    auto field = [&](int f, int a, int part, double *cr, double &esum) -> double {
+        const double n[3] = {pv.get(f, 0, 0), cv.get(f, 1, 0), cv.get(f, 0, 1)};
+        const double m[3] = {xm[f], cv.get(f, -1, 0), cv.get(f, 0, -1)};
+        double l = 0.0;
 #pragma unroll
-    for (int f = 0; f < 12; f++) xm.v[f] = opaque(xm_in.v[f]);
-    const double c0m = opaque(c0m_in), s0m = opaque(s0m_in), idx1 = opaque(idx1_in);
-    DiagGrad o{0.0, 0.0, 0.0, 0.0};
-    double cr[3], ci[3];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        double cP, sP, cM, sM;
-        sincos_bounded(X(sc, FTH + d, r, col), &sP, &cP);
-        if (d == 0) { cM = c0m; sM = s0m; }
-        else if (d == 1) sincos_bounded(X(sc, FTH + 1, r - 1, col), &sM, &cM);
-        else sincos_bounded(X(sc, FTH + 2, r, col - 1), &sM, &cM);
-#pragma unroll
-        for (int q = 0; q < 6; q++) {
-            const int fre = q < 3 ? FU + q : FTU + q - 3, fim = q < 3 ? FV + q : FTV + q - 3;
-            double up, vp, um, vm;
-            if (d == 0) {
-                up = X(sp, fre, r, col); vp = X(sp, fim, r, col);
-                um = xm.v[fre]; vm = xm.v[fim];
-            } else if (d == 1) {
-                up = X(sc, fre, r + 1, col); vp = X(sc, fim, r + 1, col);
-                um = X(sc, fre, r - 1, col); vm = X(sc, fim, r - 1, col);
-            } else {
-                up = X(sc, fre, r, col + 1); vp = X(sc, fim, r, col + 1);
-                um = X(sc, fre, r, col - 1); vm = X(sc, fim, r, col - 1);
-            }
-            const double DR = ((cP * up - sP * vp) - (cM * um + sM * vm)) * idx1;
-            const double DI = ((cP * vp + sP * up) - (cM * vm - sM * um)) * idx1;
-            if (q < 3) o.eg += DR * DR + DI * DI;
-            else o.etg += DR * DR + DI * DI;
-            const int qa = q - 3;
-            if (q >= 3 && qa != d) {   // curl of Theta: D_{a+1} Theta_{a+2} - D_{a+2} Theta_{a+1}
-                if (qa == (d + 1) % 3) {
-                    const int a = (d + 2) % 3;
-                    if (d < (a + 2) % 3) { cr[a] = DR; ci[a] = DI; }
-                    else { cr[a] = DR - cr[a]; ci[a] = DI - ci[a]; }
-                } else {
-                    const int a = (d + 1) % 3;
-                    if (d < (a + 1) % 3) { cr[a] = DR; ci[a] = DI; }
-                    else { cr[a] = cr[a] - DR; ci[a] = ci[a] - DI; }
+        for (int d = 0; d < 3; d++) {
+            l = d == 0 ? radd(n[0], m[0]) : radd(radd(l, n[d]), m[d]);
+            if (a != d || SUMS) {
+                const double df = rsub(n[d], m[d]);
+                if (SUMS) esum += df * df;
+                if (a != d) {   // + in curl_{d+2} when a = d+1, - in curl_{d+1} when a = d+2
+                    const bool plus = (a == (d + 1) % 3);
+                    const int t = plus ? (d + 2) % 3 : (d + 1) % 3;
+                    const int other = plus ? (t + 1) % 3 : (t + 2) % 3;
+                    if (a < other) cr[part + t] = plus ? df : -df;
+                    else cr[part + t] = plus ? radd(cr[part + t], df) : rsub(cr[part + t], df);
                 }
             }
         }
+        xm[f] = cv.get(f, 0, 0);
+        return l;
+    };
+    auto acc = [&](double x, double l, double t, double cu) {
+        return rfma(k.ei, cu, rfma(rfma(-6.0, x, l), k.idx2, rmul(t, x)));
+    };
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        lap[a] = field(FU + a, a, 0, crP, eg);
+        lap[3 + a] = field(FV + a, a, 3, crP, eg);
     }
 #pragma unroll
-    for (int a = 0; a < 3; a++) o.ec += X(sc, FU + a, r, col) * cr[a] + X(sc, FV + a, r, col) * ci[a];
-#pragma unroll
-    for (int q = 0; q < 3; q++) {   // plaquette (q, q+1) at x, the next plane in slot sp
-        const int a = q, b = (q + 1) % 3;
-        const int sa = (a == 0) ? sp : sc, ra = r + (a == 1 ? 1 : 0), ca = col + (a == 2 ? 1 : 0);
-        const int sb = (b == 0) ? sp : sc, rb = r + (b == 1 ? 1 : 0), cb = col + (b == 2 ? 1 : 0);
-        double sn, cs;
-        sincos_any(X(sc, FTH + a, r, col) + X(sa, FTH + b, ra, ca) - X(sb, FTH + a, rb, cb) - X(sc, FTH + b, r, col),
-                   &sn, &cs);
-        o.bb += 1.0 - cs;
+    for (int a = 0; a < 3; a++) {
+        const double lu = field(FTU + a, a, 0, crT, etg), lv = field(FTV + a, a, 3, crT, etg);
+        const double u = xm[FTU + a], v = xm[FTV + a];
+        out.theta(a, u, v, acc(u, lu, -k.mtheta2, crP[a]), acc(v, lv, -k.mtheta2, crP[3 + a]));
     }
-    return o;
+    double s[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) s[a] = rfma(xm[FU + a], xm[FU + a], rmul(xm[FV + a], xm[FV + a]));
+    const double den = rfma(k.kappa, rmul(rmul(s[0], s[1]), s[2]), 1.0);
+    const double nV2 = -k.mu / rmul(den, den);   // -2 V'
+    out.moduli(s, den);
+    double ec = 0.0;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const double t = rfma(nV2, rmul(s[(a + 1) % 3], s[(a + 2) % 3]), -k.m2);
+        const double u = xm[FU + a], v = xm[FV + a];
+        if (SUMS) ec += u * crT[a] + v * crT[3 + a];
+        out.phi(a, u, v, acc(u, lap[a], t, crT[a]), acc(v, lap[3 + a], t, crT[3 + a]));
+    }
+    if (SUMS) { sums.eg = eg; sums.etg = etg; sums.ec = ec; }
 }
 
-// Per-thread sums and maxima of the first diagnostics pass kept in shared
-// memory (slot q of thread t at q * NT + t), so that the synchronous launch
-// that sums them keeps its registers for the force.
-struct DiagSmem {
-    double *base;
-    int nt;
-    struct Ref {
-        double *p;
-        int nt;
-        __device__ __forceinline__ double &operator[](int q) const { return p[q * nt]; }
-    };
-    __device__ __forceinline__ Ref S() const { return Ref{base + threadIdx.x, nt}; }
-    __device__ __forceinline__ Ref M() const { return Ref{base + DS_NSUM * nt + threadIdx.x, nt}; }
-    static constexpr size_t bytes(int nt) { return sizeof(double) * kDiag1Q * (size_t)nt; }
-};
+// One work item (a tile column over one segment of planes) of one FP64 grid.
+// sync and damp are uniform per call; the single-grid kernel passes them as
+// constants, the multi-request kernel per request.  Stage stages the planes.
+template <int TX, int TY, bool GAUGED, bool FIRST, bool DIAG, class Stage>
+__device__ __forceinline__ void step_item(const StepIO<F64> &io, const StepConsts &c, const TileGrid &tg,
+                                          const Piece &pc, const bool SYNC, const bool DAMP, Stage &stg,
+                                          StepSums *sums = nullptr) {
+    const int N = c.N;
+    const int tx = stg.tx, ty = stg.ty;
+    const int k0 = pc.kt * tg.tw, j0 = pc.jt * tg.th;
+    const int i0 = pc.i0, i1 = pc.i1;
+    const int k = k0 + tx, j = j0 + ty;
+    const int nk = min(k0 + tg.tw, N) - k0, nj = min(j0 + tg.th, N) - j0;   // valid extent of the tile
+    const bool act = (tx < nk) && (ty < nj);
+    const int oc = j * N + k;                                          // in-plane offset (act only)
+    stg.begin(c, k0, j0, nk, nj);
 
-// dsum (FP64 SYNC launches only): per-thread sums of the first diagnostics
-// pass over this item's sites, the per-site terms of diag_ring.cuh / diag.cuh
-// (compute_energy_complex[_gauge], compute_charges, sfa/sim/scp_sim.c:1823-2169)
-// evaluated from the values the step holds; the Gauss-law slots are left to
-// a pass that reads E of the neighbouring sites.
-template <class P, int TX, int TY, bool GAUGED, bool FIRST, class Stage>
-__device__ __forceinline__ void step_item(const StepIO<P> &io, const StepConsts &c, const Piece &pc,
-                                          const bool SYNC, const bool DAMP, Stage &stg, const DiagSmem *dsum = nullptr) {
-    const bool DG = !P::COMP && dsum != nullptr;
-    using T = typename P::T;
+    __syncthreads();   // previous item finished reading the ring
+    stg.issue(io, i0 - 1, 0);
+    stg.issue(io, i0, 1);
+    stg.commit();
+    // planes i0+1 .. i0+NS-2, one copy group each
+    constexpr int NS = Stage::NSLOT;
+#pragma unroll
+    for (int q = 1; q <= NS - 2; q++) {
+        if (i0 + q <= i1) stg.issue(io, i0 + q, q + 1);
+        stg.commit();
+    }
+    Momenta<GAUGED> w;
+    if constexpr (Stage::MOM) {
+        stg.issue_mom(i0, 0);   // momenta of the first plane
+    } else if (act) {
+#pragma unroll
+        for (int f = 0; f < (GAUGED ? 15 : 12); f++)
+            w.v[f] = ld_early(io.win + f * c.N3 + (long long)i0 * N * N + oc);
+    }
+    stg.template wait<NS - 2>(0);
+    stg.template wait<NS - 2>(1);
+    __syncthreads();
+    GaugedCarry cy;
+    double xm[12];
+    if (act) {
+        if constexpr (GAUGED) {
+            gauged_begin(stg.view(0), stg.view(1), FTH, cy);
+        } else {
+            const auto m = stg.view(0);
+#pragma unroll
+            for (int f = 0; f < 12; f++) xm[f] = m.get(f, 0, 0);
+        }
+    }
+
+    for (int i = i0; i < i1; i++) {
+        // plane p sits in slot (p - i0 + 1) mod NS; plane i + NS - 1 reuses the slot of i - 1
+        const int sc = (i - i0 + 1) % NS, sp = (i - i0 + 2) % NS, sn = (i - i0) % NS;
+        stg.template wait<NS - 3>(sp);   // the copies of planes beyond i+1 may stay in flight
+        if constexpr (Stage::MOM) stg.wait_mom((i - i0) & 1);
+        __syncthreads();
+        if (i + NS - 1 <= i1) stg.issue(io, i + NS - 1, sn);
+        if constexpr (Stage::MOM) {   // momenta of the next plane, into the slot plane i-1 used
+            if (i + 1 < i1) stg.issue_mom(i + 1, (i + 1 - i0) & 1);
+        }
+        stg.commit();
+        if (!act) continue;
+        const long long site = (long long)i * N * N + oc;
+        if (c.prefetch && i + 1 < i1) {
+#pragma unroll
+            for (int f = 0; f < (GAUGED ? 15 : 12); f++)
+                prefetch_line_l2(io.win + f * c.N3 + site + (long long)N * N);
+        }
+        SiteUpdate<GAUGED, FIRST, DIAG, Stage> out{io, c, stg, sums, site, (i - i0) & 1, SYNC, DAMP, w,
+                                                    i + 1 < i1 ? (long long)N * N : 0};
+        if (DAMP && !FIRST) {
+            const double x = -c.L + i * c.dx, y = -c.L + j * c.dx, z = -c.L + k * c.dx;
+            const double r = sqrt(x * x + y * y + z * z);
+            const double Rd = c.L - c.damp_width;
+            if (r > Rd) {
+                double sc2 = (r - Rd) / c.damp_width;
+                if (sc2 > 1) sc2 = 1;
+                out.dmp = 1.0 - c.damp_rate * sc2 * sc2;
+            }
+        }
+        GaugedSums gs;
+        if constexpr (GAUGED) gauged_site<DIAG>(stg.view(sc), stg.view(sp), FTH, cy, GaugedConsts(c), out, gs);
+        else free_site<DIAG>(stg.view(sc), stg.view(sp), xm, c, out, gs);
+        if (SYNC && out.bad) atomicOr(io.flag, 1);
+        if constexpr (DIAG) {
+            sums->s[SS_EG] += gs.eg;
+            sums->s[SS_ETG] += gs.etg;
+            sums->s[SS_EC] += gs.ec;
+            const double x = -c.L + i * c.dx, y = -c.L + j * c.dx, z = -c.L + k * c.dx;
+            sums->s[SS_CX] += x * out.rho2;
+            sums->s[SS_CY] += y * out.rho2;
+            sums->s[SS_CZ] += z * out.rho2;
+            if (x * x + y * y + z * z <= c.R2) sums->s[SS_QC] += out.rho;
+            if constexpr (GAUGED) io.drho[site] = out.rho;
+        }
+    }
+}
+
+// ---------------------------------------------------------------- compensated FP32, one site per thread
+
+template <int TX, int TY, bool GAUGED, bool FIRST>
+__device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepConsts &c, const TileGrid &tg,
+                                            const Piece &pc, const bool SYNC, const bool DAMP,
+                                            CpStage<F32C, TX, TY, GAUGED> &stg) {
+    using P = F32C;
+    using T = float;
+    using Stage = CpStage<F32C, TX, TY, GAUGED>;
     using LY = StepLayout<P, TX, TY, GAUGED>;
     constexpr int NF = LY::NF;
     constexpr int NR = LY::NR;
-    auto XS = [&](int slot, int f, int r, int col) -> T { return stg.at(slot, f, r, col); };
     const int N = c.N;
     const long long N3 = c.N3;
-    const int tid = threadIdx.x;
-    const int tx = tid % TX, ty = tid / TX;
+    const int tx = stg.tx, ty = stg.ty;
+    auto XS = [&](int slot, int f, int r, int col) -> T { return stg.view(slot).get(f, r - ty - 1, col - tx - 1); };
     const T dt = (T)c.dt, hdt = (T)c.hdt, idx1 = (T)c.idx1, idx2 = (T)c.idx2;
     const float dt_lo = (float)(c.dt - (double)(float)c.dt);
     const float hdt_lo = (float)(c.hdt - (double)(float)c.hdt);
 
     {
-        const int k0 = pc.kt * TX, j0 = pc.jt * TY;
+        const int k0 = pc.kt * tg.tw, j0 = pc.jt * tg.th;
         const int i0 = pc.i0, i1 = pc.i1;
         const int k = k0 + tx, j = j0 + ty;
-        const int nk = min(k0 + TX, N) - k0, nj = min(j0 + TY, N) - j0;   // valid extent of the tile
+        const int nk = min(k0 + tg.tw, N) - k0, nj = min(j0 + tg.th, N) - j0;   // valid extent of the tile
         const bool act = (tx < nk) && (ty < nj);
         const int oc = j * N + k;                                          // in-plane offset (act only)
         stg.begin(c, k0, j0, nk, nj);
@@ -422,19 +666,6 @@ __device__ __forceinline__ void step_item(const StepIO<P> &io, const StepConsts 
                 }
             }
             if (!act) continue;
-            // diagnostics: gradient, coupling and plaquette terms, formed before the
-            // force while few of its values are live (link 0 at x - i is still the carry)
-            DiagGrad gr{0.0, 0.0, 0.0, 0.0};
-            if constexpr (!P::COMP && GAUGED && std::is_same<Stage, CpStage<P, TX, TY, GAUGED>>::value) {
-                if (DG) {
-                    Plane12 xp;
-#pragma unroll
-                    for (int f = 0; f < 12; f++) xp.v[f] = (double)xm[f];
-                    gr = diag_grad_gauged<TX, TY>(stg.xs, sc, sp, ty + 1, tx + 1, xp, (double)c0m, (double)s0m,
-                                                  c.idx1);
-                }
-            }
-
             T acc[12];
             T K[3] = {T(0), T(0), T(0)};
             T ctr[NF];
@@ -486,30 +717,6 @@ __device__ __forceinline__ void step_item(const StepIO<P> &io, const StepConsts 
                     acc[FTU + a] = lap(FTU + a) - mt2 * x + eta * curl(FU, a);
                     x = ctr[FTV + a];
                     acc[FTV + a] = lap(FTV + a) - mt2 * x + eta * curl(FV, a);
-                }
-                if constexpr (!P::COMP) {
-                    if (DG) {   // gradient energies and the Cosserat coupling energy
-                        double eg = 0.0, etg = 0.0;
-#pragma unroll
-                        for (int d = 0; d < 3; d++) {
-#pragma unroll
-                            for (int q = 0; q < 6; q++) {
-                                const int fre = q < 3 ? FU + q : FTU + q - 3, fim = q < 3 ? FV + q : FTV + q - 3;
-                                // rounded products of their own (the step's fused ones stay as they are)
-                                const double DR = __dmul_rn(nb(fre, 2 * d) - nb(fre, 2 * d + 1), idx1);
-                                const double DI = __dmul_rn(nb(fim, 2 * d) - nb(fim, 2 * d + 1), idx1);
-                                const double e2 = __fma_rn(DR, DR, __dmul_rn(DI, DI));
-                                if (q < 3) eg += e2;
-                                else etg += e2;
-                            }
-                        }
-                        const auto S = dsum->S();
-                        S[DS_EG] += 0.5 * eg * c.dV;
-                        S[DS_ETG] += 0.5 * etg * c.dV;
-#pragma unroll
-                        for (int a = 0; a < 3; a++)
-                            S[DS_EC] -= c.eta * (ctr[FU + a] * curl(FTU, a) + ctr[FV + a] * curl(FTV, a)) * c.dV;
-                    }
                 }
             } else {
                 // compute_forces_complex_gauge pass C, scp_sim.c:1112-1262
@@ -640,7 +847,6 @@ __device__ __forceinline__ void step_item(const StepIO<P> &io, const StepConsts 
                 }
             }
             bool bad = false;
-            double vv[NF];   // diagnostics: v_{n+1}, E_{n+1}
 #pragma unroll
             for (int f = 0; f < 12; f++) {
                 T v, wn, xn;
@@ -659,12 +865,6 @@ __device__ __forceinline__ void step_item(const StepIO<P> &io, const StepConsts 
                     float e;
                     two_sum(ctr[f], y, &xn, &e);
                     io.loout[f * N3 + site] = f_to_bf16(e);
-                } else {
-                    v = FIRST ? w[f] : w[f] + hdt * acc[f];
-                    if (DAMP && !FIRST) v *= dmp;
-                    wn = v + hdt * acc[f];
-                    xn = ctr[f] + dt * wn;
-                    vv[f] = v;
                 }
                 st_cs(io.xout + f * N3 + site, xn);
                 io.wout[f * N3 + site] = wn;
@@ -696,12 +896,6 @@ __device__ __forceinline__ void step_item(const StepIO<P> &io, const StepConsts 
                             two_sum(t1, lnew, &th, &lnew);
                         }
                         io.tloout[d * N3 + site] = lnew;
-                    } else {
-                        E = FIRST ? w[FTH + d] : w[FTH + d] + hdt * K[d];
-                        if (DAMP && !FIRST) E *= dmp;
-                        Eh = E + hdt * K[d];
-                        th = link_wrap(ctr[FTH + d] + gad * Eh);
-                        vv[FTH + d] = E;
                     }
                     st_cs(io.xout + (FTH + d) * N3 + site, th);
                     io.wout[(FTH + d) * N3 + site] = Eh;
@@ -712,73 +906,6 @@ __device__ __forceinline__ void step_item(const StepIO<P> &io, const StepConsts 
                 }
             }
             if (SYNC && bad) atomicOr(io.flag, 1);
-            if constexpr (!P::COMP) {
-                if (DG) {   // energies, charges, core and centroid moments at (x_{n+1}, v_{n+1})
-                    // squares of the positions by rounded products of their own, so
-                    // that they do not merge with the force's (whose fused
-                    // multiply-adds would then change): the step's arithmetic is the
-                    // same with and without these sums
-                    const auto S = dsum->S();
-                    const auto M = dsum->M();
-                    const double dV = c.dV;
-                    double s2[3];
-#pragma unroll
-                    for (int a = 0; a < 3; a++) {
-                        const double u = ctr[FU + a], w0 = ctr[FV + a], tu = ctr[FTU + a], tv = ctr[FTV + a];
-                        s2[a] = __fma_rn(u, u, __dmul_rn(w0, w0));
-                        const double pu = vv[FU + a], pv = vv[FV + a], ptu = vv[FTU + a], ptv = vv[FTV + a];
-                        S[DS_EPK] += 0.5 * (pu * pu + pv * pv) * dV;
-                        S[DS_ETK] += 0.5 * (ptu * ptu + ptv * ptv) * dV;
-                        S[DS_EM] += 0.5 * c.m2 * s2[a] * dV;
-                        S[DS_ETM] += 0.5 * c.mtheta2 * __fma_rn(tu, tu, __dmul_rn(tv, tv)) * dV;
-                        M[DM_PM] = fmax(M[DM_PM], sqrt(s2[a]));
-                    }
-                    const double s3 = s2[0] * s2[1] * s2[2];
-                    S[DS_EP] += (c.mu / 2.0) * s3 / (1.0 + c.kappa * s3) * dV;
-                    M[DM_PMAX] = fmax(M[DM_PMAX], sqrt(s3));
-                    S[DS_PINT] += sqrt(s3) * dV;
-#pragma unroll
-                    for (int a = 0; a < 3; a++)
-                        S[DS_TRS] += __fma_rn(ctr[FTU + a], ctr[FTU + a], __dmul_rn(ctr[FTV + a], ctr[FTV + a]));
-                    const double x = -c.L + i * c.dx, y = -c.L + j * c.dx, z = -c.L + k * c.dx;
-                    double rho2 = 0.0, qp = 0.0, qt = 0.0, sprod = 1.0;
-#pragma unroll
-                    for (int a = 0; a < 3; a++) {
-                        const double qa = ctr[FU + a] * vv[FV + a] - ctr[FV + a] * vv[FU + a];
-                        qp += qa;
-                        S[DS_QP0 + a] += qa;
-                        qt += ctr[FTU + a] * vv[FTV + a] - ctr[FTV + a] * vv[FTU + a];
-                        const double s2a = s2[a];
-                        rho2 += s2a;
-                        sprod *= s2a;
-                    }
-                    S[DS_QP] += qp;
-                    S[DS_QT] += qt;
-                    if (x * x + y * y + z * z <= c.R2) S[DS_QC] += qp + qt;
-                    M[DM_SMAX] = fmax(M[DM_SMAX], sprod);
-                    S[DS_M0] += rho2;
-                    S[DS_CX] += x * rho2;
-                    S[DS_CY] += y * rho2;
-                    S[DS_CZ] += z * rho2;
-                    if constexpr (GAUGED && std::is_same<Stage, CpStage<P, TX, TY, GAUGED>>::value) {
-                        // gradient, coupling and plaquette energies; Gauss charge density; E_em
-                        S[DS_EG] += 0.5 * gr.eg * dV;
-                        S[DS_ETG] += 0.5 * gr.etg * dV;
-                        S[DS_EC] -= c.eta * gr.ec * dV;
-                        const double bbE = gr.bb;
-                        double rho = 0.0;
-#pragma unroll
-                        for (int a = 0; a < 3; a++)
-                            rho += ctr[FU + a] * vv[FV + a] - ctr[FV + a] * vv[FU + a] +
-                                   ctr[FTU + a] * vv[FTV + a] - ctr[FTV + a] * vv[FTU + a];
-                        io.drho[site] = rho;
-                        const double E0 = vv[FTH], E1 = vv[FTH + 1], E2 = vv[FTH + 2];
-                        double ee = 0.5 * (E0 * E0 + E1 * E1 + E2 * E2);
-                        ee += c.bpre * bbE;
-                        S[DS_EEM] += ee * dV;
-                    }
-                }
-            }
 #pragma unroll
             for (int f = 0; f < 12; f++) xm[f] = ctr[f];
         }
@@ -786,38 +913,46 @@ __device__ __forceinline__ void step_item(const StepIO<P> &io, const StepConsts 
 }
 
 // Single grid: persistent CTAs over the grid's work items.
-// resident CTAs per SM the register allocation is sized for
-// (FP64 at 3 CTAs of 128 threads would spill the gauged force; FP32C fits)
+// Resident CTAs per SM the register allocation is sized for.
 template <class P, int TX, int TY, bool GAUGED>
 struct MinBlocks {
     static constexpr int value = (TX * TY > 128) ? 1 : (P::COMP ? 3 : 2);
 };
 
+template <class P, int TX, int TY, bool GAUGED, bool FIRST, class Stage>
+__device__ __forceinline__ void step_one(const StepIO<P> &io, const StepConsts &c, const TileGrid &tg, const Piece &pc,
+                                         const bool SYNC, const bool DAMP, Stage &stg) {
+    if constexpr (P::COMP) step_item_c<TX, TY, GAUGED, FIRST>(io, c, tg, pc, SYNC, DAMP, stg);
+    else step_item<TX, TY, GAUGED, FIRST, false>(io, c, tg, pc, SYNC, DAMP, stg);
+}
+
 template <class P, int TX, int TY, bool GAUGED, bool FIRST, bool SYNC, bool DAMP>
 __global__ void __launch_bounds__(TX * TY, (MinBlocks<P, TX, TY, GAUGED>::value))
 step_kernel(StepIO<P> io, StepConsts c, TileGrid tg) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    CpStage<P, TX, TY, GAUGED> stg(smem_raw);
-    if constexpr (SYNC && !FIRST && !P::COMP) {
-        if (io.dpart) {   // uniform: this launch also sums the first diagnostics pass
-            using LY = StepLayout<P, TX, TY, GAUGED>;
-            const DiagSmem dsm{reinterpret_cast<double *>(smem_raw + LY::smem_bytes), TX * TY};
-#pragma unroll
-            for (int q = 0; q < kDiag1Q; q++) dsm.base[q * TX * TY + threadIdx.x] = 0.0;
-            for_each_piece(tg, c.N, [&](const Piece &pc) {
-                step_item<P, TX, TY, GAUGED, FIRST>(io, c, pc, SYNC, DAMP, stg, &dsm);
-            });
-            __syncthreads();   // the ring is free: its first 7.4 KB serve as the fold's scratch
-            DiagSums acc;
-#pragma unroll
-            for (int q = 0; q < DS_NSUM; q++) acc.S[q] = dsm.S()[q];
-#pragma unroll
-            for (int q = 0; q < DM_NMAX; q++) acc.M[q] = dsm.M()[q];
-            block_fold<DS_NSUM, DM_NMAX>(acc.S, acc.M, reinterpret_cast<double *>(smem_raw), io.dpart);
-            return;
-        }
-    }
-    for_each_piece(tg, c.N, [&](const Piece &pc) { step_item<P, TX, TY, GAUGED, FIRST>(io, c, pc, SYNC, DAMP, stg); });
+    CpStage<P, TX, TY, GAUGED> stg(smem_raw, tg.tw);
+    for_each_piece(tg, c.N, [&](const Piece &pc) {
+        step_one<P, TX, TY, GAUGED, FIRST>(io, c, tg, pc, SYNC, DAMP, stg);
+    });
+}
+
+// The synchronous FP64 launch that also sums the first diagnostics pass: the
+// sums stay in registers (two CTAs per SM hold them without spills) and are
+// folded to one partial per CTA at the end, the ring serving as scratch.
+template <int TX, int TY, bool GAUGED, bool DAMP>
+__global__ void __launch_bounds__(TX * TY, (MinBlocks<F64, TX, TY, GAUGED>::value))
+step_diag_kernel(StepIO<F64> io, StepConsts c, TileGrid tg) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    CpStage<F64, TX, TY, GAUGED> stg(smem_raw, tg.tw);
+    StepSums sums;
+    sums.clear();
+    for_each_piece(tg, c.N, [&](const Piece &pc) {
+        step_item<TX, TY, GAUGED, false, true>(io, c, tg, pc, true, DAMP, stg, &sums);
+    });
+    __syncthreads();
+    DiagSums acc;
+    step_sums(sums, c, acc);
+    block_fold<DS_NSUM, DM_NMAX>(acc.S, acc.M, reinterpret_cast<double *>(smem_raw), io.dpart);
 }
 
 // ---------------------------------------------------------------- many grids per launch
@@ -877,8 +1012,8 @@ step_multi_kernel(const ReqTable<P> *tab, int k) {
         const StepIO<P> io = q.io[(int)((s - q.s0) & 1)];
         const StepConsts c = q.c;
         const TileGrid tg = q.tg;
-        CpStage<P, TX, TY, GAUGED> stg(smem_raw);
-        step_item<P, TX, TY, GAUGED, false>(io, c, piece_of_item(tg, item - q.item0, c.N), false, DAMP, stg);
+        CpStage<P, TX, TY, GAUGED> stg(smem_raw, tg.tw);
+        step_one<P, TX, TY, GAUGED, false>(io, c, tg, piece_of_item(tg, item - q.item0, c.N), false, DAMP, stg);
     }
 }
 

@@ -103,8 +103,11 @@ struct TmaStage {
     int h_s[LY::HPT];        // this thread's halo-column doubles: shared offset in a slot,
     long long h_g[LY::HPT];  // offset in a plane of the buffer (field * N^3 + j * N + k), -1: none
     bool timed_out = false;
+    int tx, ty;
 
     __device__ __forceinline__ TmaStage(unsigned char *smem, const TmaMaps *m, int *fl) : maps(m), flag(fl) {
+        ty = (int)threadIdx.x / TX;
+        tx = (int)threadIdx.x - ty * TX;
         // round up to 128 bytes by offsetting the shared array itself (an
         // integer round trip would hide the address space and turn every ring
         // read into a generic load)
@@ -192,10 +195,18 @@ struct TmaStage {
         }
         phase ^= 1u << s;
     }
-    __device__ __forceinline__ double at(int slot, int f, int r, int col) const {
-        const int off = (col == 0) ? LY::LEFT + r : (col == TX + 1 ? LY::RIGHT + r : r * TX + col - 1);
-        return xs[slot * LY::SLOT + f * LY::FS + off];
-    }
+    // the values around this thread's site in one slot (rows from j0 - 1)
+    struct View {
+        const double *p;
+        int tx, ty;
+        __device__ __forceinline__ double get(int f, int dj, int dk) const {
+            const int r = ty + 1 + dj, col = tx + 1 + dk;
+            const int off = (dk < 0 && col == 0) ? LY::LEFT + r : ((dk > 0 && col == TX + 1) ? LY::RIGHT + r : r * TX + col - 1);
+            return p[f * LY::FS + off];
+        }
+        __device__ __forceinline__ double again(int f) const { return get(f, 0, 0); }
+    };
+    __device__ __forceinline__ View view(int slot) const { return View{xs + slot * LY::SLOT, tx, ty}; }
 };
 
 // The cp.async position ring with the momenta staged through TMA: one dense
@@ -223,7 +234,7 @@ struct CpMomStage : CpStage<F64, TX, TY, GAUGED> {
     bool timed_out = false;
 
     __device__ __forceinline__ CpMomStage(unsigned char *smem, const CUtensorMap *m, int *fl)
-        : Base(smem), mmap(m), flag(fl) {
+        : Base(smem, TX), mmap(m), flag(fl) {
         const unsigned base = smem_u32(smem);
         const unsigned off = ((base + (unsigned)ring_bytes + 127u) & ~127u) - base;
         ms = reinterpret_cast<double *>(smem + off);
@@ -266,27 +277,27 @@ struct CpMomStage : CpStage<F64, TX, TY, GAUGED> {
 };
 
 template <int TX, int TY, bool GAUGED, bool FIRST, bool SYNC, bool DAMP>
-__global__ void __launch_bounds__(TX * TY, (MinBlocks<F64, TX, TY, GAUGED>::value))
+__global__ void __launch_bounds__(TX * TY, TX * TY > 128 ? 1 : 2)
 step_cpm_kernel(StepIO<F64> io, StepConsts c, TileGrid tg, const __grid_constant__ CUtensorMap mmap) {
     extern __shared__ __align__(16) unsigned char cpm_smem[];
     CpMomStage<TX, TY, GAUGED> stg(cpm_smem, &mmap, io.flag);
     bool stop = false;
     for_each_piece(tg, c.N, [&](const Piece &pc) {
         if (stop) return;
-        step_item<F64, TX, TY, GAUGED, FIRST>(io, c, pc, SYNC, DAMP, stg);
+        step_item<TX, TY, GAUGED, FIRST, false>(io, c, tg, pc, SYNC, DAMP, stg);
         stop = __syncthreads_or(stg.timed_out);   // every thread leaves together
     });
 }
 
 template <int TX, int TY, bool GAUGED, bool FIRST, bool SYNC, bool DAMP>
-__global__ void __launch_bounds__(TX * TY, (MinBlocks<F64, TX, TY, GAUGED>::value))
+__global__ void __launch_bounds__(TX * TY, TX * TY > 128 ? 1 : 2)
 step_tma_kernel(StepIO<F64> io, StepConsts c, TileGrid tg, const __grid_constant__ TmaMaps maps) {
     extern __shared__ __align__(16) unsigned char tma_smem[];   // aligned to 128 bytes by TmaStage
     TmaStage<TX, TY, GAUGED> stg(tma_smem, &maps, io.flag);
     bool stop = false;
     for_each_piece(tg, c.N, [&](const Piece &pc) {
         if (stop) return;
-        step_item<F64, TX, TY, GAUGED, FIRST>(io, c, pc, SYNC, DAMP, stg);
+        step_item<TX, TY, GAUGED, FIRST, false>(io, c, tg, pc, SYNC, DAMP, stg);
         stop = __syncthreads_or(stg.timed_out);   // every thread leaves together
     });
 }

@@ -105,6 +105,103 @@ __device__ __forceinline__ void sincos_any(double x, double *sn, double *cs) {
     }
 }
 
+// ---------------------------------------------------------------- batches
+//
+// Several angles of one site together (FP64), so that the range reduction --
+// needed only beyond pi/4 (sine and cosine) or pi/2 (sine alone) -- is one
+// branch for the batch: link and plaquette angles of a smooth state lie
+// inside.  The reduced argument goes through near-minimax polynomials (Remez
+// exchange on the absolute error, coefficients rounded to double):
+//   |r| <= pi/4: sine to r^13 (8e-18), cosine to r^14 (2e-18)
+//   |r| <= pi/2: sine to r^17 (4e-17, the rounding of 1/6)
+// Two parts of pi (53 bits each) suffice for the reduction, since each product
+// k * P is exact inside its fused multiply-add.
+
+__device__ __forceinline__ unsigned abs_hi(double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; }
+__device__ __forceinline__ double flip_sign(double x, unsigned bit) {   // bit: 0 or 1
+    return __hiloint2double(__double2hiint(x) ^ (int)(bit << 31), __double2loint(x));
+}
+constexpr double kRintMagic = 6755399441055744.0;   // 1.5 * 2^52: adding it rounds to an integer
+
+// sines and cosines of n angles, |a| < 2^20
+template <int n>
+__device__ __forceinline__ void sincos_batch(const double (&ang)[n], double (&sn)[n], double (&cs)[n]) {
+    double r[n];
+    unsigned q[n], big = 0;
+#pragma unroll
+    for (int i = 0; i < n; i++) {
+        r[i] = ang[i];
+        q[i] = 0;
+        big |= (abs_hi(ang[i]) >= 0x3fe921fbu) ? 1u : 0u;   // high word of pi/4
+    }
+    if (big) {
+#pragma unroll
+        for (int i = 0; i < n; i++) {
+            const double t = __fma_rn(ang[i], 0x1.45f306dc9c883p-1, kRintMagic);   // 2/pi
+            const double kq = __dadd_rn(t, -kRintMagic);
+            r[i] = __fma_rn(-kq, 0x1.921fb54442d18p+0, ang[i]);
+            r[i] = __fma_rn(-kq, 0x1.1a62633145c07p-54, r[i]);
+            q[i] = (unsigned)__double2loint(t) & 3u;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < n; i++) {
+        const double x = r[i], s = __dmul_rn(x, x);
+        double p = __fma_rn(0x1.5d64c939ea033p-33, s, -0x1.ae5db478930bap-26);
+        p = __fma_rn(p, s, 0x1.71de347564b0ep-19);
+        p = __fma_rn(p, s, -0x1.a01a019ab4ae1p-13);
+        p = __fma_rn(p, s, 0x1.111111110eb1fp-7);
+        p = __fma_rn(p, s, -0x1.555555555553dp-3);
+        sn[i] = __fma_rn(__dmul_rn(x, s), p, x);
+        double c = __fma_rn(-0x1.8f806eafe7abbp-37, s, 0x1.1ee984acd9d7cp-29);
+        c = __fma_rn(c, s, -0x1.27e4f7537ae12p-22);
+        c = __fma_rn(c, s, 0x1.a01a019b6f8afp-16);
+        c = __fma_rn(c, s, -0x1.6c16c16c13f18p-10);
+        c = __fma_rn(c, s, 0x1.555555555553cp-5);
+        c = __fma_rn(c, s, -0.5);
+        cs[i] = __fma_rn(s, c, 1.0);
+    }
+    if (big) {   // x = r + q pi/2: rotate by q quarter turns
+#pragma unroll
+        for (int i = 0; i < n; i++) {
+            const double s1 = (q[i] & 1) ? cs[i] : sn[i];
+            const double c1 = (q[i] & 1) ? -sn[i] : cs[i];
+            sn[i] = flip_sign(s1, q[i] >> 1);
+            cs[i] = flip_sign(c1, q[i] >> 1);
+        }
+    }
+}
+
+// n angles replaced by their sines, |a| < 2^20
+template <int n>
+__device__ __forceinline__ void sin_batch(double (&x)[n]) {
+    unsigned big = 0;
+#pragma unroll
+    for (int i = 0; i < n; i++) big |= (abs_hi(x[i]) >= 0x3ff921fbu) ? 1u : 0u;   // high word of pi/2
+    if (big) {
+#pragma unroll
+        for (int i = 0; i < n; i++) {   // x = r + k pi: sin x = (-1)^k sin r
+            const double t = __fma_rn(x[i], 0x1.45f306dc9c883p-2, kRintMagic);   // 1/pi
+            const double kq = __dadd_rn(t, -kRintMagic);
+            double r = __fma_rn(-kq, 0x1.921fb54442d18p+1, x[i]);
+            r = __fma_rn(-kq, 0x1.1a62633145c07p-53, r);
+            x[i] = flip_sign(r, (unsigned)__double2loint(t) & 1u);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < n; i++) {
+        const double r = x[i], s = __dmul_rn(r, r);
+        double p = __fma_rn(0x1.87c6cf61f7134p-49, s, -0x1.ae3f19d8db60ep-41);
+        p = __fma_rn(p, s, 0x1.6123ba0dcfa88p-33);
+        p = __fma_rn(p, s, -0x1.ae64547e9f285p-26);
+        p = __fma_rn(p, s, 0x1.71de3a51c6a39p-19);
+        p = __fma_rn(p, s, -0x1.a01a01a012737p-13);
+        p = __fma_rn(p, s, 0x1.1111111111093p-7);
+        p = __fma_rn(p, s, -0x1.5555555555555p-3);
+        x[i] = __fma_rn(__dmul_rn(r, s), p, r);
+    }
+}
+
 template <class T>
 __device__ __forceinline__ T sin_bounded(T x) {
     T s, c;
