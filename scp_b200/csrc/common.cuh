@@ -87,6 +87,21 @@ __device__ __forceinline__ double wrap_angle(double v) {
     return v - twopi * rint(v / twopi);
 }
 
+// link wrap into (-pi, pi] (reference: v - 2*pi*rint(v/(2*pi)), scp_sim.c:1647);
+// |v| < 3 never wraps, so the division only runs for the rare large angles
+__device__ __forceinline__ double link_wrap(double v) {
+    if (fabs(v) < 3.0) return v;
+    return wrap_angle(v);
+}
+
+// A load that stays where it is written: the compiler does not move it down to
+// its first use, so its latency passes under what follows.
+__device__ __forceinline__ double ld_early(const double *p) {
+    double v;
+    asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
 __device__ __forceinline__ int wrapi(int x, int N) { return x < 0 ? x + N : (x >= N ? x - N : x); }
 
 // (i, j, k) of site idx = (i*N + j)*N + k: 32-bit divisions while the index

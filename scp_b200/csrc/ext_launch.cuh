@@ -60,31 +60,21 @@ struct HuIO {
 int hu_plan(bool higgs, bool g2, int N, int nsm, ExtPlan *plan);
 cudaError_t hu_step(bool higgs, bool g2, const ExtPlan &plan, const HuConsts &c, const HuIO &io, cudaStream_t st);
 
-// One fabric's matter step, and the shared links' step.
+// One fabric's matter step, with the shared links' step in the last one.
+// Array groups: [0] the fabric's 12 matter arrays, [1] the links (th; E).
 struct FabIO {
-    const double *x;      // the fabric's 12 matter positions x_{n+1}
-    const double *th;     // the 3 link angles x_{n+1}
-    double *xout;         // 12 matter positions x_{n+2}
-    const double *win;    // 12 momenta
-    double *wout, *sout;
-    double *kacc;         // 3 arrays of accumulated currents
+    const double *src[2];   // positions x_{n+1}
+    double *xout[2];
+    const double *win[2];
+    double *wout[2], *sout[2];
+    double *kacc;           // 3 arrays of accumulated currents
     int *flag;
-    double qf, gqf;       // force charge and current weight
-    double qx, gqx;       // second current over the same fields (second != 0)
-    int first, sync, damp, accumulate, second;
+    double qf, gqf;         // force charge and current weight g qf / dx
+    double qx, gqx;         // second current over the same fields (second != 0)
+    int first, sync, damp, accumulate, second, links;
 };
-struct LinkIO {
-    const double *th;     // x_{n+1}
-    double *thout;
-    const double *kacc;
-    const double *win;    // E
-    double *wout, *sout;
-    int *flag;
-    int first, sync, damp;
-};
-int fabric_plan(int N, int nsm, ExtPlan *fabric, ExtPlan *second, ExtPlan *link);
+int fabric_plan(int N, int nsm, ExtPlan *plan);
 cudaError_t fabric_step(const ExtPlan &plan, const FabConsts &c, const FabIO &io, cudaStream_t st);
-cudaError_t link_step(const ExtPlan &plan, const FabConsts &c, const LinkIO &io, cudaStream_t st);
 
 // Real mode with the optional terms: positions / momenta are 6 arrays (phi,
 // theta); aux holds C and B (6 arrays) when the strain or hardening is on.

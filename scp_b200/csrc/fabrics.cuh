@@ -12,17 +12,22 @@
 // q_Q force (the Q pass overwrites C's accelerations) while both fabrics add
 // their currents, g q_C J_C(C) + g q_Q J_Q(C).  Here Q's arrays are C's.
 //
-// Structure.  One time step is one ring launch per fabric and one for the
-// links.  A fabric launch stages the fabric's 12 matter fields and the three
-// link angles, advances the fabric's matter by the fused leapfrog, and adds
-// its currents g q J to a per-site accumulator; the link launch stages the
-// angles, forms the plaquette term, and kicks E and drifts the angles with
-// the accumulated currents.  Positions (two alternating buffers) and momenta
-// hold C with the links (15 arrays, the fused step's order), then L (12),
-// then Q (12) when it is not locked.
+// Structure.  One time step is one walker launch (walk.cuh) per moving fabric:
+// it stages the fabric's 12 matter fields and the three link angles, advances
+// the fabric's matter by the fused leapfrog, and adds its currents g q J to a
+// per-site accumulator; the last fabric's launch takes the sum instead, forms
+// the plaquette term from the angles it staged anyway, kicks E and drifts the
+// angles.  Positions (two alternating buffers) and momenta hold C with the
+// links (15 arrays, the fused step's order), then L (12), then Q (12) when it
+// is not locked.
+//
+// What bounds it: DRAM, 936 B per site with Q locked (432 for C, 504 for L
+// with the links) against 864 that no split can avoid; 370 us a step at 128^3
+// (0.76 of a plain copy's rate on the 864 B) against 524 with four resident
+// planes, momenta loaded at their own plane and a launch of its own for the
+// links.
 #pragma once
-#include "multiplet.cuh"
-#include "ring.cuh"
+#include "walk.cuh"
 
 namespace scp {
 
@@ -33,196 +38,125 @@ struct FabConsts {
     double mu, kappa, m2, mtheta2, eta;
     double g, stp, gad;
     double damp_width, damp_rate;
+    double ei, cross, gi;   // eta/(2dx), eta dx/2, and (unused here) g/dx
 };
+
+// Forward-transport current of one fabric under links of charge qx, in units
+// of 1/dx, cross terms included (the locked pair's C current).
+template <class V>
+__device__ __forceinline__ void fabric_current(const V &c, const V &p, int fth, double qx, double r0, double (&K)[3]) {
+    double ang[3], sn[3], cs[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        ang[d] = rmul(qx, c.get(fth + d, 0, 0));
+        K[d] = 0.0;
+    }
+    sincos_batch<3, true>(ang, sn, cs);
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+        const int fre = field_re(q), fim = field_im(q), a = q % 3;
+        const double u = c.get(fre, 0, 0), v = c.get(fim, 0, 0);
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            const double up = d == 0 ? p.get(fre, 0, 0) : c.get(fre, d == 1, d == 2);
+            const double vp = d == 0 ? p.get(fim, 0, 0) : c.get(fim, d == 1, d == 2);
+            const double fr = rfma(-sn[d], vp, rmul(cs[d], up)), fi = rfma(sn[d], up, rmul(cs[d], vp));
+            double gu = u, gv = v;
+            if (a != d) {
+                const int b = 3 - d - a, o = q < 3 ? 3 + b : b;
+                const double r = (a == (d + 1) % 3) ? r0 : -r0;
+                gu = rfma(r, c.again(field_re(o)), u);
+                gv = rfma(r, c.again(field_im(o)), v);
+            }
+            K[d] = rfma(gu, fi, K[d]);
+            K[d] = rfma(-gv, fr, K[d]);
+        }
+    }
+}
 
 // One fabric's matter step.  The force uses links of charge qf; the current
 // g qf J(qf) goes to the accumulator, preceded, with SECOND, by g qx J(qx)
-// over the same fields (the locked pair's C current).
-template <bool SECOND>
+// over the same fields (the locked pair's C current), and with ACC added to
+// what the fabrics before left there.  With LINKS the launch
+// also steps the shared links with the accumulated currents.
+template <class MODE, bool SECOND, bool ACC, bool LINKS>
 struct FabricPass {
+    static_assert(!LINKS || ACC, "the links come with the last fabric");
     static constexpr int TH = 12;
-    static constexpr int NR = 15;
+    static constexpr int NR = 15, NA = 12, CF = LINKS ? 12 : 15;
+    static constexpr int NM = LINKS ? 15 : 12;
     static constexpr int MIN_CTAS = 1;
+    static constexpr bool HALO_APART = true;
 
     struct Args {
-        RingSrc<NR> src;      // this fabric's 12 matter positions, then th
+        const double *src[2];   // this fabric's 12 matter positions; th
         int N;
         FabConsts c;
-        double qf, gqf;       // force charge, current weight g qf
-        double qx, gqx;       // second current (SECOND)
-        const double *win;    // 12 momenta: w_n (v_0 on the first launch)
-        double *wout, *xout, *sout;
-        double *kacc;         // 3 arrays: accumulated currents
-        int *flag;
-        int first, sync, damp, accumulate;
+        double qf, gqf;         // force charge, current weight g qf / dx
+        double qx, gqx;         // second current (SECOND)
+        LeapIO io;              // matter; E and th (LINKS)
+        double *kacc;           // 3 arrays: accumulated currents
     };
 
-    struct Carry {
-        double cm, sm;        // charge-qf link phase along i at x - i
-        double cmx, smx;      // the same for qx
+    struct State {
+        GaugedCarry cy;
+        double w[NM];
+        double kin[3];          // the accumulated currents, read one plane ahead
     };
 
-    __device__ static void prefetch(const Args &A, long long idx) {
+    __device__ static __forceinline__ void load(const Args &A, State &st, long long idx) {
 #pragma unroll
-        for (int f = 0; f < 12; f++) prefetch_l2(A.win + f * A.c.N3 + idx);
-        if (A.accumulate)
+        for (int f = 0; f < NM; f++) st.w[f] = ld_early(LeapSite<MODE, NM>::at(A.io.win, f, A.c.N3) + idx);
 #pragma unroll
-            for (int d = 0; d < 3; d++) prefetch_l2(A.kacc + d * A.c.N3 + idx);
+        for (int d = 0; d < 3; d++) st.kin[d] = ACC ? ld_early(A.kacc + d * A.c.N3 + idx) : 0.0;
     }
+    template <class V>
+    __device__ static __forceinline__ void begin(const Args &A, State &st, const V &m, const V &c) {
+        gauged_begin<true, LINKS>(m, c, TH, st.cy, A.qf);
+    }
+
+    struct Out {
+        const Args &A;
+        State &st;
+        LeapSite<MODE, NM> &leap;
+        double (&kx)[3];        // g qx J(qx) dx (SECOND)
+        __device__ __forceinline__ void theta(int a, double u, double v, double au, double av) {
+            leap.put(FTU + a, u, au, leap.dmp);
+            leap.put(FTV + a, v, av, leap.dmp);
+        }
+        __device__ __forceinline__ void phi(int a, double u, double v, double au, double av) {
+            leap.put(FU + a, u, au, leap.dmp);
+            leap.put(FV + a, v, av, leap.dmp);
+        }
+        __device__ __forceinline__ void moduli(const double (&)[3], double) {}
+        __device__ __forceinline__ void angles(double, double, double) {}
+        // the fabric's current on top of what the others left
+        __device__ __forceinline__ double current(int d, double K) {
+            double t = rmul(A.gqf, K);
+            if (SECOND) t = rfma(A.gqx, kx[d], t);
+            if (ACC) t = radd(st.kin[d], t);
+            if (ACC) st.kin[d] = ld_early(A.kacc + d * A.c.N3 + leap.site + leap.next);
+            if (!LINKS) A.kacc[d * A.c.N3 + leap.site] = t;
+            return t;
+        }
+        __device__ __forceinline__ void link(int d, double th, double K) {
+            leap.put_link(FTH + d, th, K, A.c.gad, leap.dmp);
+        }
+    };
 
     template <class V>
-    __device__ static void site(const Args &A, const V &v, int i, int j, int k, long long idx, Carry &cy,
-                                bool first_plane) {
-        const FabConsts &c = A.c;
-        const long long N3 = c.N3;
-        // the momenta and the accumulated currents are loaded first, so their
-        // latency passes under the stencil instead of stalling the kicks
-        double wv[12], kin[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int f = 0; f < 12; f++) wv[f] = A.win[f * N3 + idx];
-        if (A.accumulate) {
-#pragma unroll
-            for (int d = 0; d < 3; d++) kin[d] = A.kacc[d * N3 + idx];
-        }
-        double own[12];
-#pragma unroll
-        for (int f = 0; f < 12; f++) own[f] = v(f);
-        if (first_plane) {
-            sincos_any(A.qf * v.at(TH, -1, 0, 0), &cy.sm, &cy.cm);
-            if (SECOND) sincos_any(A.qx * v.at(TH, -1, 0, 0), &cy.smx, &cy.cmx);
-        }
-        const double zero[3] = {0.0, 0.0, 0.0};
-        double kc[3];
-        if (SECOND) {   // the current of the lock partner, same fields, charge qx
-            auto lx = [&](int d, double cP[3], double sP[3], double cM[3], double sM[3], double &cW, double &sW) {
-                sincos_any(A.qx * v(TH + d), &sW, &cW);
-                double cm, sm;
-                if (d == 0) { cm = cy.cmx; sm = cy.smx; cy.cmx = cW; cy.smx = sW; }
-                else sincos_any(A.qx * nb(v, TH + d, d, -1), &sm, &cm);
-#pragma unroll
-                for (int a = 0; a < 3; a++) { cP[a] = cW; sP[a] = sW; cM[a] = cm; sM[a] = sm; }
-            };
-            MultipletOut ox;
-            covariant_multiplet<false>(v, 0, own, lx, zero, c.idx1, c.inva, c.eta, ox);
-#pragma unroll
-            for (int d = 0; d < 3; d++) kc[d] = A.gqx * ox.jlat[d];
-        }
-        auto links = [&](int d, double cP[3], double sP[3], double cM[3], double sM[3], double &cW, double &sW) {
-            sincos_any(A.qf * v(TH + d), &sW, &cW);
-            double cm, sm;
-            if (d == 0) { cm = cy.cm; sm = cy.sm; cy.cm = cW; cy.sm = sW; }
-            else sincos_any(A.qf * nb(v, TH + d, d, -1), &sm, &cm);
-#pragma unroll
-            for (int a = 0; a < 3; a++) { cP[a] = cW; sP[a] = sW; cM[a] = cm; sM[a] = sm; }
-        };
-        MultipletOut o;
-        covariant_multiplet<false>(v, 0, own, links, zero, c.idx1, c.inva, c.eta, o);
-#pragma unroll
-        for (int d = 0; d < 3; d++) kc[d] = SECOND ? kc[d] + A.gqf * o.jlat[d] : A.gqf * o.jlat[d];
-
-        double sa[3];
-#pragma unroll
-        for (int a = 0; a < 3; a++) sa[a] = own[MU + a] * own[MU + a] + own[MV + a] * own[MV + a];
-        const double den = 1.0 + c.kappa * (sa[0] * sa[1] * sa[2]);
-        const double Vp = 0.5 * c.mu / (den * den);
-        double acc[12];
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            const double others = sa[(a + 1) % 3] * sa[(a + 2) % 3];
-            const double u = own[MU + a], w = own[MV + a], tu = own[MTU + a], tw = own[MTV + a];
-            acc[MU + a] = (o.lsum[MU + a] - 6.0 * u) * c.idx2 - c.m2 * u - 2.0 * Vp * u * others + c.eta * o.curlT[a];
-            acc[MV + a] = (o.lsum[MV + a] - 6.0 * w) * c.idx2 - c.m2 * w - 2.0 * Vp * w * others +
-                          c.eta * o.curlT[3 + a];
-            acc[MTU + a] = (o.lsum[MTU + a] - 6.0 * tu) * c.idx2 - c.mtheta2 * tu + c.eta * o.curlP[a];
-            acc[MTV + a] = (o.lsum[MTV + a] - 6.0 * tw) * c.idx2 - c.mtheta2 * tw + c.eta * o.curlP[3 + a];
-        }
-#pragma unroll
-        for (int d = 0; d < 3; d++) A.kacc[d * N3 + idx] = A.accumulate ? kin[d] + kc[d] : kc[d];
-        const Leap leap{c.hdt, c.dt, A.first != 0};
-        const double dmp = (A.damp && !A.first) ? sponge_at(i, j, k, c.L, c.dx, c.damp_width, c.damp_rate) : 1.0;
-        bool bad = false;
-#pragma unroll
-        for (int f = 0; f < 12; f++) {
-            double vv, wn;
-            leap(wv[f], acc[f], dmp, &vv, &wn);
-            const double x = own[f] + c.dt * wn;
-            st_cs(A.xout + f * N3 + idx, x);
-            A.wout[f * N3 + idx] = wn;
-            if (A.sync) {
-                st_cs(A.sout + f * N3 + idx, vv);
-                bad |= !isfinite(x) || !isfinite(vv);
-            }
-        }
-        if (A.sync && bad) atomicOr(A.flag, 1);
-    }
-};
-
-// The shared links: plaquette term plus the accumulated currents kick E
-// (damped in the sponge), then the angles drift and wrap.
-struct LinkPass {
-    static constexpr int NR = 3;
-    static constexpr int MIN_CTAS = 2;
-
-    struct Args {
-        RingSrc<NR> src;      // th
-        int N;
-        FabConsts c;
-        const double *kacc;
-        const double *win;    // E: w_n (E_0 on the first launch)
-        double *wout, *xout, *sout;
-        int *flag;
-        int first, sync, damp;
-    };
-
-    struct Carry {
-        double pm[2];         // plaquette sines (0,1), (2,0) at x - i
-    };
-
-    __device__ static void prefetch(const Args &A, long long idx) {
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            prefetch_l2(A.win + d * A.c.N3 + idx);
-            prefetch_l2(A.kacc + d * A.c.N3 + idx);
-        }
-    }
-
-    template <class V>
-    __device__ static void site(const Args &A, const V &v, int i, int j, int k, long long idx, Carry &cy,
-                                bool first_plane) {
-        const FabConsts &c = A.c;
-        const long long N3 = c.N3;
-        // E and the accumulated currents first: their latency passes under the staples
-        double wv[3], kin[3];
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            wv[d] = A.win[d * N3 + idx];
-            kin[d] = A.kacc[d * N3 + idx];
-        }
-        if (first_plane) {
-            cy.pm[0] = plaquette_sin(v, 0, 0, -1, 0, 0);
-            cy.pm[1] = plaquette_sin(v, 0, 2, -1, 0, 0);
-        }
-        double st[3], pat[2];
-        staples(v, 0, cy.pm, st, pat);
-        cy.pm[0] = pat[0];
-        cy.pm[1] = pat[1];
-        const Leap leap{c.hdt, c.dt, A.first != 0};
-        const double dmp = (A.damp && !A.first) ? sponge_at(i, j, k, c.L, c.dx, c.damp_width, c.damp_rate) : 1.0;
-        bool bad = false;
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            const double K = c.stp * st[d] + kin[d];
-            double E, Eh;
-            leap(wv[d], K, dmp, &E, &Eh);
-            const double th = wrap_angle(v(d) + c.gad * Eh);
-            st_cs(A.xout + d * N3 + idx, th);
-            A.wout[d * N3 + idx] = Eh;
-            if (A.sync) {
-                st_cs(A.sout + d * N3 + idx, E);
-                bad |= !isfinite(th) || !isfinite(E);
-            }
-        }
-        if (A.sync && bad) atomicOr(A.flag, 1);
+    __device__ static __forceinline__ void site(const Args &A, State &st, const V &c, const V &p, int i, int j, int k,
+                                                long long idx, long long next) {
+        const FabConsts &fc = A.c;
+        const double dmp = (MODE::DAMP && !MODE::FIRST)
+                               ? sponge_factor(i, j, k, fc.L, fc.dx, fc.damp_width, fc.damp_rate) : 1.0;
+        LeapSite<MODE, NM> leap{A.io, st.w, fc.N3, idx, next, fc.hdt, fc.dt, dmp};
+        double kx[3];
+        if (SECOND) fabric_current(c, p, TH, A.qx, fc.cross, kx);
+        Out out{A, st, leap, kx};
+        GaugedSums none;
+        gauged_site<false, true, LINKS>(c, p, TH, st.cy, GaugedConsts(fc), out, none, A.qf);
+        if (MODE::SYNC && leap.bad) atomicOr(A.io.flag, 1);
     }
 };
 

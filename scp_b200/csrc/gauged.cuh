@@ -38,10 +38,22 @@ __device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a,
 __device__ __forceinline__ double rsub(double a, double b) { return __dadd_rn(a, -b); }
 __device__ __forceinline__ double rfma(double a, double b, double c) { return __fma_rn(a, b, c); }
 
+// sponge factor 1 - rate * s^2 of the absorbing boundary at site (i, j, k),
+// 1 inside radius L - width (apply_damping, sfa/sim/scp_sim.c:1440-1473)
+__device__ __forceinline__ double sponge_factor(int i, int j, int k, double L, double dx, double width, double rate) {
+    const double x = rfma(i, dx, -L), y = rfma(j, dx, -L), z = rfma(k, dx, -L);
+    const double r = sqrt(rfma(z, z, rfma(y, y, rmul(x, x))));
+    const double inner = rsub(L, width);
+    if (!(r > inner)) return 1.0;
+    const double s = fmin(rsub(r, inner) / width, 1.0);
+    return rfma(rmul(-rate, s), s, 1.0);
+}
+
 // Constants derived from StepConsts that only the site function uses.
 struct GaugedConsts {
     double idx2, ei, nm2, nmt2, kappa, mu, r, gi, stp;
-    __device__ __forceinline__ explicit GaugedConsts(const StepConsts &c)
+    template <class C>
+    __device__ __forceinline__ explicit GaugedConsts(const C &c)
         : idx2(c.idx2), ei(c.ei), nm2(-c.m2), nmt2(-c.mtheta2), kappa(c.kappa), mu(c.mu), r(c.cross), gi(c.gi),
           stp(c.stp) {}
 };
@@ -73,22 +85,133 @@ __device__ __forceinline__ double plaq_angle(const V &c, const V &p, int fth, in
 __device__ __forceinline__ constexpr int field_re(int q) { return q < 3 ? FU + q : FTU + q - 3; }
 __device__ __forceinline__ constexpr int field_im(int q) { return q < 3 ? FV + q : FTV + q - 3; }
 
+// plaquette sines (0,1) and (2,0) of the plane viewed by m (next: c)
+template <class V>
+__device__ __forceinline__ void staples_begin(const V &m, const V &c, int fth, double &p0, double &p2) {
+    double pa[2] = {plaq_angle(m, c, fth, 0, 0, 0), plaq_angle(m, c, fth, 2, 0, 0)};
+    sin_batch(pa);
+    p0 = pa[0];
+    p2 = pa[1];
+}
+
 // The carry of the plane before the first one of a segment: m views plane
 // i0-1, c plane i0.
-template <class V>
-__device__ __forceinline__ void gauged_begin(const V &m, const V &c, int fth, GaugedCarry &cy) {
+template <bool CHARGED, bool LINKS, class V>
+__device__ __forceinline__ void gauged_begin(const V &m, const V &c, int fth, GaugedCarry &cy, double charge = 1.0) {
     double a0[1] = {m.get(fth, 0, 0)}, sn[1], cs[1];
-    sincos_batch(a0, sn, cs);
+    if (CHARGED) a0[0] = rmul(charge, a0[0]);
+    sincos_batch<1, CHARGED>(a0, sn, cs);
 #pragma unroll
     for (int q = 0; q < 6; q++) {
         const double u = m.get(field_re(q), 0, 0), v = m.get(field_im(q), 0, 0);
         cy.t[field_re(q)] = rfma(sn[0], v, rmul(cs[0], u));
         cy.t[field_im(q)] = rfma(-sn[0], u, rmul(cs[0], v));
     }
-    double pa[2] = {plaq_angle(m, c, fth, 0, 0, 0), plaq_angle(m, c, fth, 2, 0, 0)};
+    if constexpr (LINKS) staples_begin(m, c, fth, cy.p0, cy.p2);
+}
+
+// One complex field q through its three directions.  cs, sn: the phases of
+// its links at x (0..2), at x - j (3) and at x - k (4); t: the carried
+// backward transports along i.  Adds to the currents K (in units of 1/dx,
+// cross terms with the factor r = eta dx / 2 included), to the curl of its
+// triplet (cr, ci: differences undivided) and, with SUMS, to esum (squared
+// differences); returns the Laplacian's sum of transports in lu, lv.
+//
+// With G2 the components have phases of their own and the cross terms take
+// the first gauge's link alone on their Theta(x + d) side (cw, sw); Kw sums
+// the current weighted by the component's second charge w.
+struct TwoGauge {
+    const double *cw, *sw;   // first gauge's link phases at x, per direction
+    double w;                // second charge of this component
+    double *Kw;
+};
+template <bool SUMS, bool G2, class V>
+__device__ __forceinline__ void transport_field(const V &c, const V &p, const int q, const double *cs,
+                                                const double *sn, double *t, double *K, const double rx, double *cr,
+                                                double *ci, double &lu, double &lv, double &esum,
+                                                const TwoGauge &g2) {
+    const int fre = field_re(q), fim = field_im(q), a = q % 3;
+    const double u = c.get(fre, 0, 0), v = c.get(fim, 0, 0);
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const double cP = cs[d], sP = sn[d];
+        const double up = d == 0 ? p.get(fre, 0, 0) : c.get(fre, d == 1, d == 2);
+        const double vp = d == 0 ? p.get(fim, 0, 0) : c.get(fim, d == 1, d == 2);
+        const double fr = rfma(-sP, vp, rmul(cP, up)), fi = rfma(sP, up, rmul(cP, vp));
+        double br, bi;
+        if (d == 0) {
+            br = t[fre];
+            bi = t[fim];
+            t[fre] = rfma(sP, v, rmul(cP, u));
+            t[fim] = rfma(-sP, u, rmul(cP, v));
+        } else {
+            const double cM = cs[2 + d], sM = sn[2 + d];
+            const double um = c.get(fre, -(d == 1), -(d == 2)), vm = c.get(fim, -(d == 1), -(d == 2));
+            br = rfma(sM, vm, rmul(cM, um));
+            bi = rfma(-sM, um, rmul(cM, vm));
+        }
+        if (d == 0) { lu = radd(fr, br); lv = radd(fi, bi); }
+        else { lu = radd(radd(lu, fr), br); lv = radd(radd(lv, fi), bi); }
+        // the current; Phi_a meets Theta_b and Theta_a meets Phi_b, b the third
+        // index, with sign + where a = d+1
+        const int b = 3 - d - a, o = q < 3 ? 3 + b : b;
+        const double r = (a == (d + 1) % 3) ? rx : -rx;
+        if constexpr (!G2) {
+            double gu = u, gv = v;
+            if (a != d) {   // the own value plus r times the partner's
+                gu = rfma(r, c.again(field_re(o)), u);
+                gv = rfma(r, c.again(field_im(o)), v);
+            }
+            K[d] = rfma(gu, fi, K[d]);
+            K[d] = rfma(-gv, fr, K[d]);
+        } else {
+            const double j = rfma(-v, fr, rmul(u, fi));
+            K[d] = radd(K[d], j);
+            g2.Kw[d] = rfma(g2.w, j, g2.Kw[d]);
+            if (a != d) {
+                double xr = fr, xi = fi;
+                if (q >= 3) {
+                    xr = rfma(-g2.sw[d], vp, rmul(g2.cw[d], up));
+                    xi = rfma(g2.sw[d], up, rmul(g2.cw[d], vp));
+                }
+                const double x = rfma(-c.again(field_im(o)), xr, rmul(c.again(field_re(o)), xi));
+                K[d] = rfma(r, x, K[d]);
+            }
+        }
+        // curl_c = D_{c+1} f_{c+2} - D_{c+2} f_{c+1}
+        if (a != d || SUMS) {
+            const double dr = rsub(fr, br), di = rsub(fi, bi);
+            if (SUMS) esum += dr * dr + di * di;
+            if (a != d) {
+                const bool plus = (a == (d + 1) % 3);
+                const int s = plus ? (d + 2) % 3 : (d + 1) % 3;
+                const int other = plus ? (s + 1) % 3 : (s + 2) % 3;   // field of the other term
+                if (a < other) { cr[s] = plus ? dr : -dr; ci[s] = plus ? di : -di; }
+                else if (plus) { cr[s] = radd(cr[s], dr); ci[s] = radd(ci[s], di); }
+                else { cr[s] = rsub(cr[s], dr); ci[s] = rsub(ci[s], di); }
+            }
+        }
+    }
+}
+
+// Field kick of one gauge's plaquettes (scp_sim.c:1214-1220): staples from
+// the sines at x and at x less the other direction of the plane; p0, p2: the
+// sines at x - i, replaced by this plane's.  pa receives the site's angles.
+template <class V>
+__device__ __forceinline__ void staples(const V &c, const V &p, int fth, double &p0, double &p2, double (&st)[3],
+                                        double (&own)[3]) {
+    double pa[7] = {plaq_angle(c, p, fth, 0, 0, 0), plaq_angle(c, p, fth, 1, 0, 0), plaq_angle(c, p, fth, 2, 0, 0),
+                    plaq_angle(c, p, fth, 0, -1, 0), plaq_angle(c, p, fth, 1, -1, 0),
+                    plaq_angle(c, p, fth, 1, 0, -1), plaq_angle(c, p, fth, 2, 0, -1)};
+    own[0] = pa[0];
+    own[1] = pa[1];
+    own[2] = pa[2];
     sin_batch(pa);
-    cy.p0 = pa[0];
-    cy.p2 = pa[1];
+    st[0] = rsub(rsub(pa[0], pa[3]), rsub(pa[2], pa[6]));
+    st[1] = rsub(rsub(pa[1], pa[5]), rsub(pa[0], p0));
+    st[2] = rsub(rsub(pa[2], p2), rsub(pa[1], pa[4]));
+    p0 = pa[0];
+    p2 = pa[2];
 }
 
 // The force at one site: c views plane i, p plane i+1, cy carries plane i-1
@@ -98,79 +221,34 @@ __device__ __forceinline__ void gauged_begin(const V &m, const V &c, int fth, Ga
 //   out.phi(a, u, v, au, av)     Phi_a and its accelerations
 //   out.angles(p0, p1, p2)       the site's own plaquette angles
 //   out.link(d, th, K)           link angle d and the kick of E_d
-template <bool SUMS, class V, class Out>
+// Variants: the links carry the charge `charge` (CHARGED); LINKS = false
+// leaves the plaquettes out and hands the bare currents to out.current(d, K);
+// nhh adds nhh prod_{b != a} |Phi_b|^2 Phi_a to Phi's force (the Higgs).
+template <bool SUMS, bool CHARGED, bool LINKS, class V, class Out>
 __device__ __forceinline__ void gauged_site(const V &c, const V &p, int fth, GaugedCarry &cy, const GaugedConsts &k,
-                                            Out &out, GaugedSums &sums) {
+                                            Out &out, GaugedSums &sums, double charge = 1.0, double nhh = 0.0) {
     // link phases at x (U_0, U_1, U_2) and at x - j, x - k
     double ang[5] = {c.get(fth, 0, 0), c.get(fth + 1, 0, 0), c.get(fth + 2, 0, 0), c.get(fth + 1, -1, 0),
                      c.get(fth + 2, 0, -1)};
     double sn[5], cs[5];
-    sincos_batch(ang, sn, cs);
+    if (CHARGED) {
+#pragma unroll
+        for (int i = 0; i < 5; i++) ang[i] = rmul(charge, ang[i]);
+        sincos_batch<5, true>(ang, sn, cs);
+    } else {
+        sincos_batch(ang, sn, cs);
+    }
     double K[3] = {0.0, 0.0, 0.0};
     double crP[3], ciP[3], crT[3], ciT[3], lapU[3], lapV[3];
     double eg = 0.0, etg = 0.0;
-    // one field through its three directions
-    auto field = [&](int q, double *lu_out, double *lv_out, double *cr, double *ci, double &esum) {
-        const int fre = field_re(q), fim = field_im(q), a = q % 3;
-        const double u = c.get(fre, 0, 0), v = c.get(fim, 0, 0);
-        double lu = 0.0, lv = 0.0;
+    const TwoGauge none{};
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-            const double cP = cs[d], sP = sn[d];
-            const double up = d == 0 ? p.get(fre, 0, 0) : c.get(fre, d == 1, d == 2);
-            const double vp = d == 0 ? p.get(fim, 0, 0) : c.get(fim, d == 1, d == 2);
-            const double fr = rfma(-sP, vp, rmul(cP, up)), fi = rfma(sP, up, rmul(cP, vp));
-            double br, bi;
-            if (d == 0) {
-                br = cy.t[fre];
-                bi = cy.t[fim];
-                cy.t[fre] = rfma(sP, v, rmul(cP, u));
-                cy.t[fim] = rfma(-sP, u, rmul(cP, v));
-            } else {
-                const double cM = cs[2 + d], sM = sn[2 + d];
-                const double um = c.get(fre, -(d == 1), -(d == 2)), vm = c.get(fim, -(d == 1), -(d == 2));
-                br = rfma(sM, vm, rmul(cM, um));
-                bi = rfma(-sM, um, rmul(cM, vm));
-            }
-            if (d == 0) { lu = radd(fr, br); lv = radd(fi, bi); }
-            else { lu = radd(radd(lu, fr), br); lv = radd(radd(lv, fi), bi); }
-            // the current, cross terms included: the own value plus r times the partner's
-            double gu = u, gv = v;
-            if (a != d) {
-                // Phi_a meets Theta_b, Theta_a meets Phi_b, b the third index;
-                // sign + for (Phi, a = d+1) and (Theta, a = d+1) with reversed roles
-                const int b = 3 - d - a;
-                const int o = q < 3 ? 3 + b : b;
-                const bool plus = (a == (d + 1) % 3);
-                const double r = plus ? k.r : -k.r;
-                gu = rfma(r, c.again(field_re(o)), u);
-                gv = rfma(r, c.again(field_im(o)), v);
-            }
-            K[d] = rfma(gu, fi, K[d]);
-            K[d] = rfma(-gv, fr, K[d]);
-            // curl_c = D_{c+1} f_{c+2} - D_{c+2} f_{c+1}, differences undivided
-            if (a != d || SUMS) {
-                const double dr = rsub(fr, br), di = rsub(fi, bi);
-                if (SUMS) esum += dr * dr + di * di;
-                if (a != d) {
-                    const bool plus = (a == (d + 1) % 3);
-                    const int t = plus ? (d + 2) % 3 : (d + 1) % 3;
-                    const int other = plus ? (t + 1) % 3 : (t + 2) % 3;   // field of the other term
-                    if (a < other) { cr[t] = plus ? dr : -dr; ci[t] = plus ? di : -di; }
-                    else if (plus) { cr[t] = radd(cr[t], dr); ci[t] = radd(ci[t], di); }
-                    else { cr[t] = rsub(cr[t], dr); ci[t] = rsub(ci[t], di); }
-                }
-            }
-        }
-        *lu_out = lu;
-        *lv_out = lv;
-    };
-#pragma unroll
-    for (int a = 0; a < 3; a++) field(a, &lapU[a], &lapV[a], crP, ciP, eg);
+    for (int a = 0; a < 3; a++)
+        transport_field<SUMS, false>(c, p, a, cs, sn, cy.t, K, k.r, crP, ciP, lapU[a], lapV[a], eg, none);
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         double lu, lv;
-        field(3 + a, &lu, &lv, crT, ciT, etg);
+        transport_field<SUMS, false>(c, p, 3 + a, cs, sn, cy.t, K, k.r, crT, ciT, lu, lv, etg, none);
         const double u = c.again(FTU + a), v = c.again(FTV + a);
         out.theta(a, u, v, rfma(k.ei, crP[a], rfma(rfma(-6.0, u, lu), k.idx2, rmul(k.nmt2, u))),
                   rfma(k.ei, ciP[a], rfma(rfma(-6.0, v, lv), k.idx2, rmul(k.nmt2, v))));
@@ -184,7 +262,7 @@ __device__ __forceinline__ void gauged_site(const V &c, const V &p, int fth, Gau
             s[a] = rfma(u[a], u[a], rmul(v[a], v[a]));
         }
         const double den = rfma(k.kappa, rmul(rmul(s[0], s[1]), s[2]), 1.0);
-        const double nV2 = -k.mu / rmul(den, den);   // -2 V'
+        const double nV2 = radd(-k.mu / rmul(den, den), nhh);   // -2 V' [- kappa_H H^2]
         out.moduli(s, den);
         double ec = 0.0;
 #pragma unroll
@@ -197,21 +275,17 @@ __device__ __forceinline__ void gauged_site(const V &c, const V &p, int fth, Gau
         if (SUMS) sums.ec = ec;
     }
     if (SUMS) { sums.eg = eg; sums.etg = etg; }
-    // staples (scp_sim.c:1214-1220): plaquette sines at x, and at x less the
-    // other direction of the plane
-    double pa[7] = {plaq_angle(c, p, fth, 0, 0, 0), plaq_angle(c, p, fth, 1, 0, 0), plaq_angle(c, p, fth, 2, 0, 0),
-                    plaq_angle(c, p, fth, 0, -1, 0), plaq_angle(c, p, fth, 1, -1, 0),
-                    plaq_angle(c, p, fth, 1, 0, -1), plaq_angle(c, p, fth, 2, 0, -1)};
-    out.angles(pa[0], pa[1], pa[2]);
-    sin_batch(pa);
-    const double st0 = rsub(rsub(pa[0], pa[3]), rsub(pa[2], pa[6]));
-    const double st1 = rsub(rsub(pa[1], pa[5]), rsub(pa[0], cy.p0));
-    const double st2 = rsub(rsub(pa[2], cy.p2), rsub(pa[1], pa[4]));
-    cy.p0 = pa[0];
-    cy.p2 = pa[2];
-    out.link(0, c.again(fth), rfma(k.stp, st0, rmul(k.gi, K[0])));
-    out.link(1, c.again(fth + 1), rfma(k.stp, st1, rmul(k.gi, K[1])));
-    out.link(2, c.again(fth + 2), rfma(k.stp, st2, rmul(k.gi, K[2])));
+    if constexpr (LINKS) {
+        double st[3], own[3];
+        staples(c, p, fth, cy.p0, cy.p2, st, own);
+        out.angles(own[0], own[1], own[2]);
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+            out.link(d, c.again(fth + d), rfma(k.stp, st[d], CHARGED ? out.current(d, K[d]) : rmul(k.gi, K[d])));
+    } else {
+#pragma unroll
+        for (int d = 0; d < 3; d++) out.current(d, K[d]);
+    }
 }
 
 }  // namespace scp

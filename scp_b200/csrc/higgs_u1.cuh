@@ -21,9 +21,14 @@
 // same order (matter, E, [E2], [dH/dt]).  One launch per step reads every
 // position of the resident planes through the ring, so each word moves once
 // per step.
+//
+// What bounds it: latency at eight warps per SM.  608 B per site; with both
+// extensions a warp issues some 2000 instructions per plane (two sets of link
+// phases, two gauges' staples), 0.61 of a plain copy's rate at 128^3: 321 us a
+// step against 614 with four resident planes, a sine and cosine of every
+// plaquette and the momenta loaded at their own plane.
 #pragma once
-#include "multiplet.cuh"
-#include "ring.cuh"
+#include "walk.cuh"
 
 namespace scp {
 
@@ -36,189 +41,168 @@ struct HuConsts {
     double g2, stp2, gad2, q[3];      // second gauge
     double hv, hlam, hkap;            // Higgs
     double damp_width, damp_rate;
+    double ei, cross, gi;             // eta/(2dx), eta dx/2, g/dx
 };
 
-template <bool HIGGS, bool G2>
+constexpr int kTh2Slot = 15;   // second gauge links, after matter and th
+
+template <class MODE, bool HIGGS, bool G2>
 struct HiggsU1 {
     static constexpr int TH = 12;                        // first gauge links
-    static constexpr int TH2 = 15;                       // second gauge links
+    static constexpr int TH2 = kTh2Slot;                      // second gauge links
     static constexpr int HF = G2 ? 18 : 15;              // the Higgs field
-    static constexpr int NR = 15 + (G2 ? 3 : 0) + (HIGGS ? 1 : 0);
+    static constexpr int NR = 15 + (G2 ? 3 : 0) + (HIGGS ? 1 : 0), NA = NR, CF = 12;
     static constexpr int MIN_CTAS = 1;
+    static constexpr bool HALO_APART = false;
 
     struct Args {
-        RingSrc<NR> src;      // positions x_{n+1}
+        const double *src[2];   // positions x_{n+1}, NR arrays
         int N;
         HuConsts c;
-        const double *win;    // momenta w_n (v_0 on the first launch), NR arrays
-        double *wout;         // w_{n+1} (may alias win)
-        double *xout;         // x_{n+2}
-        double *sout;         // v_{n+1} (synchronous launches)
-        int *flag;
-        int first, sync, damp;
+        LeapIO io;
     };
 
-    struct Carry {
-        double cm[G2 ? 3 : 1], sm[G2 ? 3 : 1];   // link phase along i at x - i (per component with G2)
-        double pm[2], pm2[2];                    // plaquette sines (0,1), (2,0) at x - i, both gauges
+    struct State {
+        GaugedCarry cy;
+        double p0, p2;          // plaquette sines of the second gauge at x - i
+        double hm;              // H at x - i
+        double w[NR];
     };
 
-    __device__ static void prefetch(const Args &A, long long idx) {
+    __device__ static __forceinline__ void load(const Args &A, State &st, long long idx) {
 #pragma unroll
-        for (int f = 0; f < NR; f++) prefetch_l2(A.win + f * A.c.N3 + idx);
+        for (int f = 0; f < NR; f++) st.w[f] = ld_early(LeapSite<MODE, NR>::at(A.io.win, f, A.c.N3) + idx);
     }
 
     template <class V>
-    __device__ static void site(const Args &A, const V &v, int i, int j, int k, long long idx, Carry &cy,
-                                bool first_plane) {
-        const HuConsts &c = A.c;
-        const long long N3 = c.N3;
-        // the matter momenta are loaded first, so their latency passes under
-        // the stencil instead of stalling the kicks
-        double wv[NR];
+    __device__ static __forceinline__ void begin(const Args &A, State &st, const V &m, const V &c) {
+        if constexpr (G2) {   // a phase per component: th + q_a th2
 #pragma unroll
-        for (int f = 0; f < NR; f++) wv[f] = A.win[f * N3 + idx];
-        double own[12];
+            for (int a = 0; a < 3; a++) {
+                double ph[1] = {rfma(A.c.q[a], m.get(TH2, 0, 0), m.get(TH, 0, 0))}, sn[1], cs[1];
+                sincos_batch<1, true>(ph, sn, cs);
 #pragma unroll
-        for (int f = 0; f < 12; f++) own[f] = v(f);
-        constexpr int NC = G2 ? 3 : 1;
-        if (first_plane) {   // the values carried from plane i-1, computed from the ring once
-#pragma unroll
-            for (int a = 0; a < NC; a++) {
-                const double ph = G2 ? v.at(TH, -1, 0, 0) + c.q[a] * v.at(TH2, -1, 0, 0) : v.at(TH, -1, 0, 0);
-                sincos_any(ph, &cy.sm[a], &cy.cm[a]);
-            }
-            cy.pm[0] = plaquette_sin(v, TH, 0, -1, 0, 0);
-            cy.pm[1] = plaquette_sin(v, TH, 2, -1, 0, 0);
-            if (G2) {
-                cy.pm2[0] = plaquette_sin(v, TH2, 0, -1, 0, 0);
-                cy.pm2[1] = plaquette_sin(v, TH2, 2, -1, 0, 0);
-            }
-        }
-        // link phases of direction d: forward at x, backward at x - d; the
-        // first gauge's own phase at x for the cross term
-        auto links = [&](int d, double cP[3], double sP[3], double cM[3], double sM[3], double &cW, double &sW) {
-            const double t1 = v(TH + d);
-            sincos_bounded(t1, &sW, &cW);
-            if (G2) {
-                const double t2 = v(TH2 + d);
-                const double t1m = nb(v, TH + d, d, -1), t2m = nb(v, TH2 + d, d, -1);
-                // components of equal charge share their phase (the default
-                // charges 1, 1, -2): the same angle, so the same cos / sin
-                const bool same10 = c.q[1] == c.q[0], same20 = c.q[2] == c.q[0], same21 = c.q[2] == c.q[1];
-#pragma unroll
-                for (int a = 0; a < 3; a++) {
-                    const int src = (a == 1 && same10) ? 0 : (a == 2 && same20) ? 0 : (a == 2 && same21) ? 1 : a;
-                    if (src == a) {
-                        sincos_any(t1 + c.q[a] * t2, &sP[a], &cP[a]);
-                        if (d != 0) sincos_any(t1m + c.q[a] * t2m, &sM[a], &cM[a]);
-                    } else if (src == 0) {
-                        sP[a] = sP[0]; cP[a] = cP[0];
-                        if (d != 0) { sM[a] = sM[0]; cM[a] = cM[0]; }
-                    } else {
-                        sP[a] = sP[1]; cP[a] = cP[1];
-                        if (d != 0) { sM[a] = sM[1]; cM[a] = cM[1]; }
-                    }
-                    if (d == 0) {
-                        cM[a] = cy.cm[a]; sM[a] = cy.sm[a];
-                        cy.cm[a] = cP[a]; cy.sm[a] = sP[a];
-                    }
+                for (int q = a; q < 6; q += 3) {
+                    const double u = m.get(field_re(q), 0, 0), v = m.get(field_im(q), 0, 0);
+                    st.cy.t[field_re(q)] = rfma(sn[0], v, rmul(cs[0], u));
+                    st.cy.t[field_im(q)] = rfma(-sn[0], u, rmul(cs[0], v));
                 }
-            } else {
-                double cm, sm;
-                if (d == 0) { cm = cy.cm[0]; sm = cy.sm[0]; cy.cm[0] = cW; cy.sm[0] = sW; }
-                else sincos_bounded(nb(v, TH + d, d, -1), &sm, &cm);
-#pragma unroll
-                for (int a = 0; a < 3; a++) { cP[a] = cW; sP[a] = sW; cM[a] = cm; sM[a] = sm; }
             }
-        };
-        MultipletOut o;
-        covariant_multiplet<G2>(v, 0, own, links, c.q, c.idx1, c.inva, c.eta, o);
+            staples_begin(m, c, TH, st.cy.p0, st.cy.p2);
+            staples_begin(m, c, TH2, st.p0, st.p2);
+        } else {
+            gauged_begin<false, true>(m, c, TH, st.cy);
+        }
+        if (HIGGS) st.hm = m.get(HF, 0, 0);
+    }
 
-        // potential: s_a = |Phi_a|^2, V'(s) = (mu/2)/(1 + kappa s)^2 with s = prod s_a
-        double sa[3];
-#pragma unroll
-        for (int a = 0; a < 3; a++) sa[a] = own[MU + a] * own[MU + a] + own[MV + a] * own[MV + a];
-        const double s = sa[0] * sa[1] * sa[2];
-        const double den = 1.0 + c.kappa * s;
-        const double Vp = 0.5 * c.mu / (den * den);
-        const double h = HIGGS ? v(HF) : 0.0;
-        const double hh = h * h;
-        double acc[12];
+    struct Out {
+        const Args &A;
+        LeapSite<MODE, NR> &leap;
+        double s;               // prod_a |Phi_a|^2
+        __device__ __forceinline__ void theta(int a, double u, double v, double au, double av) {
+            leap.put(FTU + a, u, au, leap.dmp);
+            leap.put(FTV + a, v, av, leap.dmp);
+        }
+        __device__ __forceinline__ void phi(int a, double u, double v, double au, double av) {
+            leap.put(FU + a, u, au, leap.dmp);
+            leap.put(FV + a, v, av, leap.dmp);
+        }
+        __device__ __forceinline__ void moduli(const double (&m)[3], double) { s = rmul(rmul(m[0], m[1]), m[2]); }
+        __device__ __forceinline__ void angles(double, double, double) {}
+        __device__ __forceinline__ double current(int, double K) { return K; }
+        __device__ __forceinline__ void link(int d, double th, double K) {
+            leap.put_link(TH + d, th, K, A.c.gad, leap.dmp);
+        }
+    };
+
+    // The force with the second gauge: the components have phases of their
+    // own, so a component's Phi and Theta go through their directions together
+    // (one set of phases live at a time, shared by components of equal charge)
+    // and every kick waits for the last of them.
+    template <class V>
+    __device__ static __forceinline__ void two_gauge_site(const Args &A, State &st, const V &c, const V &p, Out &out,
+                                                          double nhh) {
+        const HuConsts &h = A.c;
+        const GaugedConsts k(h);
+        double wang[3] = {c.get(TH, 0, 0), c.get(TH + 1, 0, 0), c.get(TH + 2, 0, 0)}, sw[3], cw[3];
+        sincos_batch(wang, sw, cw);
+        double K[3] = {0.0, 0.0, 0.0}, Kw[3] = {0.0, 0.0, 0.0};
+        double crP[3], ciP[3], crT[3], ciT[3], lap[12], none = 0.0;
+        double sn[5], cs[5];
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-            const double others = sa[(a + 1) % 3] * sa[(a + 2) % 3];
-            const double u = own[MU + a], w = own[MV + a], tu = own[MTU + a], tw = own[MTV + a];
-            double au = (o.lsum[MU + a] - 6.0 * u) * c.idx2 - c.m2 * u - 2.0 * Vp * u * others + c.eta * o.curlT[a];
-            double aw = (o.lsum[MV + a] - 6.0 * w) * c.idx2 - c.m2 * w - 2.0 * Vp * w * others + c.eta * o.curlT[3 + a];
-            if (HIGGS) {
-                au = au - c.hkap * hh * u * others;
-                aw = aw - c.hkap * hh * w * others;
-            }
-            acc[MU + a] = au;
-            acc[MV + a] = aw;
-            acc[MTU + a] = (o.lsum[MTU + a] - 6.0 * tu) * c.idx2 - c.mtheta2 * tu + c.eta * o.curlP[a];
-            acc[MTV + a] = (o.lsum[MTV + a] - 6.0 * tw) * c.idx2 - c.mtheta2 * tw + c.eta * o.curlP[3 + a];
-        }
-        double accH = 0.0;
-        if (HIGGS) {
-            const double lapH = (v.at(HF, 1, 0, 0) + v.at(HF, -1, 0, 0) + v.at(HF, 0, 1, 0) + v.at(HF, 0, -1, 0) +
-                                 v.at(HF, 0, 0, 1) + v.at(HF, 0, 0, -1) - 6.0 * h) * c.idx2;
-            accH = lapH - c.hlam * h * (h * h - c.hv * c.hv) - c.hkap * s * h;
-        }
-        // field kicks: plaquette terms plus currents
-        double st[3], pat[2], K[3];
-        staples(v, TH, cy.pm, st, pat);
-        cy.pm[0] = pat[0]; cy.pm[1] = pat[1];
+            if (a == 0 || h.q[a] != h.q[a - 1]) {
+                double ang[5];
 #pragma unroll
-        for (int d = 0; d < 3; d++) K[d] = c.stp * st[d] + c.g * o.jlat[d];
-        double K2[3] = {0.0, 0.0, 0.0};
-        if (G2) {
-            double st2[3];
-            staples(v, TH2, cy.pm2, st2, pat);
-            cy.pm2[0] = pat[0]; cy.pm2[1] = pat[1];
-#pragma unroll
-            for (int d = 0; d < 3; d++) K2[d] = c.stp2 * st2[d] + c.g2 * c.inva * o.jw[d];
-        }
-
-        // leapfrog (fused kick / sponge / kick / drift, see ring.cuh)
-        const Leap leap{c.hdt, c.dt, A.first != 0};
-        const double dmp = (A.damp && !A.first) ? sponge_at(i, j, k, c.L, c.dx, c.damp_width, c.damp_rate) : 1.0;
-        bool bad = false;
-        auto put = [&](int f, double x, double vv, double wn) {
-            st_cs(A.xout + f * N3 + idx, x);
-            A.wout[f * N3 + idx] = wn;
-            if (A.sync) {
-                st_cs(A.sout + f * N3 + idx, vv);
-                bad |= !isfinite(x) || !isfinite(vv);
+                for (int n = 0; n < 5; n++) {
+                    const int d = n < 3 ? n : n - 2, dj = n == 3 ? -1 : 0, dk = n == 4 ? -1 : 0;
+                    ang[n] = rfma(h.q[a], c.get(TH2 + d, dj, dk), c.get(TH + d, dj, dk));
+                }
+                sincos_batch<5, true>(ang, sn, cs);
             }
+            const TwoGauge g2{cw, sw, h.q[a], Kw};
+            transport_field<false, true>(c, p, a, cs, sn, st.cy.t, K, k.r, crP, ciP, lap[FU + a], lap[FV + a], none, g2);
+            transport_field<false, true>(c, p, 3 + a, cs, sn, st.cy.t, K, k.r, crT, ciT, lap[FTU + a], lap[FTV + a],
+                                         none, g2);
+        }
+        double s[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const double u = c.again(FU + a), v = c.again(FV + a);
+            s[a] = rfma(u, u, rmul(v, v));
+        }
+        const double den = rfma(k.kappa, rmul(rmul(s[0], s[1]), s[2]), 1.0);
+        const double nV2 = radd(-k.mu / rmul(den, den), nhh);
+        out.moduli(s, den);
+        auto acc = [&](double x, double l, double t, double cu) {
+            return rfma(k.ei, cu, rfma(rfma(-6.0, x, l), k.idx2, rmul(t, x)));
         };
 #pragma unroll
-        for (int f = 0; f < 12; f++) {
-            double vv, wn;
-            leap(wv[f], acc[f], dmp, &vv, &wn);
-            put(f, own[f] + c.dt * wn, vv, wn);
+        for (int a = 0; a < 3; a++) {
+            const double t = rfma(nV2, rmul(s[(a + 1) % 3], s[(a + 2) % 3]), k.nm2);
+            const double u = c.again(FU + a), v = c.again(FV + a);
+            out.phi(a, u, v, acc(u, lap[FU + a], t, crT[a]), acc(v, lap[FV + a], t, ciT[a]));
+            const double tu = c.again(FTU + a), tv = c.again(FTV + a);
+            out.theta(a, tu, tv, acc(tu, lap[FTU + a], k.nmt2, crP[a]), acc(tv, lap[FTV + a], k.nmt2, ciP[a]));
         }
+        double stp[3], own[3];
+        staples(c, p, TH, st.cy.p0, st.cy.p2, stp, own);
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-            double E, Eh;
-            leap(wv[TH + d], K[d], dmp, &E, &Eh);
-            put(TH + d, wrap_angle(v(TH + d) + c.gad * Eh), E, Eh);
-        }
-        if (G2) {
+        for (int d = 0; d < 3; d++) out.link(d, c.again(TH + d), rfma(k.stp, stp[d], rmul(k.gi, K[d])));
+        staples(c, p, TH2, st.p0, st.p2, stp, own);
+        const double g2i = rmul(h.g2, h.inva);
 #pragma unroll
-            for (int d = 0; d < 3; d++) {
-                double E2, E2h;
-                leap(wv[TH2 + d], K2[d], 1.0, &E2, &E2h);
-                put(TH2 + d, wrap_angle(v(TH2 + d) + c.gad2 * E2h), E2, E2h);
-            }
+        for (int d = 0; d < 3; d++)   // E2 is not damped by the sponge
+            out.leap.put_link(TH2 + d, c.again(TH2 + d), rfma(h.stp2, stp[d], rmul(g2i, Kw[d])), h.gad2, 1.0);
+    }
+
+    template <class V>
+    __device__ static __forceinline__ void site(const Args &A, State &st, const V &c, const V &p, int i, int j, int k,
+                                                long long idx, long long next) {
+        const HuConsts &h = A.c;
+        const double dmp = (MODE::DAMP && !MODE::FIRST)
+                               ? sponge_factor(i, j, k, h.L, h.dx, h.damp_width, h.damp_rate) : 1.0;
+        LeapSite<MODE, NR> leap{A.io, st.w, h.N3, idx, next, h.hdt, h.dt, dmp};
+        Out out{A, leap, 0.0};
+        const double H = HIGGS ? c.get(HF, 0, 0) : 0.0;
+        const double nhh = HIGGS ? rmul(-h.hkap, rmul(H, H)) : 0.0;
+        if constexpr (G2) {
+            two_gauge_site(A, st, c, p, out, nhh);
+        } else {
+            GaugedSums none;
+            gauged_site<false, false, true>(c, p, TH, st.cy, GaugedConsts(h), out, none, 1.0, nhh);
         }
-        if (HIGGS) {
-            double hd, hdh;
-            leap(wv[HF], accH, 1.0, &hd, &hdh);
-            put(HF, h + c.dt * hdh, hd, hdh);
+        if (HIGGS) {   // lap H - lambda H (H^2 - v^2) - kappa_H s H, not damped
+            double l = radd(p.get(HF, 0, 0), st.hm);
+            l = radd(radd(l, c.get(HF, 1, 0)), c.get(HF, -1, 0));
+            l = radd(radd(l, c.get(HF, 0, 1)), c.get(HF, 0, -1));
+            st.hm = H;
+            const double v2 = rfma(H, H, rmul(-h.hv, h.hv));
+            const double t = rfma(-h.hlam, v2, rmul(-h.hkap, out.s));
+            leap.put(HF, H, rfma(rfma(-6.0, H, l), h.idx2, rmul(t, H)), 1.0);
         }
-        if (A.sync && bad) atomicOr(A.flag, 1);
+        if (MODE::SYNC && leap.bad) atomicOr(A.io.flag, 1);
     }
 };
 

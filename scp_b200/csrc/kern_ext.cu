@@ -1,11 +1,9 @@
-// kern_ext.cu -- instantiations and launchers of the extension steppers'
-// ring kernels (Higgs condensate / second gauge, three fabrics).
+// kern_ext.cu -- instantiations and launchers of the plane-ring kernels: the
+// real mode's optional terms and the FP64 diagnostics.
 #include <stdlib.h>
 
 #include "diag_ring.cuh"
 #include "ext_launch.cuh"
-#include "fabrics.cuh"
-#include "higgs_u1.cuh"
 #include "real6.cuh"
 
 namespace scp {
@@ -48,101 +46,7 @@ int ring_plan(int N, int nsm, ExtPlan *p) {
     return 0;
 }
 
-template <bool H, bool G>
-cudaError_t hu_launch(const ExtPlan &p, const HuConsts &c, const HuIO &io, cudaStream_t st) {
-    using M = HiggsU1<H, G>;
-    typename M::Args a;
-    const long long n3 = c.N3;
-    for (int f = 0; f < M::NR; f++) a.src.f[f] = io.x + f * n3;
-    a.src.prefetch = ring_prefetch();
-    a.N = c.N;
-    a.c = c;
-    a.win = io.win;
-    a.wout = io.wout;
-    a.xout = io.xout;
-    a.sout = io.sout;
-    a.flag = io.flag;
-    a.first = io.first;
-    a.sync = io.sync;
-    a.damp = io.damp;
-    ring_kernel<M, TileOf<M>::TX, TileOf<M>::TY><<<p.grid, TileOf<M>::NT, p.smem, st>>>(a, p.tg);
-    return cudaGetLastError();
-}
-
 }  // namespace
-
-int hu_plan(bool higgs, bool g2, int N, int nsm, ExtPlan *plan) {
-    if (higgs && g2) return ring_plan<HiggsU1<true, true>>(N, nsm, plan);
-    if (higgs) return ring_plan<HiggsU1<true, false>>(N, nsm, plan);
-    return ring_plan<HiggsU1<false, true>>(N, nsm, plan);
-}
-
-cudaError_t hu_step(bool higgs, bool g2, const ExtPlan &plan, const HuConsts &c, const HuIO &io, cudaStream_t st) {
-    if (higgs && g2) return hu_launch<true, true>(plan, c, io, st);
-    if (higgs) return hu_launch<true, false>(plan, c, io, st);
-    return hu_launch<false, true>(plan, c, io, st);
-}
-
-int fabric_plan(int N, int nsm, ExtPlan *fabric, ExtPlan *second, ExtPlan *link) {
-    if (ring_plan<FabricPass<false>>(N, nsm, fabric)) return -1;
-    if (ring_plan<FabricPass<true>>(N, nsm, second)) return -1;
-    return ring_plan<LinkPass>(N, nsm, link);
-}
-
-namespace {
-template <bool SECOND>
-cudaError_t fabric_launch(const ExtPlan &p, const FabConsts &c, const FabIO &io, cudaStream_t st) {
-    using M = FabricPass<SECOND>;
-    typename M::Args a;
-    const long long n3 = c.N3;
-    for (int f = 0; f < 12; f++) a.src.f[f] = io.x + f * n3;
-    for (int d = 0; d < 3; d++) a.src.f[M::TH + d] = io.th + d * n3;
-    a.src.prefetch = ring_prefetch();
-    a.N = c.N;
-    a.c = c;
-    a.qf = io.qf;
-    a.gqf = io.gqf;
-    a.qx = io.qx;
-    a.gqx = io.gqx;
-    a.win = io.win;
-    a.wout = io.wout;
-    a.xout = io.xout;
-    a.sout = io.sout;
-    a.kacc = io.kacc;
-    a.flag = io.flag;
-    a.first = io.first;
-    a.sync = io.sync;
-    a.damp = io.damp;
-    a.accumulate = io.accumulate;
-    ring_kernel<M, TileOf<M>::TX, TileOf<M>::TY><<<p.grid, TileOf<M>::NT, p.smem, st>>>(a, p.tg);
-    return cudaGetLastError();
-}
-}  // namespace
-
-cudaError_t fabric_step(const ExtPlan &plan, const FabConsts &c, const FabIO &io, cudaStream_t st) {
-    return io.second ? fabric_launch<true>(plan, c, io, st) : fabric_launch<false>(plan, c, io, st);
-}
-
-cudaError_t link_step(const ExtPlan &p, const FabConsts &c, const LinkIO &io, cudaStream_t st) {
-    LinkPass::Args a;
-    const long long n3 = c.N3;
-    for (int d = 0; d < 3; d++) a.src.f[d] = io.th + d * n3;
-    a.src.prefetch = ring_prefetch();
-    a.N = c.N;
-    a.c = c;
-    a.kacc = io.kacc;
-    a.win = io.win;
-    a.wout = io.wout;
-    a.xout = io.thout;
-    a.sout = io.sout;
-    a.flag = io.flag;
-    a.first = io.first;
-    a.sync = io.sync;
-    a.damp = io.damp;
-    using T = TileOf<LinkPass>;
-    ring_kernel<LinkPass, T::TX, T::TY><<<p.grid, T::NT, p.smem, st>>>(a, p.tg);
-    return cudaGetLastError();
-}
 
 namespace {
 template <bool G>

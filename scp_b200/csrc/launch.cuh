@@ -69,27 +69,20 @@ inline MultiFn<F32C> multi_fn<F32C>(int shape, bool g, bool d, size_t *smem) { r
         return d ? KERNEL<__VA_ARGS__, false, true> : KERNEL<__VA_ARGS__, false, false>;            \
     } while (0)
 
-// Instantiation helpers for the kern_*.cu units.
-#define SCP_PICK16(KERNEL, ...)                                                                        \
-    do {                                                                                               \
-        if (g) {                                                                                       \
-            if (f) {                                                                                   \
-                if (s) return d ? KERNEL<__VA_ARGS__, true, true, true, true>                           \
-                                : KERNEL<__VA_ARGS__, true, true, true, false>;                         \
-                return d ? KERNEL<__VA_ARGS__, true, true, false, true>                                 \
-                         : KERNEL<__VA_ARGS__, true, true, false, false>;                               \
-            }                                                                                          \
-            if (s) return d ? KERNEL<__VA_ARGS__, true, false, true, true>                              \
-                            : KERNEL<__VA_ARGS__, true, false, true, false>;                            \
+// Instantiation helper for the kern_*.cu units: <GAUGED, FIRST, SYNC, DAMP>.  A
+// first launch takes no closing kick, damps nothing and stores no synchronous
+// momenta, so it has one form.
+#define SCP_PICK16(KERNEL, ...)                                                                         \
+    do {                                                                                                \
+        if (f) return g ? KERNEL<__VA_ARGS__, true, true, false, false>                                  \
+                        : KERNEL<__VA_ARGS__, false, true, false, false>;                                \
+        if (g) {                                                                                        \
+            if (s) return d ? KERNEL<__VA_ARGS__, true, false, true, true>                               \
+                            : KERNEL<__VA_ARGS__, true, false, true, false>;                             \
             return d ? KERNEL<__VA_ARGS__, true, false, false, true> : KERNEL<__VA_ARGS__, true, false, false, false>; \
-        }                                                                                              \
-        if (f) {                                                                                       \
-            if (s) return d ? KERNEL<__VA_ARGS__, false, true, true, true>                              \
-                            : KERNEL<__VA_ARGS__, false, true, true, false>;                            \
-            return d ? KERNEL<__VA_ARGS__, false, true, false, true> : KERNEL<__VA_ARGS__, false, true, false, false>; \
-        }                                                                                              \
-        if (s) return d ? KERNEL<__VA_ARGS__, false, false, true, true>                                 \
-                        : KERNEL<__VA_ARGS__, false, false, true, false>;                               \
+        }                                                                                               \
+        if (s) return d ? KERNEL<__VA_ARGS__, false, false, true, true>                                  \
+                        : KERNEL<__VA_ARGS__, false, false, true, false>;                                \
         return d ? KERNEL<__VA_ARGS__, false, false, false, true> : KERNEL<__VA_ARGS__, false, false, false, false>; \
     } while (0)
 

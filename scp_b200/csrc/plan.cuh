@@ -1,0 +1,59 @@
+// plan.cuh -- host-side work plans of the plane-ring steppers: the tile shape
+// that suits a grid edge, and its cut into work items.
+#pragma once
+#include "common.cuh"
+
+namespace scp {
+
+// Cut a grid of edge N into tiles of tw x th sites and segments along i, for
+// `slots` resident CTAs: the segment length minimises (waves x planes per
+// item), planes per item counting the two halo planes a segment re-reads.
+// All CTAs start their items on the same plane and walk i in step, so
+// neighbouring columns read each other's halo rows while they are in L2.
+// (Equal shares of all (column, plane) pairs, which leave no slot idle, were
+// measured slower: neighbours drift apart in i and the halo rows come from
+// DRAM again, 837 against 470 MB read per 128^3 step.)
+inline void plan_tiles(int N, int tw, int th, int slots, TileGrid *out, int *grid) {
+    TileGrid tg;
+    tg.tw = tw;
+    tg.th = th;
+    tg.ntx = (N + tw - 1) / tw;
+    tg.nty = (N + th - 1) / th;
+    const int ntiles = tg.ntx * tg.nty;
+    double best = 1e300;
+    int best_nseg = 1;
+    for (int ns = 1; ns <= N; ns++) {
+        const int seg = (N + ns - 1) / ns;
+        if (ns > 1 && (N + seg - 1) / seg != ns) continue;   // the same cut as a smaller ns
+        const long long waves = ((long long)ntiles * ns + slots - 1) / slots;
+        const double cost = (double)waves * (seg + 2);
+        if (cost < best - 1e-9) { best = cost; best_nseg = ns; }
+    }
+    tg.seg = (N + best_nseg - 1) / best_nseg;
+    tg.nseg = (N + tg.seg - 1) / tg.seg;
+    tg.nitems = ntiles * tg.nseg;
+    *out = tg;
+    *grid = tg.nitems < slots ? tg.nitems : slots;
+}
+
+// Tile of the one-site cp.async kernels for a grid of edge N: up to nt sites
+// whose staged rows (halo included) fit `area` ring elements, least
+// (padded sites) x (cost of the width).  Rows of 32 sites move whole 128-byte
+// lines: width 32 costs 1.  Gauged FP64 measured against it: 16-site rows
+// 192 against 184 us at 128^3 (counted 1.08), rows that start inside a line
+// 362 against 320 us at 150^3 with 7 % fewer padded sites (1.22; 1.12 where an
+// odd N leaves every row unaligned anyway).  So 32-site rows stay except where
+// they pad: 16 x 16 takes 54 us at 80^3 against 62, 25 x 10 takes 107 us at
+// 97^3 (whose fourth column of 32-site tiles holds one site) against 123.
+inline void fit_tile(int N, int nt, int area, int *tw, int *th) {
+    double best = 1e300;
+    for (int w = 32; w >= 16; w--) {
+        int h = nt / w;
+        while (h > 1 && (w + 2) * (h + 2) > area) h--;
+        const double pad = (double)((N + w - 1) / w) * w * ((N + h - 1) / h) * h;
+        const double cost = pad * (w == 32 ? 1.0 : w == 16 ? 1.08 : (N & 1) ? 1.12 : 1.22);
+        if (cost < best - 1e-9) { best = cost; *tw = w; *th = h; }
+    }
+}
+
+}  // namespace scp

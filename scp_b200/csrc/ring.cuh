@@ -23,6 +23,7 @@
 // and runs as ring_kernel<Model, TX, TY>.
 #pragma once
 #include "common.cuh"
+#include "trig.cuh"
 
 namespace scp {
 
@@ -56,6 +57,12 @@ struct RingView {
     }
     __device__ __forceinline__ double operator()(int f) const { return c[f * S::FIELD]; }
 };
+
+// field f at offset s along direction d (0: i, 1: j, 2: k)
+template <class V>
+__device__ __forceinline__ double nb(const V &v, int f, int d, int s) {
+    return v.at(f, d == 0 ? s : 0, d == 1 ? s : 0, d == 2 ? s : 0);
+}
 
 // One work item of model M; extra arguments (a reduction's per-thread sums)
 // are passed on to M::site.

@@ -23,6 +23,7 @@
 #include "snapshot.cuh"
 #include "spectral.cuh"
 #include "launch.cuh"
+#include "plan.cuh"
 #include "tma.cuh"
 #include "ext_launch.cuh"
 #include "ext_startup.cuh"
@@ -119,13 +120,13 @@ struct scp_gpu {
     // fused ring kernel per step (higgs_u1.cuh); X[0..1], W and S hold nx arrays
     int gx = 0, g2 = 0, higgs = 0;
     HuConsts hc{};
-    // three fabrics C, Q, L: one ring kernel per fabric and one for the links
-    // per step (fabrics.cuh); X[0..1], W and S hold C (15), L (12), Q (12, free)
+    // three fabrics C, Q, L: one walker launch per fabric and step, the last
+    // one with the links (fabrics.cuh); X[0..1], W and S hold C (15), L (12), Q (12, free)
     int mfab = 0, fab_lock = 0;
     double qfab[3] = {0.0, 0.0, 0.0};
     FabConsts fc{};
     double *kacc = nullptr;      // accumulated currents (3 arrays)
-    ExtPlan xplan{}, xplan2{}, lplan{};
+    ExtPlan xplan{}, xplan2{};
     ExtPlan dplan{};             // first diagnostics reduction on the plane ring (FP64 states)
     int dplan_ok = 0;
     int nx = 0;                  // position arrays per buffer of the extension layouts
@@ -245,57 +246,6 @@ static void fill_consts(scp_gpu *h) {
 
 static bool damping_on(const scp_gpu *h) {
     return h->p.bc_type == 0 && h->p.damp_width > 0 && h->p.damp_rate > 0;
-}
-
-// Cut a grid of edge N into tiles of tw x th sites and segments along i, for
-// `slots` resident CTAs: the segment length minimises (waves x planes per
-// item), planes per item counting the two halo planes a segment re-reads.
-// All CTAs start their items on the same plane and walk i in step, so
-// neighbouring columns read each other's halo rows while they are in L2.
-// (Equal shares of all (column, plane) pairs, which leave no slot idle, were
-// measured slower: neighbours drift apart in i and the halo rows come from
-// DRAM again, 837 against 470 MB read per 128^3 step.)
-static void plan_tiles(int N, int tw, int th, int slots, TileGrid *out, int *grid) {
-    TileGrid tg;
-    tg.tw = tw;
-    tg.th = th;
-    tg.ntx = (N + tw - 1) / tw;
-    tg.nty = (N + th - 1) / th;
-    const int ntiles = tg.ntx * tg.nty;
-    double best = 1e300;
-    int best_nseg = 1;
-    for (int ns = 1; ns <= N; ns++) {
-        const int seg = (N + ns - 1) / ns;
-        if (ns > 1 && (N + seg - 1) / seg != ns) continue;   // the same cut as a smaller ns
-        const long long waves = ((long long)ntiles * ns + slots - 1) / slots;
-        const double cost = (double)waves * (seg + 2);
-        if (cost < best - 1e-9) { best = cost; best_nseg = ns; }
-    }
-    tg.seg = (N + best_nseg - 1) / best_nseg;
-    tg.nseg = (N + tg.seg - 1) / tg.seg;
-    tg.nitems = ntiles * tg.nseg;
-    *out = tg;
-    *grid = tg.nitems < slots ? tg.nitems : slots;
-}
-
-// Tile of the one-site cp.async kernels for a grid of edge N: up to nt sites
-// whose staged rows (halo included) fit `area` ring elements, least
-// (padded sites) x (cost of the width).  Rows of 32 sites move whole 128-byte
-// lines: width 32 costs 1.  Gauged FP64 measured against it: 16-site rows
-// 192 against 184 us at 128^3 (counted 1.08), rows that start inside a line
-// 362 against 320 us at 150^3 with 7 % fewer padded sites (1.22; 1.12 where an
-// odd N leaves every row unaligned anyway).  So 32-site rows stay except where
-// they pad: 16 x 16 takes 54 us at 80^3 against 62, 25 x 10 takes 107 us at
-// 97^3 (whose fourth column of 32-site tiles holds one site) against 123.
-static void fit_tile(int N, int nt, int area, int *tw, int *th) {
-    double best = 1e300;
-    for (int w = 32; w >= 16; w--) {
-        int h = nt / w;
-        while (h > 1 && (w + 2) * (h + 2) > area) h--;
-        const double pad = (double)((N + w - 1) / w) * w * ((N + h - 1) / h) * h;
-        const double cost = pad * (w == 32 ? 1.0 : w == 16 ? 1.08 : (N & 1) ? 1.12 : 1.22);
-        if (cost < best - 1e-9) { best = cost; *tw = w; *th = h; }
-    }
 }
 
 template <class P>
@@ -672,7 +622,7 @@ static int gauss2_startup(scp_gpu *h) {
     double *tmp = nullptr;
     CK(cudaMallocAsync(&tmp, sizeof(double) * 5 * n3, h->stream));
     double *b = tmp, *x = tmp + n3, *r = tmp + 2 * n3, *p = tmp + 3 * n3, *Ap = tmp + 4 * n3;
-    double *E2 = h->S + (size_t)HiggsU1<false, true>::TH2 * n3;
+    double *E2 = h->S + (size_t)kTh2Slot * n3;
     hu_gauss2_rhs_kernel<<<nb, kRedThreads, 0, h->stream>>>(h->X[0], h->S, E2, h->hc, b, h->part);
     int iters = 0, rc;
     if ((rc = cg_solve(h, nb, b, x, r, p, Ap, &iters))) {
@@ -968,6 +918,9 @@ static int init_gext(scp_gpu *h, const double *const *cols, bool on_device) {
     k.stp2 = h->g2 ? 1.0 / (p.g_gauge2 * p.dx * p.dx * p.dx) : 0.0;
     k.gad2 = -p.g_gauge2 * p.dx * p.dt;
     for (int a = 0; a < 3; a++) k.q[a] = p.gauge2_q[a];
+    k.ei = k.eta * k.idx1;
+    k.cross = 0.5 * k.eta * k.dx;
+    k.gi = k.g * k.inva;
     k.hv = p.higgs_v; k.hlam = p.higgs_lam; k.hkap = p.higgs_kap;
     k.damp_width = p.damp_width; k.damp_rate = p.damp_rate;
     int nsm = 0;
@@ -1025,57 +978,50 @@ static FabView fab_view(const scp_gpu *h, const double *X, const double *P) {
 }
 
 // one step of the three-fabric stepper: C (with the locked Q's force and
-// currents), Q when free, L, then the links
+// currents), Q when free, then L with the links
 static int fab_launch_step(scp_gpu *h, bool first, bool sync) {
     const size_t n3 = h->N3;
     const double *X = h->X[h->cur];
     double *Xo = h->X[h->cur ^ 1];
     const double *Win = first ? h->S : h->W;
     const double g = h->p.g_gauge;
-    auto fabric = [&](size_t slot, double qf, bool second, double qx, bool acc) -> int {
+    // the accumulator starts with the first fabric's current; the last fabric
+    // (L) steps the links with the sum
+    auto fabric = [&](size_t slot, double qf, bool second, double qx) -> int {
         FabIO io;
-        io.x = X + slot * n3;
-        io.th = X + (size_t)FTH * n3;
-        io.xout = Xo + slot * n3;
-        io.win = Win + slot * n3;
-        io.wout = h->W + slot * n3;
-        io.sout = h->S + slot * n3;
+        const size_t at[2] = {slot * n3, (size_t)FTH * n3};
+        for (int b = 0; b < 2; b++) {
+            io.src[b] = X + at[b];
+            io.xout[b] = Xo + at[b];
+            io.win[b] = Win + at[b];
+            io.wout[b] = h->W + at[b];
+            io.sout[b] = h->S + at[b];
+        }
         io.kacc = h->kacc;
         io.flag = h->flag;
         io.qf = qf;
-        io.gqf = g * qf;
+        io.gqf = g * qf * h->fc.inva;
         io.qx = qx;
-        io.gqx = g * qx;
+        io.gqx = g * qx * h->fc.inva;
         io.first = first;
         io.sync = sync;
         io.damp = damping_on(h);
-        io.accumulate = acc;
+        io.accumulate = slot != 0;
         io.second = second;
-        CK(fabric_step(second ? h->xplan2 : h->xplan, h->fc, io, h->stream));
+        io.links = slot == (size_t)kFabL;
+        CK(fabric_step(h->xplan, h->fc, io, h->stream));
         return SCP_OK;
     };
     int rc;
     const double qC = h->qfab[0], qQ = h->qfab[1], qL = h->qfab[2];
     if (h->fab_lock) {
-        // C moves under the q_Q force; its q_C current precedes the q_Q one (none when q_C = 0)
-        if ((rc = fabric(0, qQ, qC != 0.0, qC, false))) return rc;
+        // C moves under the q_Q force; its q_C current joins the q_Q one (none when q_C = 0)
+        if ((rc = fabric(0, qQ, qC != 0.0, qC))) return rc;
     } else {
-        if ((rc = fabric(0, qC, false, 0.0, false))) return rc;
-        if ((rc = fabric(kFabQ, qQ, false, 0.0, true))) return rc;
+        if ((rc = fabric(0, qC, false, 0.0))) return rc;
+        if ((rc = fabric(kFabQ, qQ, false, 0.0))) return rc;
     }
-    if ((rc = fabric(kFabL, qL, false, 0.0, true))) return rc;
-    LinkIO io;
-    io.th = X + (size_t)FTH * n3;
-    io.thout = Xo + (size_t)FTH * n3;
-    io.kacc = h->kacc;
-    io.win = Win + (size_t)FTH * n3;
-    io.wout = h->W + (size_t)FTH * n3;
-    io.sout = h->S + (size_t)FTH * n3;
-    io.flag = h->flag;
-    io.first = first;
-    io.sync = sync;
-    io.damp = damping_on(h);
-    CK(link_step(h->lplan, h->fc, io, h->stream));
+    if ((rc = fabric(kFabL, qL, false, 0.0))) return rc;
     h->cur ^= 1;
     return SCP_OK;
 }
@@ -1144,10 +1090,13 @@ static int init_mf(scp_gpu *h, const double *const *cols, bool on_device) {
     k.g = p.g_gauge;
     k.stp = 1.0 / (p.g_gauge * p.dx * p.dx * p.dx);
     k.gad = -p.g_gauge * p.dx * p.dt;
+    k.ei = k.eta * k.idx1;
+    k.cross = 0.5 * k.eta * k.dx;
+    k.gi = k.g * k.inva;
     k.damp_width = p.damp_width; k.damp_rate = p.damp_rate;
     int nsm = 0;
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
-    if (fabric_plan(h->N, nsm, &h->xplan, &h->xplan2, &h->lplan)) return SCP_EUNSUPPORTED;
+    if (fabric_plan(h->N, nsm, &h->xplan)) return SCP_EUNSUPPORTED;
     if ((rc = mf_gauss_startup(h))) return rc;
     return fab_launch_step(h, true, false);
 }

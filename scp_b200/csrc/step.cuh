@@ -107,14 +107,6 @@ struct StepLayout {
 __device__ __forceinline__ void cp_async_elem(double *s, const double *g) { cp_async8(s, g); }
 __device__ __forceinline__ void cp_async_elem(float *s, const float *g) { cp_async4(s, g); }
 
-// A load that stays where it is written: the compiler does not move it down to
-// its first use, so its latency passes under what follows.
-__device__ __forceinline__ double ld_early(const double *p) {
-    double v;
-    asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
-}
-
 __device__ __forceinline__ double ldg_t(const double *p) { return __ldg(p); }
 __device__ __forceinline__ float ldg_t(const float *p) { return __ldg(p); }
 
@@ -129,13 +121,6 @@ __device__ __forceinline__ void two_sum(float a, float b, float *s, float *e) {
     const float bb = t - a;
     *e = (a - (t - bb)) + (b - bb);
     *s = t;
-}
-
-// link wrap into (-pi, pi] (reference: v - 2*pi*rint(v/(2*pi)), scp_sim.c:1647);
-// |v| < 3 never wraps, so the division only runs for the rare large angles
-__device__ __forceinline__ double link_wrap(double v) {
-    if (fabs(v) < 3.0) return v;
-    return wrap_angle(v);
 }
 
 // Plane staging of the classic ring: every thread copies its own site with
@@ -310,7 +295,9 @@ struct SiteUpdate {
     const int mslot;       // momentum slot of the staging (Stage::MOM)
     const bool SYNC, DAMP;
     Momenta<GAUGED> &w;
-    const long long next;   // elements to the next plane's site, 0 on a segment's last plane
+    const long long next;   // elements to the next plane's site, 0 on a segment's last plane (what is then
+                            // read is not used; a load behind a branch would be copied, and waited
+                            // for, where the branch joins)
     double dmp = 1.0;
     bool bad = false;
     double rho = 0.0, rho2 = 0.0;   // charge density and sum of |Phi_a|^2 of the site (DIAG)
@@ -322,7 +309,7 @@ struct SiteUpdate {
     // the momentum of the next plane, once this plane's is used
     __device__ __forceinline__ void ahead(int f) const {
         if constexpr (!Stage::MOM)
-            if (next) w.v[f] = ld_early(io.win + f * c.N3 + site + next);
+            w.v[f] = ld_early(io.win + f * c.N3 + site + next);
     }
     __device__ __forceinline__ double kick(double w, double a, double *wn) const {
         double v = FIRST ? w : rfma(c.hdt, a, w);
@@ -381,6 +368,7 @@ struct SiteUpdate {
             sums->s[SS_BB] += 2.0 * (h[0] * h[0] + h[1] * h[1] + h[2] * h[2]);
         }
     }
+    __device__ __forceinline__ double current(int, double K) const { return K; }   // charged links only
     __device__ __forceinline__ void link(int d, double th0, double K) {
         double Eh;
         const double E = kick(mom(FTH + d), K, &Eh);
@@ -503,7 +491,7 @@ __device__ __forceinline__ void step_item(const StepIO<F64> &io, const StepConst
     double xm[12];
     if (act) {
         if constexpr (GAUGED) {
-            gauged_begin(stg.view(0), stg.view(1), FTH, cy);
+            gauged_begin<false, true>(stg.view(0), stg.view(1), FTH, cy);
         } else {
             const auto m = stg.view(0);
 #pragma unroll
@@ -531,18 +519,9 @@ __device__ __forceinline__ void step_item(const StepIO<F64> &io, const StepConst
         }
         SiteUpdate<GAUGED, FIRST, DIAG, Stage> out{io, c, stg, sums, site, (i - i0) & 1, SYNC, DAMP, w,
                                                     i + 1 < i1 ? (long long)N * N : 0};
-        if (DAMP && !FIRST) {
-            const double x = -c.L + i * c.dx, y = -c.L + j * c.dx, z = -c.L + k * c.dx;
-            const double r = sqrt(x * x + y * y + z * z);
-            const double Rd = c.L - c.damp_width;
-            if (r > Rd) {
-                double sc2 = (r - Rd) / c.damp_width;
-                if (sc2 > 1) sc2 = 1;
-                out.dmp = 1.0 - c.damp_rate * sc2 * sc2;
-            }
-        }
+        if (DAMP && !FIRST) out.dmp = sponge_factor(i, j, k, c.L, c.dx, c.damp_width, c.damp_rate);
         GaugedSums gs;
-        if constexpr (GAUGED) gauged_site<DIAG>(stg.view(sc), stg.view(sp), FTH, cy, GaugedConsts(c), out, gs);
+        if constexpr (GAUGED) gauged_site<DIAG, false, true>(stg.view(sc), stg.view(sp), FTH, cy, GaugedConsts(c), out, gs);
         else free_site<DIAG>(stg.view(sc), stg.view(sp), xm, c, out, gs);
         if (SYNC && out.bad) atomicOr(io.flag, 1);
         if constexpr (DIAG) {

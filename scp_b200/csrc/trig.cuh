@@ -123,8 +123,9 @@ __device__ __forceinline__ double flip_sign(double x, unsigned bit) {   // bit: 
 }
 constexpr double kRintMagic = 6755399441055744.0;   // 1.5 * 2^52: adding it rounds to an integer
 
-// sines and cosines of n angles, |a| < 2^20
-template <int n>
+// sines and cosines of n angles, |a| < 2^20 (ANY: of any size, CUDA's sin and
+// cos beyond 2^19, where the quadrant would leave the low word)
+template <int n, bool ANY = false>
 __device__ __forceinline__ void sincos_batch(const double (&ang)[n], double (&sn)[n], double (&cs)[n]) {
     double r[n];
     unsigned q[n], big = 0;
@@ -168,6 +169,10 @@ __device__ __forceinline__ void sincos_batch(const double (&ang)[n], double (&sn
             const double c1 = (q[i] & 1) ? -sn[i] : cs[i];
             sn[i] = flip_sign(s1, q[i] >> 1);
             cs[i] = flip_sign(c1, q[i] >> 1);
+            if (ANY && abs_hi(ang[i]) >= 0x41200000u) {   // 2^19
+                sn[i] = sin(ang[i]);
+                cs[i] = cos(ang[i]);
+            }
         }
     }
 }
