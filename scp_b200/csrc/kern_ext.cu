@@ -1,7 +1,5 @@
 // kern_ext.cu -- instantiations and launchers of the plane-ring kernels: the
 // real mode's optional terms and the FP64 diagnostics.
-#include <stdlib.h>
-
 #include "diag_ring.cuh"
 #include "ext_launch.cuh"
 #include "real6.cuh"
@@ -9,16 +7,6 @@
 namespace scp {
 
 namespace {
-
-// L2 prefetch of the next plane's momenta in the ring kernels: on unless
-// SCP_RING_PREFETCH=0 in the environment (read once)
-int ring_prefetch() {
-    static const int on = [] {
-        const char *e = getenv("SCP_RING_PREFETCH");
-        return (e && e[0] == '0') ? 0 : 1;
-    }();
-    return on;
-}
 
 // Tile of a ring model: 128 threads, so that two CTAs share an SM and one
 // CTA's plane barrier overlaps the other's work; 32 x 4 while the 4-slot ring

@@ -414,7 +414,9 @@ static int setup_launch(scp_gpu *h) {
     if (rc) return rc;
     if (occ < 1) return SCP_EUNSUPPORTED;
     int tw = ts.tx, th = ts.ty;
-    if (h->p.tile_variant == 0 && !pairs && h->tma == 0)
+    if (h->p.tile_variant == 0 && pairs)
+        fit_pair_tile(h->N, &tw, &th);
+    else if (h->p.tile_variant == 0 && h->tma == 0)
         fit_tile(h->N, ts.tx * ts.ty, (ts.tx + 2) * (ts.ty + 2), &tw, &th);
     plan_tiles(h->N, tw, th, nsm * occ, &h->tg, &h->grid);
     h->tg_run = h->tg;

@@ -31,42 +31,88 @@ __device__ __forceinline__ void two_sum2(V2 a, V2 b, V2 *s, V2 *e) {
     *s = t;
 }
 
-// sin and cos of both lanes, |x| <= 2^12: the reduction and Taylor
-// polynomials of sincos_bounded<float> (trig.cuh) in packed arithmetic.  The
-// quadrant k = rint(x*2/pi) comes from adding 1.5*2^23, which leaves k in the
-// low mantissa bits (round to nearest even, as rintf).
-__device__ __forceinline__ void sincos2(V2 x, V2 *sn, V2 *cs) {
-    using C = TrigConsts<float>;
-    const float MAGIC = 12582912.0f;   // 1.5 * 2^23
-    const V2 t = fma2(x, V2(C::TWO_OVER_PI), V2(MAGIC));
-    const V2 kq = t - V2(MAGIC);
-    V2 r = fma2(kq, V2(-C::P1), x);
-    r = fma2(kq, V2(-C::P2), r);
-    r = fma2(kq, V2(-C::P3), r);
+// Batches of pairs of angles of one site pair, |x| <= 2^12: the reduction and
+// Taylor polynomials of sincos_bounded<float> (trig.cuh) in packed arithmetic,
+// with the range reduction -- needed only beyond pi/4, where the quadrant
+// k = rint(x*2/pi) is not 0 -- as one branch for the batch.  The quadrant
+// comes from adding 1.5*2^23, which leaves k in the low mantissa bits (round
+// to nearest even, as rintf).
+template <int n>
+__device__ __forceinline__ bool any_beyond_quarter(const V2 (&x)[n]) {
+    float m = 0.f;
+    bool nan = false;
+#pragma unroll
+    for (int i = 0; i < n; i++) {
+        m = fmaxf(m, fmaxf(fabsf(x[i].v.x), fabsf(x[i].v.y)));
+        nan |= isnan(x[i].v.x) || isnan(x[i].v.y);
+    }
+    return m > 0.785398f || nan;
+}
+__device__ __forceinline__ V2 taylor_sin2(V2 r) {
     const V2 s = r * r;
     V2 p = fma2(V2(-2.5052108385441718775e-8f), s, V2(2.7557319223985890653e-6f));   // -1/11!, 1/9!
     p = fma2(p, s, V2(-1.9841269841269841270e-4f));                                   // -1/7!
     p = fma2(p, s, V2(8.3333333333333333333e-3f));                                    // 1/5!
     p = fma2(p, s, V2(-1.6666666666666666667e-1f));                                   // -1/3!
-    const V2 sr = fma2(r * s, p, r);
+    return fma2(r * s, p, r);
+}
+__device__ __forceinline__ V2 taylor_cos2(V2 r) {
+    const V2 s = r * r;
     V2 q = fma2(V2(-2.7557319223985890653e-7f), s, V2(2.4801587301587301587e-5f));   // -1/10!, 1/8!
     q = fma2(q, s, V2(-1.3888888888888888889e-3f));                                   // -1/6!
     q = fma2(q, s, V2(4.1666666666666666667e-2f));                                    // 1/4!
     q = fma2(q, s, V2(-0.5f));                                                         // -1/2!
-    const V2 cr = fma2(s, q, V2(1.0f));
-    // x = r + k*pi/2: rotate (sin r, cos r) by k quarter turns, per lane
-    const unsigned kx = __float_as_uint(t.v.x), ky = __float_as_uint(t.v.y);
-    const unsigned gx = (kx & 2u) << 30, gy = (ky & 2u) << 30;   // sign flip for k = 2, 3 (mod 4)
-    const float s1x = (kx & 1u) ? cr.v.x : sr.v.x, c1x = (kx & 1u) ? -sr.v.x : cr.v.x;
-    const float s1y = (ky & 1u) ? cr.v.y : sr.v.y, c1y = (ky & 1u) ? -sr.v.y : cr.v.y;
-    *sn = V2(__uint_as_float(__float_as_uint(s1x) ^ gx), __uint_as_float(__float_as_uint(s1y) ^ gy));
-    *cs = V2(__uint_as_float(__float_as_uint(c1x) ^ gx), __uint_as_float(__float_as_uint(c1y) ^ gy));
+    return fma2(s, q, V2(1.0f));
 }
 
-__device__ __forceinline__ V2 sin2(V2 x) {
-    V2 s, c;
-    sincos2(x, &s, &c);
-    return s;
+template <int n>
+__device__ __forceinline__ void sincos2_batch(const V2 (&ang)[n], V2 (&sn)[n], V2 (&cs)[n]) {
+    using C = TrigConsts<float>;
+    const float MAGIC = 12582912.0f;   // 1.5 * 2^23
+    V2 r[n];
+    const bool big = any_beyond_quarter(ang);
+#pragma unroll
+    for (int i = 0; i < n; i++) r[i] = ang[i];
+    if (big) {
+#pragma unroll
+        for (int i = 0; i < n; i++) {
+            const V2 kq = fma2(ang[i], V2(C::TWO_OVER_PI), V2(MAGIC)) - V2(MAGIC);
+            r[i] = fma2(kq, V2(-C::P1), ang[i]);
+            r[i] = fma2(kq, V2(-C::P2), r[i]);
+            r[i] = fma2(kq, V2(-C::P3), r[i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < n; i++) {
+        sn[i] = taylor_sin2(r[i]);
+        cs[i] = taylor_cos2(r[i]);
+    }
+    if (big) {   // x = r + k*pi/2: rotate (sin r, cos r) by k quarter turns, per lane
+#pragma unroll
+        for (int i = 0; i < n; i++) {
+            const V2 t = fma2(ang[i], V2(C::TWO_OVER_PI), V2(MAGIC));
+            const unsigned kx = __float_as_uint(t.v.x), ky = __float_as_uint(t.v.y);
+            const unsigned gx = (kx & 2u) << 30, gy = (ky & 2u) << 30;   // sign flip for k = 2, 3 (mod 4)
+            const float s1x = (kx & 1u) ? cs[i].v.x : sn[i].v.x, c1x = (kx & 1u) ? -sn[i].v.x : cs[i].v.x;
+            const float s1y = (ky & 1u) ? cs[i].v.y : sn[i].v.y, c1y = (ky & 1u) ? -sn[i].v.y : cs[i].v.y;
+            sn[i] = V2(__uint_as_float(__float_as_uint(s1x) ^ gx), __uint_as_float(__float_as_uint(s1y) ^ gy));
+            cs[i] = V2(__uint_as_float(__float_as_uint(c1x) ^ gx), __uint_as_float(__float_as_uint(c1y) ^ gy));
+        }
+    }
+}
+
+// sines in place
+template <int n>
+__device__ __forceinline__ void sin2_batch(V2 (&x)[n]) {
+    if (any_beyond_quarter(x)) {
+        V2 s[n], c[n];
+        sincos2_batch(x, s, c);
+#pragma unroll
+        for (int i = 0; i < n; i++) x[i] = s[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < n; i++) x[i] = taylor_sin2(x[i]);
+    }
 }
 
 }  // namespace scp
