@@ -24,6 +24,7 @@ struct DiagConsts {
     long long N3;
     double L, dx, dV, idx1;
     double m2, mtheta2, eta, mu, kappa;
+    double ei;                // eta/(2dx)
     int gauged;               // covariant energy, plaquette energy (g != 0)
     int links;                // th / E columns present: Gauss residual, E_em, Q_flux
     int real;                 // real 6-field mode (imaginary sector zero): theta_rms over 3 components
@@ -232,16 +233,62 @@ __global__ void __launch_bounds__(kRedThreads) diag_pass2_kernel(View V, DiagCon
     block_fold<1, 1>(S, M, scratch, part);
 }
 
-// Pass 2 after a synchronous step launch that summed pass 1 itself (step.cuh,
-// StepIO::dpart): r_core and the argmax site as diag_pass2_kernel, and the
-// Gauss-law slots of pass 1 (compute_gauss, scp_sim.c:2186-2243), which need
-// E_{n+1} of the neighbouring sites, from the charge density the launch
-// stored (rho, N^3; links only).
-// part per CTA: sums [rsum, GL2, NOM, FSUM, NC], maxima [-min_idx, GMAX].
+// Final scalar reads: omega_core at the argmax-s site and the two theta probes.
+// out[0]=omega_core out[1..4]=thp1u thp1v thp2u thp2v
+// negidx: the folded -(lowest qualifying site index).
 template <class View>
-__global__ void __launch_bounds__(kRedThreads) diag_pass2g_kernel(View V, DiagConsts c, const double *fin1,
-                                                                  const double *rho, double *part) {
-    __shared__ double scratch[7 * 32];
+__device__ __forceinline__ void diag_points(const View &V, const DiagConsts &c, double negidx, double probe1,
+                                            double probe2, double *out) {
+    const int N = c.N;
+    const long long NN = (long long)N * N;
+    out[0] = 0.0;
+    if (isfinite(negidx)) {
+        const long long idx = (long long)(-negidx);
+        const double u0 = V.q(FU, idx), v0 = V.q(FV, idx), ud0 = V.p(FU, idx), vd0 = V.p(FV, idx);
+        const double den = u0 * u0 + v0 * v0;
+        if (den >= 1e-20) out[0] = (u0 * vd0 - v0 * ud0) / den;
+    }
+    int jc = (int)llround(c.L / c.dx);
+    jc = jc < 0 ? 0 : (jc > N - 1 ? N - 1 : jc);
+    int i1 = (int)llround((probe1 + c.L) / c.dx);
+    i1 = i1 < 0 ? 0 : (i1 > N - 1 ? N - 1 : i1);
+    int i2 = (int)llround((probe2 + c.L) / c.dx);
+    i2 = i2 < 0 ? 0 : (i2 > N - 1 ? N - 1 : i2);
+    const long long p1 = (long long)i1 * NN + (long long)jc * N + jc;
+    const long long p2 = (long long)i2 * NN + (long long)jc * N + jc;
+    out[1] = V.q(FTU + 1, p1); out[2] = V.q(FTV + 1, p1);
+    out[3] = V.q(FTU + 1, p2); out[4] = V.q(FTV + 1, p2);
+}
+
+template <class View>
+__global__ void diag_point_kernel(View V, DiagConsts c, const double *negidx_p, double probe1, double probe2,
+                                  double *out) {
+    if (threadIdx.x == 0 && blockIdx.x == 0) diag_points(V, c, *negidx_p, probe1, probe2, out);
+}
+
+// Where the folded values of one diagnostics call lie (device array `fold`,
+// and its copy in host memory): pass 1's sums and maxima, pass 2's sums and
+// maxima, the point values, and room for an extension's own sums.
+enum : int { DF_PASS1 = 0, DF_PASS2 = 32, DF_POINT = 40, DF_EXT = 48, DF_EXT2 = 80, DF_N = 96 };
+
+// Pass 2 and the end of a diagnostics call: r_core and the argmax site as
+// diag_pass2_kernel, and with GAUSS (after a synchronous step launch that
+// summed pass 1 itself, step.cuh, StepIO::dpart) the Gauss-law slots of pass 1
+// (compute_gauss, scp_sim.c:2186-2243), which need E_{n+1} of the neighbouring
+// sites, from the charge density the launch stored (rho, N^3).  The last CTA
+// to finish folds the partials, reads the point values and writes every
+// folded value to host memory, so a call is two launches and one wait: the
+// separate folds, point reads and copies took 55 us at 32^3 where this takes 26,
+// and a copy of a frame in flight no longer holds up the values
+// (both would use the device-to-host engine).
+// part per CTA: sums [rsum, GL2, NOM, FSUM, NC], maxima [-min_idx, GMAX].
+template <class View, bool GAUSS>
+__global__ void __launch_bounds__(kRedThreads) diag_finish_kernel(View V, DiagConsts c, double *fold,
+                                                                  const double *rho, double *part, unsigned *count,
+                                                                  double probe1, double probe2, double *host) {
+    __shared__ double scratch[kRedThreads];   // 7 x 32 for the block's fold, a row of 32 per warp for the last one
+    static_assert(kRedThreads >= 7 * 32, "scratch of the block fold");
+    const double *fin1 = fold + DF_PASS1;
     const double M0 = fin1[DS_M0] * c.dV;
     const double cx = M0 < 1e-30 ? 0.0 : fin1[DS_CX] * c.dV / M0;
     const double cy = M0 < 1e-30 ? 0.0 : fin1[DS_CY] * c.dV / M0;
@@ -256,6 +303,7 @@ __global__ void __launch_bounds__(kRedThreads) diag_pass2g_kernel(View V, DiagCo
         site_ijk(idx, N, &i, &j, &k);
         const double x = -c.L + i * c.dx, y = -c.L + j * c.dx, z = -c.L + k * c.dx;
         double rho2 = 0.0, sp = 1.0;
+#pragma unroll
         for (int a = 0; a < 3; a++) {
             const double u = V.q(FU + a, idx), v = V.q(FV + a, idx);
             rho2 += u * u + v * v;
@@ -263,7 +311,7 @@ __global__ void __launch_bounds__(kRedThreads) diag_pass2g_kernel(View V, DiagCo
         }
         S[0] += ((x - cx) * (x - cx) + (y - cy) * (y - cy) + (z - cz) * (z - cz)) * rho2;
         if (sp >= sthr) M[0] = fmax(M[0], -(double)idx);
-        if (c.links) {
+        if constexpr (GAUSS) {
             const long long im = (long long)wrapi(i - 1, N) * NN + (long long)j * N + k;
             const long long jm = (long long)i * NN + (long long)wrapi(j - 1, N) * N + k;
             const long long km = (long long)i * NN + (long long)j * N + wrapi(k - 1, N);
@@ -282,35 +330,11 @@ __global__ void __launch_bounds__(kRedThreads) diag_pass2g_kernel(View V, DiagCo
         }
     }
     block_fold<5, 2>(S, M, scratch, part);
-}
-
-// Final scalar reads: omega_core at the argmax-s site and the two theta probes.
-// out[0]=omega_core out[1..4]=thp1u thp1v thp2u thp2v
-// negidx_p: the folded -(lowest qualifying site index).
-template <class View>
-__global__ void diag_point_kernel(View V, DiagConsts c, const double *negidx_p, double probe1, double probe2,
-                                  double *out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const int N = c.N;
-    const long long NN = (long long)N * N;
-    out[0] = 0.0;
-    const double negidx = *negidx_p;
-    if (isfinite(negidx)) {
-        const long long idx = (long long)(-negidx);
-        const double u0 = V.q(FU, idx), v0 = V.q(FV, idx), ud0 = V.p(FU, idx), vd0 = V.p(FV, idx);
-        const double den = u0 * u0 + v0 * v0;
-        if (den >= 1e-20) out[0] = (u0 * vd0 - v0 * ud0) / den;
-    }
-    int jc = (int)llround(c.L / c.dx);
-    jc = jc < 0 ? 0 : (jc > N - 1 ? N - 1 : jc);
-    int i1 = (int)llround((probe1 + c.L) / c.dx);
-    i1 = i1 < 0 ? 0 : (i1 > N - 1 ? N - 1 : i1);
-    int i2 = (int)llround((probe2 + c.L) / c.dx);
-    i2 = i2 < 0 ? 0 : (i2 > N - 1 ? N - 1 : i2);
-    const long long p1 = (long long)i1 * NN + (long long)jc * N + jc;
-    const long long p2 = (long long)i2 * NN + (long long)jc * N + jc;
-    out[1] = V.q(FTU + 1, p1); out[2] = V.q(FTV + 1, p1);
-    out[3] = V.q(FTU + 1, p2); out[4] = V.q(FTV + 1, p2);
+    if (!last_block_done(count)) return;
+    fold_rows_block<5, 2>(part, gridDim.x, scratch, fold + DF_PASS2);
+    if (threadIdx.x == 0) diag_points(V, c, fold[DF_PASS2 + 5], probe1, probe2, fold + DF_POINT);
+    __syncthreads();
+    for (int q = threadIdx.x; q < DF_N; q += blockDim.x) host[q] = fold[q];
 }
 
 }  // namespace scp

@@ -83,10 +83,10 @@ template <class MODE, bool SECOND, bool ACC, bool LINKS>
 struct FabricPass {
     static_assert(!LINKS || ACC, "the links come with the last fabric");
     static constexpr int TH = 12;
-    static constexpr int NR = 15, NA = 12, CF = LINKS ? 12 : 15;
+    static constexpr int NR = 15, CF = LINKS ? 12 : 15;
     static constexpr int NM = LINKS ? 15 : 12;
     static constexpr int MIN_CTAS = 1;
-    static constexpr bool HALO_APART = true;
+    static constexpr bool HALO_APART = true, CONVERT = false;
 
     struct Args {
         const double *src[2];   // this fabric's 12 matter positions; th
@@ -97,6 +97,12 @@ struct FabricPass {
         LeapIO io;              // matter; E and th (LINKS)
         double *kacc;           // 3 arrays: accumulated currents
     };
+
+    static constexpr int NR_FEW = NR;   // always all of them
+    __device__ static __forceinline__ bool few(const Args &) { return false; }
+    __device__ static __forceinline__ const double *src(const Args &A, int f, long long n3) {
+        return f < 12 ? A.src[0] + f * n3 : A.src[1] + (f - 12) * n3;
+    }
 
     struct State {
         GaugedCarry cy;

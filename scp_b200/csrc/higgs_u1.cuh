@@ -51,16 +51,20 @@ struct HiggsU1 {
     static constexpr int TH = 12;                        // first gauge links
     static constexpr int TH2 = kTh2Slot;                      // second gauge links
     static constexpr int HF = G2 ? 18 : 15;              // the Higgs field
-    static constexpr int NR = 15 + (G2 ? 3 : 0) + (HIGGS ? 1 : 0), NA = NR, CF = 12;
+    static constexpr int NR = 15 + (G2 ? 3 : 0) + (HIGGS ? 1 : 0), CF = 12;
     static constexpr int MIN_CTAS = 1;
-    static constexpr bool HALO_APART = false;
+    static constexpr bool HALO_APART = false, CONVERT = false;
 
     struct Args {
-        const double *src[2];   // positions x_{n+1}, NR arrays
+        const double *x;        // positions x_{n+1}, NR arrays
         int N;
         HuConsts c;
         LeapIO io;
     };
+
+    static constexpr int NR_FEW = NR;   // always all of them
+    __device__ static __forceinline__ bool few(const Args &) { return false; }
+    __device__ static __forceinline__ const double *src(const Args &A, int f, long long n3) { return A.x + f * n3; }
 
     struct State {
         GaugedCarry cy;

@@ -1,6 +1,5 @@
-// kern_ext.cu -- instantiations and launchers of the plane-ring kernels: the
-// real mode's optional terms and the FP64 diagnostics.
-#include "diag_ring.cuh"
+// kern_ext.cu -- instantiations and launchers of the plane-ring kernels of the
+// real mode's optional terms.
 #include "ext_launch.cuh"
 #include "real6.cuh"
 
@@ -35,49 +34,6 @@ int ring_plan(int N, int nsm, ExtPlan *p) {
 }
 
 }  // namespace
-
-namespace {
-template <bool G>
-int diag_plan_t(int N, int nsm, ExtPlan *p) {
-    using M = DiagRing<G>;
-    constexpr int TX = TileOf<M>::TX, TY = TileOf<M>::TY;
-    using S = RingShape<M::NR, TX, TY>;
-    auto fn = diag_ring_kernel<G, TX, TY>;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem_bytes) != cudaSuccess)
-        return -1;
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, TX * TY, S::smem_bytes) != cudaSuccess || occ < 1)
-        return -1;
-    plan_ring_tiles(N, TX, TY, nsm * occ, p);
-    p->smem = S::smem_bytes;
-    return 0;
-}
-template <bool G>
-cudaError_t diag_launch_t(const ExtPlan &p, const DiagConsts &c, const DiagRingIO &io, double *part,
-                          cudaStream_t st) {
-    typename DiagRing<G>::Args a;
-    for (int f = 0; f < 12; f++) a.src.f[f] = io.x[f];
-    for (int d = 0; d < 3; d++) {   // without links: any valid arrays, never read
-        a.src.f[DiagRing<G>::TH + d] = io.th ? io.th + d * c.N3 : io.x[d];
-        a.src.f[DiagRing<G>::EF + d] = io.E ? io.E + d * c.N3 : io.x[3 + d];
-    }
-    a.N = c.N;
-    a.c = c;
-    a.mom = io.mom;
-    using T = TileOf<DiagRing<G>>;
-    diag_ring_kernel<G, T::TX, T::TY><<<p.grid, T::NT, p.smem, st>>>(a, p.tg, part);
-    return cudaGetLastError();
-}
-}  // namespace
-
-int diag_ring_plan(bool gauged, bool, int N, int nsm, ExtPlan *plan) {
-    return gauged ? diag_plan_t<true>(N, nsm, plan) : diag_plan_t<false>(N, nsm, plan);
-}
-
-cudaError_t diag_ring_pass1(bool gauged, bool, const ExtPlan &plan, const DiagConsts &c, const DiagRingIO &io,
-                            double *part, cudaStream_t st) {
-    return gauged ? diag_launch_t<true>(plan, c, io, part, st) : diag_launch_t<false>(plan, c, io, part, st);
-}
 
 int r6_plan(bool aux, int N, int nsm, ExtPlan *aux_plan, ExtPlan *step_plan) {
     if (aux) {

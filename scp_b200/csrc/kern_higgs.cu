@@ -22,7 +22,7 @@ cudaError_t hu_launch(const ExtPlan &p, const HuConsts &c, const HuIO &io, cudaS
     using M = HiggsU1<MODE, H, G>;
     typename M::Args a;
     const long long n3 = c.N3, at[2] = {0, 12 * n3};
-    a.src[0] = a.src[1] = io.x;   // NR consecutive arrays
+    a.x = io.x;
     a.N = c.N;
     a.c = c;
     for (int b = 0; b < 2; b++) {

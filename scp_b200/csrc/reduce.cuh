@@ -91,6 +91,38 @@ __device__ __forceinline__ void fold_partials_block(const double *part, int nb, 
     }
 }
 
+// Fold of nb partial rows of NS sums and NM maxima (at most 32 slots) by the
+// last CTA of a grid to finish: lane q of every warp takes slot q, the warps
+// take rows in turn (coalesced, sixteen in flight; one row at a time per slot
+// cost 9 us for 256 rows), then the warps' values are joined in warp order.
+// scratch: 32 doubles per warp.
+template <int NS, int NM>
+__device__ __forceinline__ void fold_rows_block(const double *part, int nb, double *scratch, double *out) {
+    constexpr int NQ = NS + NM, FLY = 16;
+    static_assert(NQ <= 32, "one lane per slot");
+    const int q = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const bool is_max = q >= NS;
+    double acc = is_max ? -INFINITY : 0.0;
+    if (q < NQ)
+        for (int b0 = w; b0 < nb; b0 += nw * FLY) {
+            double v[FLY];
+#pragma unroll
+            for (int n = 0; n < FLY; n++) v[n] = b0 + n * nw < nb ? __ldcg(part + (size_t)(b0 + n * nw) * NQ + q) : 0.0;
+#pragma unroll
+            for (int n = 0; n < FLY; n++)
+                if (b0 + n * nw < nb) acc = is_max ? fmax(acc, v[n]) : acc + v[n];
+        }
+    scratch[w * 32 + q] = acc;
+    __syncthreads();
+    if (threadIdx.x < NQ) {
+        acc = scratch[threadIdx.x];
+        for (int n = 1; n < nw; n++)
+            acc = is_max ? fmax(acc, scratch[n * 32 + threadIdx.x]) : acc + scratch[n * 32 + threadIdx.x];
+        out[threadIdx.x] = acc;
+    }
+    __syncthreads();
+}
+
 // After block_fold: true in exactly one CTA, the last to finish, once every
 // CTA's partial is visible to it.  count is reset by that CTA for the next
 // launch.  No CTA waits for another.

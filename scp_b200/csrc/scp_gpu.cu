@@ -18,6 +18,7 @@
 #include "../../include/scp_gpu.h"
 #include "common.cuh"
 #include "diag.cuh"
+#include "diag_walk.cuh"
 #include "gauss.cuh"
 #include "reduce.cuh"
 #include "snapshot.cuh"
@@ -38,6 +39,7 @@
 #include <algorithm>
 #include <type_traits>
 #include <mutex>
+#include <vector>
 
 using namespace scp;
 
@@ -127,7 +129,7 @@ struct scp_gpu {
     FabConsts fc{};
     double *kacc = nullptr;      // accumulated currents (3 arrays)
     ExtPlan xplan{}, xplan2{};
-    ExtPlan dplan{};             // first diagnostics reduction on the plane ring (FP64 states)
+    ExtPlan dplan{};             // first diagnostics reduction on the plane walker
     int dplan_ok = 0;
     int nx = 0;                  // position arrays per buffer of the extension layouts
     int device;
@@ -148,6 +150,7 @@ struct scp_gpu {
     int *flag = nullptr;
     unsigned *count = nullptr;   // last-CTA counter of the fused CG launches
     double h_small[64];          // host landing area of the small device-to-host reads
+    double *res = nullptr;       // page-locked: the folded values of a diagnostics call, written by the device
     void *stage = nullptr;       // snapshot down-conversion staging (N3 doubles)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // asynchronous snapshots: device staging of every column, copies on their own stream
@@ -452,6 +455,8 @@ static int launch_step(scp_gpu *h, bool first, bool sync) {
         const bool dg = sync && !first && h->dfuse;
         io.dpart = dg ? h->dpart : nullptr;
         io.drho = dg ? h->drho : nullptr;
+        io.dfold = h->fold + DF_PASS1;
+        io.dcount = h->count;
         h->dvalid = dg ? 1 : 0;
         if (h->tma == 1) {
             TmaStepFn fn = step_tma_fn(h->shape, h->gauged, first, sync, damping_on(h), &smem);
@@ -659,11 +664,37 @@ static void keep_pool(int dev) {
 // the running chunks instead of queueing behind them.
 static thread_local int t_stream_priority = 0;
 
+// Page-locked slots of DF_N doubles for the results of diagnostics calls: a
+// block of 256 is pinned when none is free (pinning costs the better part of a
+// millisecond, and the server makes and frees handles at a high rate), a slot
+// returns to the free list with its handle.
+static std::mutex g_res_mu;
+static std::vector<double *> g_res_free;
+static double *result_slot() {
+    constexpr int kBlock = 256;
+    std::lock_guard<std::mutex> lk(g_res_mu);
+    if (g_res_free.empty()) {
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, sizeof(double) * DF_N * kBlock, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
+            return nullptr;
+        for (int q = kBlock - 1; q >= 0; q--) g_res_free.push_back((double *)p + (size_t)q * DF_N);
+    }
+    double *r = g_res_free.back();
+    g_res_free.pop_back();
+    return r;
+}
+static void result_slot_free(double *r) {
+    std::lock_guard<std::mutex> lk(g_res_mu);
+    g_res_free.push_back(r);
+}
+
 static int alloc_common(scp_gpu *h) {
     keep_pool(h->device);
     CK(cudaStreamCreateWithPriority(&h->stream, cudaStreamNonBlocking, t_stream_priority));
     CK(cudaMallocAsync(&h->part, sizeof(double) * kRedMaxBlocks * 32, h->stream));
-    CK(cudaMallocAsync(&h->fold, sizeof(double) * 64, h->stream));
+    CK(cudaMallocAsync(&h->fold, sizeof(double) * DF_N, h->stream));
+    CK(cudaMemsetAsync(h->fold, 0, sizeof(double) * DF_N, h->stream));
+    if (!(h->res = result_slot())) return SCP_ENOMEM;
     CK(cudaMallocAsync(&h->cg, sizeof(double) * 16, h->stream));
     CK(cudaMallocAsync(&h->point, sizeof(double) * 8, h->stream));
     CK(cudaMallocAsync(&h->flag, sizeof(int), h->stream));
@@ -672,7 +703,7 @@ static int alloc_common(scp_gpu *h) {
     CK(cudaMemsetAsync(h->count, 0, sizeof(unsigned), h->stream));
     CK(cudaEventCreate(&h->ev0));
     CK(cudaEventCreate(&h->ev1));
-    h->dev_bytes += sizeof(double) * (kRedMaxBlocks * 32 + 64 + 16 + 8);
+    h->dev_bytes += sizeof(double) * (kRedMaxBlocks * 32 + DF_N + 16 + 8);
     return SCP_OK;
 }
 
@@ -941,27 +972,19 @@ static int init_gext(scp_gpu *h, const double *const *cols, bool on_device) {
     return hu_launch_step(h, true, false);
 }
 
-// Higgs energy of the current state (the reference adds it to E_total, scp_sim.c:2034)
-static int gext_higgs_energy(scp_gpu *h, double *e) {
+// enqueue the Higgs energy of the current state (the reference adds it to
+// E_total, scp_sim.c:2034) into fold + DF_EXT
+static int gext_higgs_energy(scp_gpu *h) {
     const int nb = red_blocks(h->N3);
     const size_t hf = (size_t)(15 + 3 * h->g2) * h->N3;
     const double *X = h->X[h->cur ^ 1];
     hu_higgs_energy_kernel<<<nb, kRedThreads, 0, h->stream>>>(X, X + hf, h->S + hf, h->hc, h->part);
-    fold_partials_kernel<1, 0><<<1, 1024, 0, h->stream>>>(h->part, nb, h->fold);
+    fold_partials_kernel<1, 0><<<1, 1024, 0, h->stream>>>(h->part, nb, h->fold + DF_EXT);
     CK(cudaGetLastError());
-    int rc;
-    if ((rc = fold_to_host(h, 1))) return rc;
-    *e = fold_get(h, 0);
     return SCP_OK;
 }
 
 // ---------------------------------------------------------------- three fabrics
-
-static DiagConsts diag_consts(const scp_gpu *h);
-template <class View>
-static int diag_with(scp_gpu *h, const View &V, scp_gpu_diag_out *out);
-static int diag_pass1_ring(scp_gpu *h, const DiagConsts &c, const double *Xm, const double *Pm, const double *th,
-                           const double *E, int *rows);
 
 // slots of the three-fabric layout
 constexpr int kFabL = 15, kFabQ = 27;
@@ -1101,42 +1124,6 @@ static int init_mf(scp_gpu *h, const double *const *cols, bool on_device) {
     if (fabric_plan(h->N, nsm, &h->xplan)) return SCP_EUNSUPPORTED;
     if ((rc = mf_gauss_startup(h))) return rc;
     return fab_launch_step(h, true, false);
-}
-
-// fabric C's diagnostics, plus fabric L's energies (compute_energy_complex_gauge,
-// scp_sim.c:1977-2028), the Gauss norm with rho_em and the fabric charges
-static int mf_diag(scp_gpu *h, scp_gpu_diag_out *out) {
-    const double *X = h->X[h->cur ^ 1], *P = h->S;
-    const size_t n3 = h->N3;
-    ViewF64 V{X, P, h->N3};
-    int rc = diag_with(h, V, out);
-    if (rc && rc != SCP_ENONFINITE) return rc;
-    const int nb = red_blocks(h->N3);
-    const DiagConsts c = diag_consts(h);
-    int nb1 = 0;
-    if ((rc = diag_pass1_ring(h, c, X + kFabL * n3, P + kFabL * n3, X + FTH * n3, P + FTH * n3, &nb1))) return rc;
-    fold_partials_kernel<DS_NSUM, DM_NMAX><<<1, 1024, 0, h->stream>>>(h->part, nb1, h->fold);
-    CK(cudaGetLastError());
-    if ((rc = fold_to_host(h, DS_EC + 1))) return rc;
-    double *o = out->v;
-    for (int q = 0; q <= DS_EC; q++) o[SCP_DIAG_E_PHI_KIN + q] += h->h_small[q];   // DS_EPK..DS_EC = slots 0..7
-    o[SCP_DIAG_E_TOTAL] = o[SCP_DIAG_E_PHI_KIN] + o[SCP_DIAG_E_THETA_KIN] + o[SCP_DIAG_E_GRAD] + o[SCP_DIAG_E_MASS] +
-                          o[SCP_DIAG_E_POT] + o[SCP_DIAG_E_TGRAD] + o[SCP_DIAG_E_TMASS] + o[SCP_DIAG_E_COUPLING] +
-                          o[SCP_DIAG_E_EM];
-    const scp_gpu_params &p = h->p;
-    fabric_diag_kernel<<<nb, kRedThreads, 0, h->stream>>>(fab_view(h, X, P), h->N, p.L, p.dx, p.g_gauge, c.Rint2,
-                                                          h->G_offset, h->part);
-    fold_partials_kernel<FS_NSUM, 1><<<1, 1024, 0, h->stream>>>(h->part, nb, h->fold);
-    CK(cudaGetLastError());
-    if ((rc = fold_to_host(h, FS_NSUM + 1))) return rc;
-    const double *f = h->h_small, dV = c.dV;
-    o[SCP_DIAG_GAUSS_MAX] = f[FS_NSUM];
-    o[SCP_DIAG_GAUSS_L2] = f[FS_NIN] > 0 ? sqrt(f[FS_GL2] / f[FS_NIN]) : 0.0;
-    o[SCP_DIAG_Q_C] = f[FS_QC] * dV;
-    o[SCP_DIAG_Q_Q] = f[FS_QQ] * dV;
-    o[SCP_DIAG_Q_L] = f[FS_QL] * dV;
-    o[SCP_DIAG_Q_EM] = f[FS_QEM] * dV;
-    return isfinite(o[SCP_DIAG_E_TOTAL]) ? SCP_OK : SCP_ENONFINITE;
 }
 
 // columns of a snapshot: th2 and E2 follow the 30 gauged ones with the second
@@ -1322,6 +1309,7 @@ static DiagConsts diag_consts_for(const scp_gpu_params &p, int gauged, int links
     c.N = p.N; c.N3 = (long long)p.N * p.N * p.N; c.L = p.L; c.dx = p.dx; c.dV = p.dx * p.dx * p.dx;
     c.idx1 = 1.0 / (2.0 * p.dx);
     c.m2 = p.m2; c.mtheta2 = p.mtheta2; c.eta = p.eta; c.mu = p.mu; c.kappa = p.kappa;
+    c.ei = c.eta * c.idx1;
     c.gauged = gauged;
     c.links = links;
     c.real = real;
@@ -1339,82 +1327,120 @@ static DiagConsts diag_consts(const scp_gpu *h) {
     return diag_consts_for(h->p, h->gauged, h->links, h->real, h->G_offset);
 }
 
-// First diagnostics reduction of an FP64 state on the plane ring: matter
-// positions Xm and momenta Pm (12 arrays each), links and E (3 each, or null);
-// the partial rows land in h->part, their count in *rows.
-static int diag_pass1_ring(scp_gpu *h, const DiagConsts &c, const double *Xm, const double *Pm, const double *th,
-                           const double *E, int *rows) {
+// First diagnostics reduction on the plane walker, folded into fold[0..]: of
+// an FP64 state (matter positions Xm and momenta Pm, 12 arrays each; links and
+// E, 3 each, or null), or of the handle's compensated state (Xm null).
+static int diag_pass1(scp_gpu *h, const DiagConsts &c, const double *Xm, const double *Pm, const double *th,
+                      const double *E, double *fold) {
+    const bool comp = !Xm;
     if (!h->dplan_ok) {
         int nsm = 0;
         CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
-        if (diag_ring_plan(c.gauged, c.links, h->N, nsm, &h->dplan)) return SCP_EUNSUPPORTED;
+        if (diag_walk_plan(c.gauged, comp, h->N, nsm, &h->dplan)) return SCP_EUNSUPPORTED;
         h->dplan_ok = 1;
     }
-    DiagRingIO io;
-    for (int f = 0; f < 12; f++) io.x[f] = Xm + (size_t)f * h->N3;
-    io.th = th;
-    io.E = E;
-    io.mom = Pm;
-    CK(diag_ring_pass1(c.gauged, c.links, h->dplan, c, io, h->part, h->stream));
-    *rows = h->dplan.grid;
+    DiagWalkArgs a;
+    a.N = h->N;
+    a.c = c;
+    a.x = Xm;
+    a.th = th;
+    a.E = E;
+    a.mom = Pm;
+    a.x32 = comp ? h->X32[h->cur ^ 1] : nullptr;
+    a.lo = comp ? h->LO[h->cur ^ 1] : nullptr;
+    a.tlo = comp ? h->TLO[h->cur ^ 1] : nullptr;
+    a.s32 = comp ? h->S32 : nullptr;
+    a.part = h->part;
+    a.fold = fold;
+    a.count = h->count;
+    CK(diag_walk(c.gauged, comp, h->dplan, a, h->stream));
     return SCP_OK;
 }
 
-template <class View>
-static int diag_with(scp_gpu *h, const View &V, scp_gpu_diag_out *out) {
+// One diagnostics call: pass 1 unless the synchronous step launch that
+// produced this state summed it, an extension's own sums (extra, enqueued by
+// the caller's function into fold + DF_EXT...), the finishing pass, one wait.
+// The folded values are then in h->res.
+template <class View, class Extra>
+static int diag_with(scp_gpu *h, const View &V, scp_gpu_diag_out *out, Extra extra) {
     const scp_gpu_params &p = h->p;
     const DiagConsts c = diag_consts(h);
     const int nb = red_blocks(h->N3);
-    int nb1 = nb;
-    const double *part1 = h->part;
-    // pass 1 already summed by the synchronous step launch that produced this state
+    int rc;
     const bool fused = std::is_same<View, ViewF64>::value && h->dvalid;
-    if constexpr (std::is_same<View, ViewF64>::value) {
-        if (fused) {
-            nb1 = h->grid_diag;
-            part1 = h->dpart;
-        } else {
+    if (!fused) {
+        if constexpr (std::is_same<View, ViewF64>::value) {
             const size_t th = (size_t)FTH * h->N3;
-            int rc = diag_pass1_ring(h, c, V.X, V.S, c.links ? V.X + th : nullptr, c.links ? V.S + th : nullptr,
-                                     &nb1);
-            if (rc) return rc;
+            rc = diag_pass1(h, c, V.X, V.S, c.links ? V.X + th : nullptr, c.links ? V.S + th : nullptr,
+                            h->fold + DF_PASS1);
+        } else {
+            rc = diag_pass1(h, c, nullptr, nullptr, nullptr, nullptr, h->fold + DF_PASS1);
         }
-    } else {
-        diag_pass1_kernel<View><<<nb, kRedThreads, 0, h->stream>>>(V, c, h->part);
+        if (rc) return rc;
     }
-    fold_partials_kernel<DS_NSUM, DM_NMAX><<<1, 1024, 0, h->stream>>>(part1, nb1, h->fold);
-    // pass 2 (r_core, argmax site), with the Gauss-law slots when pass 1 was fused
+    rc = extra(c);
+    if (rc) return rc;
     const bool gauss2 = fused && c.links;
-    const double *negidx;
-    if (gauss2) {
-        diag_pass2g_kernel<View><<<nb, kRedThreads, 0, h->stream>>>(V, c, h->fold, h->drho, h->part);
-        fold_partials_kernel<5, 2><<<1, 1024, 0, h->stream>>>(h->part, nb, h->fold + 44);
-        negidx = h->fold + 49;
-    } else {
-        diag_pass2_kernel<View><<<nb, kRedThreads, 0, h->stream>>>(V, c, h->fold, h->part);
-        fold_partials_kernel<1, 1><<<1, 1024, 0, h->stream>>>(h->part, nb, h->fold + 40);
-        negidx = h->fold + 41;
-    }
-    diag_point_kernel<View><<<1, 32, 0, h->stream>>>(V, c, negidx, p.qdiag_probe1, p.qdiag_probe2, h->point);
+    if (gauss2)
+        diag_finish_kernel<View, true><<<nb, kRedThreads, 0, h->stream>>>(
+            V, c, h->fold, h->drho, h->part, h->count, p.qdiag_probe1, p.qdiag_probe2, h->res);
+    else
+        diag_finish_kernel<View, false><<<nb, kRedThreads, 0, h->stream>>>(
+            V, c, h->fold, nullptr, h->part, h->count, p.qdiag_probe1, p.qdiag_probe2, h->res);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(h->h_small, h->fold, sizeof(double) * 51, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(h->h_small + 56, h->point, sizeof(double) * 5, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    double f1[kDiag1Q], f2[2] = {h->h_small[40], h->h_small[41]};
-    memcpy(f1, h->h_small, sizeof f1);
-    if (gauss2) {   // [rsum, GL2, NOM, FSUM, NC | -min_idx, GMAX]
-        const double *g = h->h_small + 44;
-        f2[0] = g[0];
-        f2[1] = g[5];
+    double f1[kDiag1Q];
+    memcpy(f1, h->res + DF_PASS1, sizeof f1);
+    const double *g = h->res + DF_PASS2;   // [rsum, GL2, NOM, FSUM, NC | -min_idx, GMAX]
+    const double f2[2] = {g[0], g[5]};
+    if (gauss2) {
         f1[DS_GL2] = g[1];
         f1[DS_NOM] = g[2];
         f1[DS_FSUM] = g[3];
         f1[DS_NC] = g[4];
         f1[DS_NSUM + DM_GMAX] = g[6];
     }
-    diag_assemble(f1, f2, h->h_small + 56, c, h->N3, p.g_gauge, out);
+    diag_assemble(f1, f2, h->res + DF_POINT, c, h->N3, p.g_gauge, out);
     if (!isfinite(out->v[SCP_DIAG_E_TOTAL])) return SCP_ENONFINITE;
     return SCP_OK;
+}
+template <class View>
+static int diag_with(scp_gpu *h, const View &V, scp_gpu_diag_out *out) {
+    return diag_with(h, V, out, [](const DiagConsts &) { return (int)SCP_OK; });
+}
+
+// fabric C's diagnostics, plus fabric L's energies (compute_energy_complex_gauge,
+// scp_sim.c:1977-2028), the Gauss norm with rho_em and the fabric charges
+static int mf_diag(scp_gpu *h, scp_gpu_diag_out *out) {
+    const double *X = h->X[h->cur ^ 1], *P = h->S;
+    const size_t n3 = h->N3;
+    ViewF64 V{X, P, h->N3};
+    const int rc = diag_with(h, V, out, [&](const DiagConsts &c) -> int {
+        int rc2 = diag_pass1(h, c, X + kFabL * n3, P + kFabL * n3, X + FTH * n3, P + FTH * n3, h->fold + DF_EXT);
+        if (rc2) return rc2;
+        const scp_gpu_params &p = h->p;
+        const int nb = red_blocks(h->N3);
+        fabric_diag_kernel<<<nb, kRedThreads, 0, h->stream>>>(fab_view(h, X, P), h->N, p.L, p.dx, p.g_gauge, c.Rint2,
+                                                              h->G_offset, h->part);
+        fold_partials_kernel<FS_NSUM, 1><<<1, 1024, 0, h->stream>>>(h->part, nb, h->fold + DF_EXT2);
+        CK(cudaGetLastError());
+        return SCP_OK;
+    });
+    if (rc && rc != SCP_ENONFINITE) return rc;
+    double *o = out->v;
+    const double *fl = h->res + DF_EXT;
+    for (int q = 0; q <= DS_EC; q++) o[SCP_DIAG_E_PHI_KIN + q] += fl[q];   // DS_EPK..DS_EC = slots 0..7
+    o[SCP_DIAG_E_TOTAL] = o[SCP_DIAG_E_PHI_KIN] + o[SCP_DIAG_E_THETA_KIN] + o[SCP_DIAG_E_GRAD] + o[SCP_DIAG_E_MASS] +
+                          o[SCP_DIAG_E_POT] + o[SCP_DIAG_E_TGRAD] + o[SCP_DIAG_E_TMASS] + o[SCP_DIAG_E_COUPLING] +
+                          o[SCP_DIAG_E_EM];
+    const double *f = h->res + DF_EXT2, dV = h->p.dx * h->p.dx * h->p.dx;
+    o[SCP_DIAG_GAUSS_MAX] = f[FS_NSUM];
+    o[SCP_DIAG_GAUSS_L2] = f[FS_NIN] > 0 ? sqrt(f[FS_GL2] / f[FS_NIN]) : 0.0;
+    o[SCP_DIAG_Q_C] = f[FS_QC] * dV;
+    o[SCP_DIAG_Q_Q] = f[FS_QQ] * dV;
+    o[SCP_DIAG_Q_L] = f[FS_QL] * dV;
+    o[SCP_DIAG_Q_EM] = f[FS_QEM] * dV;
+    return isfinite(o[SCP_DIAG_E_TOTAL]) ? SCP_OK : SCP_ENONFINITE;
 }
 
 extern "C" {
@@ -1427,11 +1453,11 @@ int scp_gpu_diag(scp_gpu *h, scp_gpu_diag_out *out) {
     if (h->mfab) return mf_diag(h, out);
     if (h->gx) {
         ViewF64 V{h->X[h->cur ^ 1], h->S, h->N3};
-        int rc = diag_with(h, V, out);
+        const int rc = diag_with(h, V, out, [&](const DiagConsts &) -> int {
+            return h->higgs ? gext_higgs_energy(h) : (int)SCP_OK;
+        });
         if (rc || !h->higgs) return rc;
-        double eh = 0.0;
-        if ((rc = gext_higgs_energy(h, &eh))) return rc;
-        out->v[SCP_DIAG_E_TOTAL] += eh;
+        out->v[SCP_DIAG_E_TOTAL] += h->res[DF_EXT];
         return isfinite(out->v[SCP_DIAG_E_TOTAL]) ? SCP_OK : SCP_ENONFINITE;
     }
     if (h->prec == SCP_PREC_FP64) {
@@ -1650,6 +1676,7 @@ void scp_gpu_free(scp_gpu *h) {
             if (b) cudaFreeAsync(b, h->stream);
         cudaStreamSynchronize(h->stream);
     }
+    if (h->res) result_slot_free(h->res);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
     if (h->snap_ready) cudaEventDestroy(h->snap_ready);

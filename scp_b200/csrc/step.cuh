@@ -89,6 +89,8 @@ struct StepIO {
     // charge density of every site into drho (gauged)
     double *dpart = nullptr;
     double *drho = nullptr;
+    double *dfold = nullptr;      // the last CTA folds the partials here
+    unsigned *dcount = nullptr;   // CTAs done
 };
 
 template <class P, int TX, int TY, bool GAUGED>
@@ -227,7 +229,7 @@ struct CpStage {
 // ---------------------------------------------------------------- FP64
 
 // Per-thread sums of the first diagnostics pass (energies, charges, core and
-// centroid moments, the per-site terms of diag_ring.cuh) over the sites a
+// centroid moments, the per-site terms of diag_walk.cuh) over the sites a
 // synchronous launch advances, without the constant factors, which step_sums
 // applies once per thread.
 enum : int {
@@ -246,7 +248,8 @@ struct StepSums {
 
 // The slots of the first pass from one thread's sums (the Gauss-law slots are
 // left to the pass that reads E of the neighbouring sites).
-__device__ __forceinline__ void step_sums(const StepSums &t, const StepConsts &c, DiagSums &o) {
+template <class C>
+__device__ __forceinline__ void step_sums(const StepSums &t, const C &c, DiagSums &o) {
     o.clear();
     const double hV = 0.5 * c.dV, g2 = c.idx1 * c.idx1;
     o.S[DS_EPK] = hV * t.s[SS_EPK];
@@ -554,7 +557,7 @@ __device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepCo
     const long long N3 = c.N3;
     const int tx = stg.tx, ty = stg.ty;
     auto XS = [&](int slot, int f, int r, int col) -> T { return stg.view(slot).get(f, r - ty - 1, col - tx - 1); };
-    const T dt = (T)c.dt, hdt = (T)c.hdt, idx1 = (T)c.idx1, idx2 = (T)c.idx2;
+    const T hdt = (T)c.hdt, idx1 = (T)c.idx1, idx2 = (T)c.idx2;
     const float dt_lo = (float)(c.dt - (double)(float)c.dt);
     const float hdt_lo = (float)(c.hdt - (double)(float)c.hdt);
 
@@ -932,6 +935,8 @@ step_diag_kernel(StepIO<F64> io, StepConsts c, TileGrid tg) {
     DiagSums acc;
     step_sums(sums, c, acc);
     block_fold<DS_NSUM, DM_NMAX>(acc.S, acc.M, reinterpret_cast<double *>(smem_raw), io.dpart);
+    if (last_block_done(io.dcount))
+        fold_rows_block<DS_NSUM, DM_NMAX>(io.dpart, gridDim.x, reinterpret_cast<double *>(smem_raw), io.dfold);
 }
 
 // ---------------------------------------------------------------- many grids per launch

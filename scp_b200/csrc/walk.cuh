@@ -8,14 +8,18 @@
 // one plane ahead, stay in registers.
 //
 // A model supplies
-//   NR, NA, CF     staged fields: the first NA are consecutive N^3 arrays at
-//                  src[0], the rest at src[1]; fields from CF on are staged
-//                  at the two corners (j+1, k-1) and (j-1, k+1) too
+//   NR, CF         staged fields, of which those from CF on are staged at the
+//                  two corners (j+1, k-1) and (j-1, k+1) too
+//   src(args, f, n3)   the N^3 array of staged field f
+//   NR_FEW, few(args)  a launch may stage only the first NR_FEW fields
+//   CONVERT        the fields are not FP64 arrays: value(args, f, n3, at) is
+//                  field f at element `at`, prefetch() its L2 prefetch; a plane
+//                  is then staged through registers, prefetched a plane ahead
 //   HALO_APART     own copies of a plane first, then the halo's, instead of
 //                  field by field: 375 against 397 us for a step of three
 //                  fabrics at 128^3, but 365 against 321 with the 19 fields of
 //                  the Higgs and second gauge
-//   Args           kernel arguments, with `const double *src[2]`, `int N`
+//   Args           kernel arguments, with `int N`
 //   State          per-thread state kept along the i walk
 //   load(args, st, idx)                first plane's global loads
 //   begin(args, st, m, c)              carry from the plane before the first
@@ -25,6 +29,8 @@
 //                  branch would be copied where the branch joins, and wait)
 // and runs as walk_kernel<Model, TX, TY>.
 #pragma once
+#include <type_traits>
+
 #include "gauged.cuh"
 
 namespace scp {
@@ -78,36 +84,68 @@ struct WalkStage {
         h_s = r * pitch + col;
         h_g = wrapi(j0 - 1 + r, N) * N + wrapi(k0 - 1 + col, N);
     }
+    // f(the number of fields this launch stages, as a constant)
+    template <class F>
+    __device__ __forceinline__ static void with_staged(const typename M::Args &a, F &&f) {
+        if (M::NR_FEW < M::NR && M::few(a)) f(std::integral_constant<int, M::NR_FEW>());
+        else f(std::integral_constant<int, M::NR>());
+    }
     __device__ __forceinline__ void issue(const typename M::Args &a, long long n3, int plane, int slot) {
         const long long pb = (long long)wrapi(plane, a.N) * a.N * a.N;
         double *sb = xs + slot * LY::PLANE;
-        auto src = [&](int f) { return (f < M::NA ? a.src[0] + f * n3 : a.src[1] + (f - M::NA) * n3) + pb; };
-        if constexpr (M::HALO_APART) {
-            if (act) {
+        if constexpr (M::CONVERT) {
+            static_assert(M::CF == M::NR, "converted staging brings no corners");
+            const long long nb = (long long)wrapi(plane + 1, a.N) * a.N * a.N + own_g;
+            with_staged(a, [&](auto nf) {   // own sites, the next plane's prefetch, the halo
+                constexpr int NF = decltype(nf)::value;
+                if (act) {
+                    double v[NF];
 #pragma unroll
-                for (int f = 0; f < M::NR; f++) cp_async8(sb + f * LY::FS + c_s, src(f) + own_g);
-            }
-            if (h_f0 == 0) {
+                    for (int f = 0; f < NF; f++) v[f] = M::value(a, f, n3, pb + own_g);
 #pragma unroll
-                for (int f = 0; f < M::NR; f++) cp_async8(sb + f * LY::FS + h_s, src(f) + h_g);
-            } else if (M::CF < M::NR && h_f0 == M::CF) {
+                    for (int f = 0; f < NF; f++) M::prefetch(a, f, n3, nb);
 #pragma unroll
-                for (int f = M::CF; f < M::NR; f++) cp_async8(sb + f * LY::FS + h_s, src(f) + h_g);
+                    for (int f = 0; f < NF; f++) sb[f * LY::FS + c_s] = v[f];
+                }
+                if (h_f0 == 0) {
+                    double v[NF];
+#pragma unroll
+                    for (int f = 0; f < NF; f++) v[f] = M::value(a, f, n3, pb + h_g);
+#pragma unroll
+                    for (int f = 0; f < NF; f++) sb[f * LY::FS + h_s] = v[f];
+                }
+            });
+        } else if constexpr (M::HALO_APART) {
+            with_staged(a, [&](auto nf) {
+                constexpr int NF = decltype(nf)::value;
+                if (act) {
+#pragma unroll
+                    for (int f = 0; f < NF; f++) cp_async8(sb + f * LY::FS + c_s, M::src(a, f, n3) + pb + own_g);
+                }
+                if (h_f0 == 0) {
+#pragma unroll
+                    for (int f = 0; f < NF; f++) cp_async8(sb + f * LY::FS + h_s, M::src(a, f, n3) + pb + h_g);
+                }
+            });
+            if (M::CF < M::NR && h_f0 == M::CF) {
+#pragma unroll
+                for (int f = M::CF; f < M::NR; f++) cp_async8(sb + f * LY::FS + h_s, M::src(a, f, n3) + pb + h_g);
             }
         } else {
 #pragma unroll
             for (int f = 0; f < M::NR; f++) {
-                if (act) cp_async8(sb + f * LY::FS + c_s, src(f) + own_g);
-                if (f >= h_f0) cp_async8(sb + f * LY::FS + h_s, src(f) + h_g);
+                if (act) cp_async8(sb + f * LY::FS + c_s, M::src(a, f, n3) + pb + own_g);
+                if (f >= h_f0) cp_async8(sb + f * LY::FS + h_s, M::src(a, f, n3) + pb + h_g);
             }
         }
         cp_async_commit();
     }
 };
 
-template <class M, int TX, int TY>
+// Extra arguments (a reduction's per-thread sums) are passed on to M::site.
+template <class M, int TX, int TY, class... Extra>
 __device__ __forceinline__ void walk_item(const typename M::Args &a, const TileGrid &tg, const Piece &pc,
-                                          WalkStage<M, TX, TY> &stg) {
+                                          WalkStage<M, TX, TY> &stg, Extra &...extra) {
     const int N = a.N;
     const long long NN = (long long)N * N, n3 = NN * N;
     const int k0 = pc.kt * tg.tw, j0 = pc.jt * tg.th, i0 = pc.i0, i1 = pc.i1;
@@ -129,7 +167,8 @@ __device__ __forceinline__ void walk_item(const typename M::Args &a, const TileG
         __syncthreads();
         if (i + 2 <= i1) stg.issue(a, n3, i + 2, sn);
         if (stg.act)
-            M::site(a, st, stg.view(sc), stg.view(sp), i, j, k, (long long)i * NN + stg.own_g, i + 1 < i1 ? NN : 0);
+            M::site(a, st, stg.view(sc), stg.view(sp), i, j, k, (long long)i * NN + stg.own_g, i + 1 < i1 ? NN : 0,
+                    extra...);
     }
 }
 

@@ -13,9 +13,8 @@ namespace {
 constexpr int kWalkX = 32, kWalkY = 8;
 
 template <class M>
-int walk_plan(int N, int nsm, ExtPlan *p) {
+int walk_plan_fn(const void *fn, int N, int nsm, ExtPlan *p) {
     using LY = WalkLayout<M, kWalkX, kWalkY>;
-    auto fn = walk_kernel<M, kWalkX, kWalkY>;
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LY::smem_bytes) != cudaSuccess)
         return -1;
     int occ = 0;
@@ -28,6 +27,11 @@ int walk_plan(int N, int nsm, ExtPlan *p) {
     p->ty = th;
     p->smem = LY::smem_bytes;
     return 0;
+}
+
+template <class M>
+int walk_plan(int N, int nsm, ExtPlan *p) {
+    return walk_plan_fn<M>((const void *)walk_kernel<M, kWalkX, kWalkY>, N, nsm, p);
 }
 
 template <class M>
