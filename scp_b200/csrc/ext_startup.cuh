@@ -220,7 +220,8 @@ struct ViewFabric {
 enum : int { R6_EPK = 0, R6_ETK, R6_EG, R6_EM, R6_EP, R6_ETG, R6_ETM, R6_EC, R6_PINT, R6_TH2, R6_NSUM };
 enum : int { R6_PHIMAX = 0, R6_PMAX, R6_NMAX };
 
-__global__ void __launch_bounds__(256) r6_energy_kernel(const double *X, const double *V, R6Consts c, double *part) {
+__global__ void __launch_bounds__(256) r6_energy_kernel(const double *X, const double *V, R6Consts c, double *part,
+                                                        unsigned *count, double *host) {
     __shared__ double scratch[(R6_NSUM + R6_NMAX) * 32];
     double S[R6_NSUM], M[R6_NMAX];
     for (int q = 0; q < R6_NSUM; q++) S[q] = 0.0;
@@ -291,6 +292,8 @@ __global__ void __launch_bounds__(256) r6_energy_kernel(const double *X, const d
         for (int a = 0; a < 3; a++) S[R6_EC] -= c.eta * p[a] * curl(th, a) * dV;
     }
     block_fold<R6_NSUM, R6_NMAX>(S, M, scratch, part);
+    // the last CTA folds the partials into host memory
+    if (last_block_done(count)) fold_rows_block<R6_NSUM, R6_NMAX>(part, gridDim.x, scratch, host);
 }
 
 }  // namespace scp

@@ -45,11 +45,12 @@ inline void plan_tiles(int N, int tw, int th, int slots, TileGrid *out, int *gri
 // odd N leaves every row unaligned anyway).  So 32-site rows stay except where
 // they pad: 16 x 16 takes 54 us at 80^3 against 62, 25 x 10 takes 107 us at
 // 97^3 (whose fourth column of 32-site tiles holds one site) against 123.
-inline void fit_tile(int N, int nt, int area, int *tw, int *th) {
+// wide, wide_area: a second limit, for fields staged `wide` sites further out.
+inline void fit_tile(int N, int nt, int area, int *tw, int *th, int wide = 0, int wide_area = 0) {
     double best = 1e300;
     for (int w = 32; w >= 16; w--) {
         int h = nt / w;
-        while (h > 1 && (w + 2) * (h + 2) > area) h--;
+        while (h > 1 && ((w + 2) * (h + 2) > area || (w + 2 + wide) * (h + 2 + wide) > (wide ? wide_area : 1 << 30))) h--;
         const double pad = (double)((N + w - 1) / w) * w * ((N + h - 1) / h) * h;
         const double cost = pad * (w == 32 ? 1.0 : w == 16 ? 1.08 : (N & 1) ? 1.12 : 1.22);
         if (cost < best - 1e-9) { best = cost; *tw = w; *th = h; }

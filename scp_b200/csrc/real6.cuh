@@ -12,14 +12,23 @@
 // -alpha curl(C) and -2 curl(B), B = (beta/2)|theta|^2 curl(phi), on phi: the
 // curl of a field that itself holds a curl, a stencil two sites wide.
 //
-// Structure.  A step is one or two ring launches: when alpha or beta is set,
-// an auxiliary launch stages phi and theta and writes C and B at every site;
-// the step launch then stages phi, theta (and C, B), evaluates every force
-// term at the site and advances the state with the fused leapfrog of the
-// other steppers.  Buffers: positions X[0..1] and momenta W, S of 6 arrays
-// (phi_0..2, theta_0..2), and 6 auxiliary arrays (C_0..2, B_0..2).
+// Structure.  A step is one launch: a CTA streams its tile column plane by
+// plane through a shared-memory ring of phi and theta, and with strain or
+// hardening (AUX) forms C and B of plane i+1 -- on its tile and one site
+// around it -- into a two-slot table while it updates plane i, whose curls of
+// C and B it reads from the table (in the plane) and from its own site's
+// values of planes i-1 and i+1 (registers).  So phi is staged two sites wide
+// and four planes deep (i, i+1, i+2 resident, i+3 in flight), theta one site
+// wide, and C and B never leave the SM.  Momenta are read one plane ahead.
+// Buffers: positions X[0..1] and momenta W, S of 6 arrays (phi_0..2,
+// theta_0..2).
+//
+// What bounds it: dependency chains at twelve warps per SM beside DRAM, 192 B
+// per site: 0.55 of a plain copy's rate at 128^3, 113 us a step against 197
+// with C and B written by a launch of their own (336 B).  Every operation that reaches the
+// state is explicitly rounded, so a run's bits do not depend on its launches.
 #pragma once
-#include "ring.cuh"
+#include "walk.cuh"
 
 namespace scp {
 
@@ -33,154 +42,313 @@ struct R6Consts {
     double damp_width, damp_rate;
 };
 
-// curl_a of the 3-vector held in ring fields f0..f0+2, central differences
-template <class V>
-__device__ __forceinline__ double ring_curl(const V &v, int f0, int a, double idx1) {
-    // curl_a = d_{a+1} F_{a+2} - d_{a+2} F_{a+1}
-    const int b = (a + 1) % 3, c = (a + 2) % 3;
-    auto d = [&](int dir, int f) {
-        return v.at(f0 + f, dir == 0, dir == 1, dir == 2) - v.at(f0 + f, -(dir == 0), -(dir == 1), -(dir == 2));
-    };
-    return (d(b, c) - d(c, b)) * idx1;
-}
+// Kernel arguments: positions x_{n+1} and the leapfrog's arrays, 6 each.
+struct R6Args {
+    const double *x;
+    int N;
+    R6Consts c;
+    LeapIO io;
+};
 
-// phi_0 phi_1 phi_2 at a ring offset
-template <class V>
-__device__ __forceinline__ double ring_P(const V &v, int di, int dj, int dk) {
-    return v.at(0, di, dj, dk) * v.at(1, di, dj, dk) * v.at(2, di, dj, dk);
-}
+template <bool AUX, int TX, int TY>
+struct R6Layout {
+    static constexpr int H = AUX ? 2 : 1;                          // halo of phi
+    static constexpr int NS = AUX ? 4 : 3;                         // ring slots
+    static constexpr int PFS = (TX + 2 * H) * (TY + 2 * H);        // phi, one field of a slot
+    static constexpr int TFS = (TX + 2) * (TY + 2);                // theta, C, B
+    static constexpr int SLOT = 3 * PFS + 3 * TFS;
+    static constexpr int NT = TX * TY;
+    static constexpr int CP = (PFS + NT - 1) / NT, CT = (TFS + NT - 1) / NT;   // copies per thread and field
+    static constexpr int AUXN = AUX ? 2 * 6 * TFS : 0;
+    static constexpr size_t smem_bytes = sizeof(double) * (size_t)(NS * SLOT + AUXN);
+};
 
-// Auxiliary fields C = curl(phi)/2 - theta and B = (beta/2)|theta|^2 curl(phi).
-struct R6Aux {
-    static constexpr int NR = 6;
-    static constexpr int MIN_CTAS = 2;
-    struct Args {
-        RingSrc<NR> src;
-        int N;
-        R6Consts c;
-        double *aux;          // 6 arrays
-    };
-    struct Carry {};
-    __device__ static void prefetch(const Args &, long long) {}
-    template <class V>
-    __device__ static void site(const Args &A, const V &v, int, int, int, long long idx, Carry &, bool) {
-        const R6Consts &c = A.c;
-        const long long N3 = c.N3;
-        double cp[3];
+template <class MODE, bool AUX, int TX, int TY>
+struct R6Tile {
+    using LY = R6Layout<AUX, TX, TY>;
+    static constexpr int H = LY::H, NS = LY::NS, L = NS - 2;   // planes beyond i that are resident
+    const R6Args &a;
+    double *ring, *aux;
+    int N, tx, ty, pp, pt;                // pitches of phi and theta rows
+    long long NN, n3;
+    int own_p, own_t;                     // own site in a phi field / a theta field
+    int ps[LY::CP], pg[LY::CP], ts[LY::CT], tg_[LY::CT];   // copies: slot offset (-1: none), plane offset
+    bool act;
+    int halo_p, halo_t;                   // the site around the tile whose C, B this thread forms (-1: none)
+
+    __device__ __forceinline__ R6Tile(const R6Args &args, double *smem, int tw)
+        : a(args), ring(smem), aux(smem + NS * LY::SLOT), N(args.N) {
+        ty = (int)threadIdx.x / tw;
+        tx = (int)threadIdx.x - ty * tw;
+        pp = tw + 2 * H;
+        pt = tw + 2;
+        NN = (long long)N * N;
+        n3 = NN * N;
+        own_p = (ty + H) * pp + tx + H;
+        own_t = (ty + 1) * pt + tx + 1;
+    }
+    __device__ __forceinline__ void begin(int k0, int j0, int nk, int nj) {
+        act = tx < nk && ty < nj;
+        const int wp = nk + 2 * H, wt = nk + 2;
 #pragma unroll
-        for (int a = 0; a < 3; a++) cp[a] = ring_curl(v, 0, a, c.idx1);
-        const double t0 = v(3), t1 = v(4), t2 = v(5);
-        if (c.alpha != 0.0) {
-            A.aux[0 * N3 + idx] = cp[0] * 0.5 - t0;
-            A.aux[1 * N3 + idx] = cp[1] * 0.5 - t1;
-            A.aux[2 * N3 + idx] = cp[2] * 0.5 - t2;
+        for (int q = 0; q < LY::CP; q++) {
+            const int h = (int)threadIdx.x + q * LY::NT, r = h / wp, col = h - r * wp;
+            ps[q] = r < nj + 2 * H ? r * pp + col : -1;
+            pg[q] = wrapi(j0 - H + r, N) * N + wrapi(k0 - H + col, N);
         }
-        if (c.beta != 0.0) {
-            const double w = 0.5 * c.beta * (t0 * t0 + t1 * t1 + t2 * t2);
 #pragma unroll
-            for (int a = 0; a < 3; a++) A.aux[(3 + a) * N3 + idx] = w * cp[a];
+        for (int q = 0; q < LY::CT; q++) {
+            const int h = (int)threadIdx.x + q * LY::NT, r = h / wt, col = h - r * wt;
+            ts[q] = r < nj + 2 ? r * pt + col : -1;
+            tg_[q] = wrapi(j0 - 1 + r, N) * N + wrapi(k0 - 1 + col, N);
+        }
+        halo_p = halo_t = -1;
+        if (AUX) {   // rows -1 and nj, columns -1 and nk (no corners)
+            const int h = threadIdx.x;
+            int r = 0, col = -2;
+            if (h < nk) { r = -1; col = h; }
+            else if (h < 2 * nk) { r = nj; col = h - nk; }
+            else if (h < 2 * nk + nj) { r = h - 2 * nk; col = -1; }
+            else if (h < 2 * nk + 2 * nj) { r = h - 2 * nk - nj; col = nk; }
+            if (col > -2) {
+                halo_p = (r + H) * pp + col + H;
+                halo_t = (r + 1) * pt + col + 1;
+            }
+        }
+    }
+    __device__ __forceinline__ void issue(int plane, int slot) {
+        const double *g = a.x + (long long)wrapi(plane, N) * NN;
+        double *sp = ring + slot * LY::SLOT, *st = sp + 3 * LY::PFS;
+#pragma unroll
+        for (int q = 0; q < LY::CP; q++)
+            if (ps[q] >= 0) {
+#pragma unroll
+                for (int f = 0; f < 3; f++) cp_async8(sp + f * LY::PFS + ps[q], g + f * n3 + pg[q]);
+            }
+#pragma unroll
+        for (int q = 0; q < LY::CT; q++)
+            if (ts[q] >= 0) {
+#pragma unroll
+                for (int f = 0; f < 3; f++) cp_async8(st + f * LY::TFS + ts[q], g + (3 + f) * n3 + tg_[q]);
+            }
+        cp_async_commit();
+    }
+    __device__ __forceinline__ const double *phi(int slot) const { return ring + slot * LY::SLOT; }
+    __device__ __forceinline__ const double *theta(int slot) const { return ring + slot * LY::SLOT + 3 * LY::PFS; }
+
+    // curl of phi at offset o of slot c, neighbours along i in slots m and p
+    __device__ __forceinline__ void curl_phi(const double *m, const double *c, const double *p, int o,
+                                             double (&cp)[3]) const {
+        const double idx1 = a.c.idx1;
+        auto d = [&](int dir, int f) {
+            const int at = f * LY::PFS + o;
+            return dir == 0 ? rsub(p[at], m[at])
+                            : dir == 1 ? rsub(c[at + pp], c[at - pp]) : rsub(c[at + 1], c[at - 1]);
+        };
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const int b = (q + 1) % 3, e = (q + 2) % 3;
+            cp[q] = rmul(rsub(d(b, e), d(e, b)), idx1);
+        }
+    }
+    // C and B from the curl of phi and theta at one site
+    __device__ __forceinline__ void fields(const double (&cp)[3], double t0, double t1, double t2, double (&C)[3],
+                                           double (&B)[3]) const {
+        const double w = rmul(0.5 * a.c.beta, rfma(t2, t2, rfma(t1, t1, rmul(t0, t0))));
+        C[0] = rfma(0.5, cp[0], -t0);
+        C[1] = rfma(0.5, cp[1], -t1);
+        C[2] = rfma(0.5, cp[2], -t2);
+#pragma unroll
+        for (int q = 0; q < 3; q++) B[q] = rmul(w, cp[q]);
+    }
+    // C, B of one plane (slot c; m, p beside it) at phi offset op / theta offset ot into table slot s
+    __device__ __forceinline__ void table(int m, int c, int p, int op, int ot, int s, double (&cp)[3], double (&C)[3],
+                                          double (&B)[3]) const {
+        curl_phi(phi(m), phi(c), phi(p), op, cp);
+        const double *t = theta(c) + ot;
+        fields(cp, t[0], t[LY::TFS], t[2 * LY::TFS], C, B);
+        double *o = aux + s * 6 * LY::TFS + ot;
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            o[q * LY::TFS] = C[q];
+            o[(3 + q) * LY::TFS] = B[q];
         }
     }
 };
 
-template <bool AUX>
-struct R6Step {
-    static constexpr int NR = AUX ? 12 : 6;
-    static constexpr int MIN_CTAS = 1;
-    struct Args {
-        RingSrc<NR> src;      // phi, theta, [C, B]
-        int N;
-        R6Consts c;
-        const double *win;
-        double *wout, *xout, *sout;
-        int *flag;
-        int first, sync, damp;
-    };
-    struct Carry {};
-    __device__ static void prefetch(const Args &A, long long idx) {
+template <class MODE, bool AUX, int TX, int TY>
+__device__ __forceinline__ void r6_item(R6Tile<MODE, AUX, TX, TY> &T, const TileGrid &tg, const Piece &pc) {
+    using LY = R6Layout<AUX, TX, TY>;
+    constexpr int NS = LY::NS, L = NS - 2, FS = LY::PFS, TS = LY::TFS;
+    const R6Args &A = T.a;
+    const R6Consts &c = A.c;
+    const int N = T.N, k0 = pc.kt * tg.tw, j0 = pc.jt * tg.th, i0 = pc.i0, i1 = pc.i1;
+    T.begin(k0, j0, min(tg.tw, N - k0), min(tg.th, N - j0));
+    const int j = j0 + T.ty, k = k0 + T.tx, own_g = j * N + k;
+    // plane q sits in slot (q - i0 + L) mod NS
+    auto slot = [&](int q) { return (q - i0 + L) % NS; };
+    __syncthreads();   // the previous item's last plane has been read
 #pragma unroll
-        for (int f = 0; f < 6; f++) prefetch_l2(A.win + f * A.c.N3 + idx);
+    for (int q = 0; q < NS; q++) T.issue(i0 - L + q, q);   // planes i0-L .. i0+1
+    double w[6], xm[6], cpc[3], Cm[2], Bm[2];   // momenta; x, and C_1, C_2, B_1, B_2 at x - i; curl phi at x
+    if (T.act) {
+#pragma unroll
+        for (int f = 0; f < 6; f++) w[f] = ld_early(A.io.win[0] + f * T.n3 + (long long)i0 * T.NN + own_g);
     }
-
-    template <class V>
-    __device__ static void site(const Args &A, const V &v, int i, int j, int k, long long idx, Carry &, bool) {
-        const R6Consts &c = A.c;
-        const long long N3 = c.N3;
-        // momenta first: their latency passes under the stencil
-        double wv[6];
+    cp_async_wait<0>();
+    __syncthreads();
+    {
+        const int sm = slot(i0 - 1), sc = slot(i0), sp = slot(i0 + 1);
+        double cp[3], C[3], B[3];
+        if (T.act) {
 #pragma unroll
-        for (int f = 0; f < 6; f++) wv[f] = A.win[f * N3 + idx];
-        const double p[3] = {v(0), v(1), v(2)}, t[3] = {v(3), v(4), v(5)};
-        const double sig = p[0] * p[0] + p[1] * p[1] + p[2] * p[2];
-        const double m2e = (c.mode == 1) ? c.ia / (1.0 + c.ib * sig) : c.m2;
-        const double ke = (c.mode == 3) ? c.kappa / (1.0 + c.kg * sig) : c.kappa;
-        const double P = p[0] * p[1] * p[2], P2 = P * P;
-        const double q = 1.0 + ke * P2;
-        const double dVdP = c.mu * P / (q * q);
-        double extra = 0.0;   // mode 3's additional -extra * phi_a
-        if (c.mode == 3 && c.kg > 0) {
-            const double D = 1.0 + c.kg * sig + c.kappa * P2;
-            extra = c.mu * c.kg * c.kappa * P2 * P2 / (D * D);
-        }
-        double cp[3], ct[3];
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            cp[a] = ring_curl(v, 0, a, c.idx1);
-            ct[a] = ring_curl(v, 3, a, c.idx1);
-        }
-        const double hel = p[0] * cp[0] + p[1] * cp[1] + p[2] * cp[2];
-        const double cp2 = cp[0] * cp[0] + cp[1] * cp[1] + cp[2] * cp[2];
-        double gP2[3] = {0.0, 0.0, 0.0};   // gradient of P^2
-        if (c.kh != 0.0) {
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-                const double Pp = ring_P(v, d == 0, d == 1, d == 2), Pm = ring_P(v, -(d == 0), -(d == 1), -(d == 2));
-                gP2[d] = (Pp * Pp - Pm * Pm) * c.idx1;
+            for (int f = 0; f < 3; f++) {
+                xm[f] = T.phi(sm)[f * FS + T.own_p];
+                xm[3 + f] = T.theta(sm)[f * TS + T.own_t];
+            }
+            if constexpr (AUX) {
+                T.curl_phi(T.phi(slot(i0 - 2)), T.phi(sm), T.phi(sc), T.own_p, cp);
+                T.fields(cp, xm[3], xm[4], xm[5], C, B);
+                Cm[0] = C[1]; Cm[1] = C[2]; Bm[0] = B[1]; Bm[1] = B[2];
+                T.table(sm, sc, sp, T.own_p, T.own_t, 0, cpc, C, B);
             }
         }
-        double acc[6];
+        if constexpr (AUX) {
+            if (T.halo_p >= 0) T.table(sm, sc, sp, T.halo_p, T.halo_t, 0, cp, C, B);
+            __syncthreads();   // plane i0-2 has been read: its slot takes plane i0+2
+            T.issue(i0 + 2, slot(i0 + 2));
+        }
+    }
+    for (int i = i0; i < i1; i++) {
+        const int sc = slot(i), sp = slot(i + 1);
+        if constexpr (AUX) cp_async_wait<0>();   // plane i+2 (without AUX the prologue or the last round waited)
+        else if (i > i0) cp_async_wait<0>();
+        __syncthreads();   // copies and the table of plane i are visible; plane i-1 and its table are free
+        if (i + L + 1 <= i1 + L - 1) T.issue(i + L + 1, slot(i + L + 1));
+        double Cn[3], Bn[3], cpn[3];
+        const int an = (i + 1 - i0) & 1;         // table slot of plane i+1
+        if constexpr (AUX) {
+            const int s2 = slot(i + 2);
+            if (T.act) T.table(sc, sp, s2, T.own_p, T.own_t, an, cpn, Cn, Bn);
+            if (T.halo_p >= 0 && i + 1 < i1) {
+                double cp[3], C[3], B[3];
+                T.table(sc, sp, s2, T.halo_p, T.halo_t, an, cp, C, B);
+            }
+        }
+        if (!T.act) continue;
+        const double *ph = T.phi(sc) + T.own_p, *php = T.phi(sp) + T.own_p;
+        const double *th = T.theta(sc) + T.own_t, *thp = T.theta(sp) + T.own_t;
+        const double p[3] = {ph[0], ph[FS], ph[2 * FS]}, t[3] = {th[0], th[TS], th[2 * TS]};
+        // neighbours of field f (phi 0-2, theta 3-5): direction d, side s
+        auto nbr = [&](int f, int d, int s) -> double {
+            if (d == 0) return s < 0 ? xm[f] : (f < 3 ? php[f * FS] : thp[(f - 3) * TS]);
+            if (f < 3) return ph[f * FS + s * (d == 1 ? T.pp : 1)];
+            return th[(f - 3) * TS + s * (d == 1 ? T.pt : 1)];
+        };
+        const double sig = rfma(p[2], p[2], rfma(p[1], p[1], rmul(p[0], p[0])));
+        const double m2e = (c.mode == 1) ? c.ia / rfma(c.ib, sig, 1.0) : c.m2;
+        const double ke = (c.mode == 3) ? c.kappa / rfma(c.kg, sig, 1.0) : c.kappa;
+        const double P = rmul(rmul(p[0], p[1]), p[2]), P2 = rmul(P, P);
+        const double q = rfma(ke, P2, 1.0);
+        const double dVdP = rmul(c.mu, P) / rmul(q, q);
+        double extra = 0.0;   // mode 3's additional -extra * phi_a
+        if (c.mode == 3 && c.kg > 0) {
+            const double D = rfma(c.kappa, P2, rfma(c.kg, sig, 1.0));
+            extra = rmul(rmul(rmul(rmul(c.mu, c.kg), c.kappa), P2), P2) / rmul(D, D);
+        }
+        double ct[3], cp[3];
 #pragma unroll
         for (int a = 0; a < 3; a++) {
             const int b = (a + 1) % 3, e = (a + 2) % 3;
-            const double lap = (v.at(a, 1, 0, 0) + v.at(a, -1, 0, 0) + v.at(a, 0, 1, 0) + v.at(a, 0, -1, 0) +
-                                v.at(a, 0, 0, 1) + v.at(a, 0, 0, -1) - 6.0 * p[a]) * c.idx2;
-            const double dPa = p[b] * p[e];   // dP / dphi_a
-            double chiral = 0.0;
+            ct[a] = rmul(rsub(rsub(nbr(3 + e, b, 1), nbr(3 + e, b, -1)), rsub(nbr(3 + b, e, 1), nbr(3 + b, e, -1))),
+                         c.idx1);
+            cp[a] = AUX ? cpc[a]
+                        : rmul(rsub(rsub(nbr(e, b, 1), nbr(e, b, -1)), rsub(nbr(b, e, 1), nbr(b, e, -1))), c.idx1);
+        }
+        const double cp2 = rfma(cp[2], cp[2], rfma(cp[1], cp[1], rmul(cp[0], cp[0])));
+        double hel = 0.0, gP2[3] = {0.0, 0.0, 0.0};   // phi . curl phi, gradient of P^2
+        if (c.kh != 0.0) {
+            hel = rfma(p[2], cp[2], rfma(p[1], cp[1], rmul(p[0], cp[0])));
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const double Pp = rmul(rmul(nbr(0, d, 1), nbr(1, d, 1)), nbr(2, d, 1));
+                const double Pm = rmul(rmul(nbr(0, d, -1), nbr(1, d, -1)), nbr(2, d, -1));
+                gP2[d] = rmul(rfma(Pp, Pp, -rmul(Pm, Pm)), c.idx1);
+            }
+        }
+        // curls of C and B: in the plane from the table, along i from this
+        // site's own values
+        double cC[3] = {0.0, 0.0, 0.0}, cB[3] = {0.0, 0.0, 0.0};
+        if constexpr (AUX) {
+            const double *ax = T.aux + ((i - i0) & 1) * 6 * TS + T.own_t;
+            auto curl = [&](const double *f, const double (&n)[3], const double (&m)[2], double (&o)[3]) {
+                auto dj = [&](int q2) { return rsub(f[q2 * TS + T.pt], f[q2 * TS - T.pt]); };
+                auto dk = [&](int q2) { return rsub(f[q2 * TS + 1], f[q2 * TS - 1]); };
+                o[0] = rmul(rsub(dj(2), dk(1)), c.idx1);
+                o[1] = rmul(rsub(dk(0), rsub(n[2], m[1])), c.idx1);
+                o[2] = rmul(rsub(rsub(n[1], m[0]), dj(0)), c.idx1);
+            };
+            curl(ax, Cn, Cm, cC);
+            curl(ax + 3 * TS, Bn, Bm, cB);
+        }
+        const double dmp = (MODE::DAMP && !MODE::FIRST) ? sponge_factor(i, j, k, c.L, c.dx, c.damp_width, c.damp_rate)
+                                                        : 1.0;
+        const long long site = (long long)i * T.NN + own_g;
+        LeapSite<MODE, 6> leap{A.io, w, T.n3, site, i + 1 < i1 ? T.NN : 0, c.hdt, c.dt, dmp};
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const int b = (a + 1) % 3, e = (a + 2) % 3;
+            auto lap = [&](int f, double x) {
+                double l = radd(nbr(f, 0, 1), nbr(f, 0, -1));
+                l = radd(radd(l, nbr(f, 1, 1)), nbr(f, 1, -1));
+                l = radd(radd(l, nbr(f, 2, 1)), nbr(f, 2, -1));
+                return rmul(rfma(-6.0, x, l), c.idx2);
+            };
+            const double dPa = rmul(p[b], p[e]);   // dP / dphi_a
+            double f = rfma(-m2e, p[a], lap(a, p[a]));
+            f = rfma(-dVdP, dPa, f);
+            f = rfma(-extra, p[a], f);
+            f = rfma(c.eta, ct[a], f);
             if (c.kh != 0.0) {
                 // kappa_h [2 P dP/dphi_a (phi.curl phi) + 2 P^2 curl_a phi + (grad P^2 x phi)_a]
-                const double cross = gP2[b] * p[e] - gP2[e] * p[b];
-                chiral = c.kh * (2.0 * P * dPa * hel + 2.0 * P2 * cp[a] + cross);
+                const double cross = rfma(gP2[b], p[e], -rmul(gP2[e], p[b]));
+                const double ch = rfma(rmul(rmul(2.0, P), dPa), hel, rfma(rmul(2.0, P2), cp[a], cross));
+                f = rfma(c.kh, ch, f);
             }
-            double f = lap - m2e * p[a] - dVdP * dPa - extra * p[a] + c.eta * ct[a] + chiral;
-            if (AUX) {
-                const double strain = -c.alpha * ring_curl(v, 6, a, c.idx1);
-                const double hard = -2.0 * ring_curl(v, 9, a, c.idx1);
-                f = f + strain + hard;
+            if constexpr (AUX) {
+                f = rfma(-c.alpha, cC[a], f);
+                f = rfma(-2.0, cB[a], f);
             }
-            acc[a] = f;
-            const double lapt = (v.at(3 + a, 1, 0, 0) + v.at(3 + a, -1, 0, 0) + v.at(3 + a, 0, 1, 0) +
-                                 v.at(3 + a, 0, -1, 0) + v.at(3 + a, 0, 0, 1) + v.at(3 + a, 0, 0, -1) - 6.0 * t[a]) *
-                                c.idx2;
-            const double strain_t = (AUX && c.alpha != 0.0) ? 2.0 * c.alpha * v(6 + a) : 0.0;
-            acc[3 + a] = lapt - c.mtheta2 * t[a] + c.eta * cp[a] + strain_t + -c.beta * cp2 * t[a];
+            double g = rfma(-c.mtheta2, t[a], lap(3 + a, t[a]));
+            g = rfma(c.eta, cp[a], g);
+            if constexpr (AUX) {
+                g = rfma(rmul(2.0, c.alpha), rfma(0.5, cp[a], -t[a]), g);   // 2 alpha C_a
+                g = rfma(rmul(-c.beta, cp2), t[a], g);
+            }
+            leap.put(a, p[a], f, dmp);
+            leap.put(3 + a, t[a], g, dmp);
         }
-        const Leap leap{c.hdt, c.dt, A.first != 0};
-        const double dmp = (A.damp && !A.first) ? sponge_at(i, j, k, c.L, c.dx, c.damp_width, c.damp_rate) : 1.0;
-        bool bad = false;
+        if (MODE::SYNC && leap.bad) atomicOr(A.io.flag, 1);
 #pragma unroll
-        for (int f = 0; f < 6; f++) {
-            double vv, wn;
-            leap(wv[f], acc[f], dmp, &vv, &wn);
-            const double x = (f < 3 ? p[f] : t[f - 3]) + c.dt * wn;
-            st_cs(A.xout + f * N3 + idx, x);
-            A.wout[f * N3 + idx] = wn;
-            if (A.sync) {
-                st_cs(A.sout + f * N3 + idx, vv);
-                bad |= !isfinite(x) || !isfinite(vv);
-            }
+        for (int f = 0; f < 3; f++) {
+            xm[f] = p[f];
+            xm[3 + f] = t[f];
         }
-        if (A.sync && bad) atomicOr(A.flag, 1);
+        if constexpr (AUX) {
+            // plane i's own C, B become those at x - i
+            const double *ax = T.aux + ((i - i0) & 1) * 6 * TS + T.own_t;
+            Cm[0] = ax[TS]; Cm[1] = ax[2 * TS]; Bm[0] = ax[4 * TS]; Bm[1] = ax[5 * TS];
+#pragma unroll
+            for (int a = 0; a < 3; a++) cpc[a] = cpn[a];
+        }
     }
-};
+}
+
+template <class MODE, bool AUX, int TX, int TY>
+__global__ void __launch_bounds__(TX *TY, 1) r6_kernel(R6Args a, TileGrid tg) {
+    extern __shared__ __align__(16) double r6_smem[];
+    R6Tile<MODE, AUX, TX, TY> T(a, r6_smem, tg.tw);
+    for_each_piece(tg, a.N, [&](const Piece &pc) { r6_item<MODE, AUX, TX, TY>(T, tg, pc); });
+}
 
 }  // namespace scp

@@ -113,10 +113,10 @@ struct scp_gpu {
     int gauged, nf, prec;
     int links;                   // th / E columns carried (complex_gauge; with g = 0 they stay constant)
     int real;                    // real 6-field mode: 12 host columns, imaginary sector held at zero
-    // real 6-field mode with optional terms: ring kernels of real6.cuh; X[0..1],
-    // W and S hold 6 arrays, raux the auxiliary C and B (strain, hardening)
+    // real 6-field mode with optional terms (real6.cuh): X[0..1], W and S hold 6
+    // arrays; raux: the strain or hardening term is on
     int rp = 0;
-    double *raux = nullptr;
+    int raux = 0;
     R6Consts r6{};
     // gauged stepper with the Higgs condensate and/or the second gauge: one
     // fused ring kernel per step (higgs_u1.cuh); X[0..1], W and S hold nx arrays
@@ -128,7 +128,7 @@ struct scp_gpu {
     double qfab[3] = {0.0, 0.0, 0.0};
     FabConsts fc{};
     double *kacc = nullptr;      // accumulated currents (3 arrays)
-    ExtPlan xplan{}, xplan2{};
+    ExtPlan xplan{};
     ExtPlan dplan{};             // first diagnostics reduction on the plane walker
     int dplan_ok = 0;
     int nx = 0;                  // position arrays per buffer of the extension layouts
@@ -807,7 +807,7 @@ static bool real_optional(const scp_gpu_params *p) {
 
 static int ext_slab(scp_gpu *h, int nx);
 
-// one step of the real mode: [auxiliary fields,] forces and fused leapfrog
+// one step of the real mode: forces and fused leapfrog
 static int r6_launch_step(scp_gpu *h, bool first, bool sync) {
     R6IO io;
     io.x = h->X[h->cur];
@@ -815,12 +815,11 @@ static int r6_launch_step(scp_gpu *h, bool first, bool sync) {
     io.win = first ? h->S : h->W;
     io.wout = h->W;
     io.sout = h->S;
-    io.aux = h->raux;
     io.flag = h->flag;
     io.first = first;
     io.sync = sync;
     io.damp = damping_on(h);
-    CK(r6_step(h->xplan2, h->xplan, h->r6, io, h->stream));
+    CK(r6_step(h->raux, h->xplan, h->r6, io, h->stream));
     h->cur ^= 1;
     return SCP_OK;
 }
@@ -831,12 +830,7 @@ static int init_real(scp_gpu *h, const double *const *cols, bool on_device) {
     const long long n3 = h->N3;
     const scp_gpu_params &p = h->p;
     if ((rc = ext_slab(h, 6))) return rc;
-    const bool aux = p.alpha_cs != 0 || p.beta_h != 0;
-    if (aux) {
-        CK(cudaMallocAsync(&h->raux, sizeof(double) * 6 * (size_t)n3, h->stream));
-        CK(cudaMemsetAsync(h->raux, 0, sizeof(double) * 6 * (size_t)n3, h->stream));
-        h->dev_bytes += sizeof(double) * 6 * n3;
-    }
+    h->raux = (p.alpha_cs != 0 || p.beta_h != 0) ? 1 : 0;
     const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     for (int c = 0; c < 12; c++)   // phi, theta, then their velocities
         CK(cudaMemcpyAsync((c < 6 ? h->X[0] + c * n3 : h->S + (c - 6) * n3), cols[c], sizeof(double) * n3, kind,
@@ -851,19 +845,16 @@ static int init_real(scp_gpu *h, const double *const *cols, bool on_device) {
     r.damp_width = p.damp_width; r.damp_rate = p.damp_rate;
     int nsm = 0;
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
-    if (r6_plan(aux, h->N, nsm, &h->xplan2, &h->xplan)) return SCP_EUNSUPPORTED;
+    if (r6_plan(h->raux, h->N, nsm, &h->xplan)) return SCP_EUNSUPPORTED;
     return r6_launch_step(h, true, false);
 }
 
 static int real_diag(scp_gpu *h, scp_gpu_diag_out *out) {
     const int nb = red_blocks(h->N3);
-    r6_energy_kernel<<<nb, kRedThreads, 0, h->stream>>>(h->X[h->cur ^ 1], h->S, h->r6, h->part);
-    fold_partials_kernel<R6_NSUM, R6_NMAX><<<1, 1024, 0, h->stream>>>(h->part, nb, h->fold);
+    r6_energy_kernel<<<nb, kRedThreads, 0, h->stream>>>(h->X[h->cur ^ 1], h->S, h->r6, h->part, h->count, h->res);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(h->h_small, h->fold, sizeof(double) * (R6_NSUM + R6_NMAX), cudaMemcpyDeviceToHost,
-                       h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    const double *f = h->h_small;
+    const double *f = h->res;
     double *o = out->v;
     for (int q = 0; q < SCP_DIAG_NSLOTS; q++) o[q] = 0.0;
     const int slot[8] = {SCP_DIAG_E_PHI_KIN, SCP_DIAG_E_THETA_KIN, SCP_DIAG_E_GRAD, SCP_DIAG_E_MASS,
@@ -1671,7 +1662,7 @@ void scp_gpu_free(scp_gpu *h) {
     if (h->copy_stream) cudaStreamSynchronize(h->copy_stream);
     if (h->stream) {
         void *bufs[] = {h->slab32, h->slab, h->part, h->fold, h->cg, h->point, h->flag, h->count, h->stage,
-                        h->snap_dev, h->raux, h->kacc, h->dpart, h->drho};
+                        h->snap_dev, h->kacc, h->dpart, h->drho};
         for (void *b : bufs)
             if (b) cudaFreeAsync(b, h->stream);
         cudaStreamSynchronize(h->stream);
