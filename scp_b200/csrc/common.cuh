@@ -71,6 +71,13 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(NPEND) : "memory");
 }
 
+// Programmatic dependent launch: a step launch's CTAs may become resident while
+// the launch before it still runs; griddep_wait returns once that launch has
+// completed and its writes are visible (at once where there is none, or for an
+// ordinary launch), griddep_launch lets the next one become resident.
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 // Bring the line holding p into L2 ahead of its use (a hint: no register, no wait).
 __device__ __forceinline__ void prefetch_line_l2(const void *p) {
     asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));

@@ -31,8 +31,7 @@ int r6_plan_of(int N, int nsm, ExtPlan *p) {
 
 template <class MODE, bool AUX>
 cudaError_t r6_launch(const ExtPlan &p, const R6Args &a, cudaStream_t st) {
-    r6_kernel<MODE, AUX, kR6X, kR6Y><<<p.grid, kR6X * kR6Y, p.smem, st>>>(a, p.tg);
-    return cudaGetLastError();
+    return launch_step_kernel(r6_kernel<MODE, AUX, kR6X, kR6Y>, a.N, p.grid, kR6X * kR6Y, p.smem, st, a, p.tg);
 }
 
 }  // namespace

@@ -348,6 +348,8 @@ template <class MODE, bool AUX, int TX, int TY>
 __global__ void __launch_bounds__(TX *TY, 1) r6_kernel(R6Args a, TileGrid tg) {
     extern __shared__ __align__(16) double r6_smem[];
     R6Tile<MODE, AUX, TX, TY> T(a, r6_smem, tg.tw);
+    griddep_wait();
+    griddep_launch();
     for_each_piece(tg, a.N, [&](const Piece &pc) { r6_item<MODE, AUX, TX, TY>(T, tg, pc); });
 }
 

@@ -469,10 +469,10 @@ static int launch_step(scp_gpu *h, bool first, bool sync) {
             fn<<<h->grid_run, h->threads, smem, h->stream>>>(io, h->c, h->tg_run);
         } else if (dg) {
             StepFnT<F64> fn = step_diag_fn(h->shape, h->gauged, damping_on(h), &smem);
-            fn<<<h->grid_diag, ts.tx * ts.ty, smem, h->stream>>>(io, h->c, h->tg_diag);
+            CK(launch_step_kernel(fn, h->N, h->grid_diag, ts.tx * ts.ty, smem, h->stream, io, h->c, h->tg_diag));
         } else {
             StepFnT<F64> fn = step_fn<F64>(h->shape, h->gauged, first, sync, damping_on(h), &smem);
-            fn<<<h->grid_run, ts.tx * ts.ty, smem, h->stream>>>(io, h->c, h->tg_run);
+            CK(launch_step_kernel(fn, h->N, h->grid_run, ts.tx * ts.ty, smem, h->stream, io, h->c, h->tg_run));
         }
     } else {
         StepIO<F32C> io;
@@ -489,10 +489,10 @@ static int launch_step(scp_gpu *h, bool first, bool sync) {
         h->dvalid = 0;
         if (h->pairs) {
             StepFnT<F32C> fn = step2_fn(h->shape, h->gauged, first, sync, damping_on(h), &smem);
-            fn<<<h->grid_run, h->threads, smem, h->stream>>>(io, h->c, h->tg_run);
+            CK(launch_step_kernel(fn, h->N, h->grid_run, h->threads, smem, h->stream, io, h->c, h->tg_run));
         } else {
             StepFnT<F32C> fn = step_fn<F32C>(h->shape, h->gauged, first, sync, damping_on(h), &smem);
-            fn<<<h->grid_run, ts.tx * ts.ty, smem, h->stream>>>(io, h->c, h->tg_run);
+            CK(launch_step_kernel(fn, h->N, h->grid_run, ts.tx * ts.ty, smem, h->stream, io, h->c, h->tg_run));
         }
     }
     CK(cudaGetLastError());

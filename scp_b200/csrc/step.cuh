@@ -913,6 +913,8 @@ __global__ void __launch_bounds__(TX * TY, (MinBlocks<P, TX, TY, GAUGED>::value)
 step_kernel(StepIO<P> io, StepConsts c, TileGrid tg) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CpStage<P, TX, TY, GAUGED> stg(smem_raw, tg.tw);
+    griddep_wait();
+    griddep_launch();
     for_each_piece(tg, c.N, [&](const Piece &pc) {
         step_one<P, TX, TY, GAUGED, FIRST>(io, c, tg, pc, SYNC, DAMP, stg);
     });
@@ -926,6 +928,8 @@ __global__ void __launch_bounds__(TX * TY, (MinBlocks<F64, TX, TY, GAUGED>::valu
 step_diag_kernel(StepIO<F64> io, StepConsts c, TileGrid tg) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CpStage<F64, TX, TY, GAUGED> stg(smem_raw, tg.tw);
+    griddep_wait();
+    griddep_launch();
     StepSums sums;
     sums.clear();
     for_each_piece(tg, c.N, [&](const Piece &pc) {

@@ -478,6 +478,8 @@ template <int TX, int TY, bool GAUGED, bool FIRST, bool SYNC, bool DAMP>
 __global__ void __launch_bounds__(Step2Layout<TX, TY, GAUGED>::NT, Step2Layout<TX, TY, GAUGED>::MIN_BLOCKS)
 step2_kernel(StepIO<F32C> io, StepConsts c, TileGrid tg) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    griddep_wait();
+    griddep_launch();
     for_each_piece(tg, c.N, [&](const Piece &pc) { step_item2<TX, TY, GAUGED, FIRST>(io, c, tg, pc, SYNC, DAMP, smem_raw); });
 }
 

@@ -176,6 +176,8 @@ template <class M, int TX, int TY>
 __global__ void __launch_bounds__(TX *TY, M::MIN_CTAS) walk_kernel(typename M::Args a, TileGrid tg) {
     extern __shared__ __align__(16) double walk_ring[];
     WalkStage<M, TX, TY> stg(walk_ring, tg.tw);
+    griddep_wait();
+    griddep_launch();
     for_each_piece(tg, a.N, [&](const Piece &pc) { walk_item<M, TX, TY>(a, tg, pc, stg); });
 }
 

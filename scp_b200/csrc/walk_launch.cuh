@@ -37,8 +37,7 @@ int walk_plan(int N, int nsm, ExtPlan *p) {
 template <class M>
 cudaError_t walk_launch(const ExtPlan &p, const typename M::Args &a, cudaStream_t st) {
     using LY = WalkLayout<M, kWalkX, kWalkY>;
-    walk_kernel<M, kWalkX, kWalkY><<<p.grid, LY::NT, LY::smem_bytes, st>>>(a, p.tg);
-    return cudaGetLastError();
+    return launch_step_kernel(walk_kernel<M, kWalkX, kWalkY>, a.N, p.grid, LY::NT, LY::smem_bytes, st, a, p.tg);
 }
 
 // run f(StepMode) for the launch's mode
