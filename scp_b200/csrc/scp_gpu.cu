@@ -1474,21 +1474,101 @@ __global__ void snap_col_kernel(View V, int field, int mom, long long n, int dty
     }
 }
 
+// Every SFA column of the current state into the staging of an asynchronous
+// snapshot, one launch: block row y takes column y.  (A launch or a copy per
+// column kept the host 167 us at 32^3, where the steps of the interval take
+// 340.)
+struct SnapCols {
+    const double *src[SCP_GPU_MAX_COLS];   // FP64 states: the column itself
+    short field[SCP_GPU_MAX_COLS], mom[SCP_GPU_MAX_COLS];
+};
+template <class View>
+__global__ void __launch_bounds__(kRedThreads) snap_pack_kernel(View V, SnapCols t, long long n, int dtype,
+                                                                void *out) {
+    const int c = blockIdx.y;
+    const double *src = t.src[c];
+    const int field = t.field[c], mom = t.mom[c];
+    const long long o = (long long)c * n;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.x * blockDim.x) {
+        double v;
+        if constexpr (std::is_same<View, ViewF64>::value) v = src[i];
+        else v = mom ? V.p(field, i) : V.q(field, i);
+        if (dtype == SCP_DTYPE_F64) ((double *)out)[o + i] = v;
+        else if (dtype == SCP_DTYPE_F32) ((float *)out)[o + i] = (float)v;
+        else ((uint16_t *)out)[o + i] = f64_to_f16_trunc(v);
+    }
+}
+
+// The page-locked allocation that holds host address p: false for pageable
+// memory, or where the driver does not say.
+static bool pinned_range(const void *p, uintptr_t *lo, uintptr_t *hi) {
+    using AttrFn = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+    static AttrFn fn = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return (AttrFn)f;
+    }();
+    unsigned type = 0;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    const CUdeviceptr d = (CUdeviceptr)(uintptr_t)p;
+    if (!fn || fn(&type, CU_POINTER_ATTRIBUTE_MEMORY_TYPE, d) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST ||
+        fn(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, d) != CUDA_SUCCESS ||
+        fn(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, d) != CUDA_SUCCESS)
+        return false;
+    *lo = (uintptr_t)start;
+    *hi = (uintptr_t)start + size;
+    return *lo <= (uintptr_t)p && (uintptr_t)p < *hi;
+}
+
+// How many of the host columns from c on (col bytes each) follow one another
+// inside one page-locked allocation, so that one copy can take them.
+static int adjacent_cols(void *const *host_cols, int c, int ncols, size_t col) {
+    int n = 1;
+    while (c + n < ncols && host_cols[c + n] == (const char *)host_cols[c] + n * col) n++;
+    if (n == 1) return 1;
+    uintptr_t lo = 0, hi = 0;
+    if (!pinned_range(host_cols[c], &lo, &hi)) return 1;
+    const size_t room = (hi - (uintptr_t)host_cols[c]) / col;
+    return (size_t)n < room ? n : (room > 0 ? (int)room : 1);
+}
+
 template <class View>
 static int snapshot_with(scp_gpu *h, const View &V, int dtype, void *const *host_cols) {
     const int ncols = snap_ncols(h);
     const long long n3 = h->N3;
     const int nb = red_blocks(n3);
     const size_t es = dtype == SCP_DTYPE_F64 ? 8 : (dtype == SCP_DTYPE_F32 ? 4 : 2);
+    if (h->prec == SCP_PREC_FP64 && dtype == SCP_DTYPE_F64) {   // straight copies of the FP64 columns
+        const double *src[SCP_GPU_MAX_COLS];
+        for (int c = 0; c < ncols; c++) {
+            if (!host_cols[c]) return SCP_EINVAL;
+            const double *Xs, *Ss;
+            int field, mom;
+            col_source(h, c, &Xs, &Ss, &field, &mom);
+            src[c] = (mom ? Ss : Xs) + (size_t)field * n3;
+        }
+        for (int c = 0; c < ncols;) {   // columns adjacent on both sides go in one copy
+            int n = 1, most = 0;
+            while (c + n < ncols && src[c + n] == src[c] + n * n3) n++;
+            if (n > 1) most = adjacent_cols(host_cols, c, c + n, sizeof(double) * n3);
+            if (most < n) n = most > 0 ? most : 1;
+            CK(cudaMemcpyAsync(host_cols[c], src[c], sizeof(double) * n3 * n, cudaMemcpyDeviceToHost, h->stream));
+            c += n;
+        }
+        CK(cudaStreamSynchronize(h->stream));
+        return SCP_OK;
+    }
     for (int c = 0; c < ncols; c++) {
         if (!host_cols[c]) return SCP_EINVAL;
         const double *Xs, *Ss;
         int field, mom;
         col_source(h, c, &Xs, &Ss, &field, &mom);
-        if (h->prec == SCP_PREC_FP64 && dtype == SCP_DTYPE_F64) {   // straight copy of the FP64 column
-            const double *src = (mom ? Ss : Xs) + (size_t)field * n3;
-            CK(cudaMemcpyAsync(host_cols[c], src, sizeof(double) * n3, cudaMemcpyDeviceToHost, h->stream));
-        } else {
+        {
             if (h->prec == SCP_PREC_FP64) {
                 ViewF64 V2{Xs, Ss, n3};
                 snap_col_kernel<ViewF64><<<nb, kRedThreads, 0, h->stream>>>(V2, field, mom, n3, dtype, h->stage);
@@ -1548,26 +1628,25 @@ static int snapshot_async_with(scp_gpu *h, const View &V, int dtype, void *const
         h->dev_bytes += need;
     }
     char *stage = (char *)h->snap_dev;
-    const int nb = red_blocks(n3);
+    SnapCols t;
     for (int c = 0; c < ncols; c++) {
         const double *Xs, *Ss;
         int field, mom;
         col_source(h, c, &Xs, &Ss, &field, &mom);
-        if (h->prec == SCP_PREC_FP64 && dtype == SCP_DTYPE_F64) {
-            const double *src = (mom ? Ss : Xs) + (size_t)field * n3;
-            CK(cudaMemcpyAsync(stage + c * col, src, col, cudaMemcpyDeviceToDevice, h->stream));
-        } else if (h->prec == SCP_PREC_FP64) {
-            ViewF64 V2{Xs, Ss, n3};
-            snap_col_kernel<ViewF64><<<nb, kRedThreads, 0, h->stream>>>(V2, field, mom, n3, dtype, stage + c * col);
-        } else {
-            snap_col_kernel<View><<<nb, kRedThreads, 0, h->stream>>>(V, field, mom, n3, dtype, stage + c * col);
-        }
+        t.src[c] = (mom ? Ss : Xs) + (size_t)field * n3;   // FP64 states
+        t.field[c] = (short)field;
+        t.mom[c] = (short)mom;
     }
+    const int bx = (int)std::min<long long>((n3 + kRedThreads - 1) / kRedThreads, 1 + 2 * kRedMaxBlocks / ncols);
+    snap_pack_kernel<View><<<dim3(bx, ncols), kRedThreads, 0, h->stream>>>(V, t, n3, dtype, stage);
     CK(cudaGetLastError());
     CK(cudaEventRecord(h->snap_ready, h->stream));
     CK(cudaStreamWaitEvent(h->copy_stream, h->snap_ready, 0));
-    for (int c = 0; c < ncols; c++)
-        CK(cudaMemcpyAsync(host_cols[c], stage + c * col, col, cudaMemcpyDeviceToHost, h->copy_stream));
+    for (int c = 0; c < ncols;) {   // host columns that follow one another take one copy
+        const int n = adjacent_cols(host_cols, c, ncols, col);
+        CK(cudaMemcpyAsync(host_cols[c], stage + c * col, n * col, cudaMemcpyDeviceToHost, h->copy_stream));
+        c += n;
+    }
     CK(cudaEventRecord(h->snap_done, h->copy_stream));
     h->snap_pending = 1;
     return SCP_OK;
