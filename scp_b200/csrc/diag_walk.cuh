@@ -41,7 +41,7 @@ struct DiagWalk {
     static constexpr int TH = 12, EF = 15;
     static constexpr int NR = 18, CF = NR;
     static constexpr int MIN_CTAS = 1;
-    static constexpr bool HALO_APART = true;
+    static constexpr bool HALO_APART = true, WIDE = false;
     static constexpr bool CONVERT = COMP;     // staged through registers, converted to FP64
     using Args = DiagWalkArgs;
     using MT = typename std::conditional<COMP, float, double>::type;

@@ -86,7 +86,7 @@ struct FabricPass {
     static constexpr int NR = 15, CF = LINKS ? 12 : 15;
     static constexpr int NM = LINKS ? 15 : 12;
     static constexpr int MIN_CTAS = 1;
-    static constexpr bool HALO_APART = true, CONVERT = false;
+    static constexpr bool HALO_APART = true, CONVERT = false, WIDE = false;
 
     struct Args {
         const double *src[2];   // this fabric's 12 matter positions; th

@@ -24,7 +24,7 @@
 //
 // What bounds it: latency at eight warps per SM.  608 B per site; with both
 // extensions a warp issues some 2000 instructions per plane (two sets of link
-// phases, two gauges' staples), 0.61 of a plain copy's rate at 128^3: 321 us a
+// phases, two gauges' staples), 0.65 of a plain copy's rate at 128^3: 303 us a
 // step against 614 with four resident planes, a sine and cosine of every
 // plaquette and the momenta loaded at their own plane.
 #pragma once
@@ -53,7 +53,7 @@ struct HiggsU1 {
     static constexpr int HF = G2 ? 18 : 15;              // the Higgs field
     static constexpr int NR = 15 + (G2 ? 3 : 0) + (HIGGS ? 1 : 0), CF = 12;
     static constexpr int MIN_CTAS = 1;
-    static constexpr bool HALO_APART = false, CONVERT = false;
+    static constexpr bool HALO_APART = false, CONVERT = false, WIDE = true;
 
     struct Args {
         const double *x;        // positions x_{n+1}, NR arrays

@@ -19,6 +19,11 @@
 //                  field by field: 375 against 397 us for a step of three
 //                  fabrics at 128^3, but 365 against 321 with the 19 fields of
 //                  the Higgs and second gauge
+//   WIDE           rows in 16-byte copies past L1 where the edge and the tile
+//                  are even: 303 against 324 us for the 19 fields of the Higgs
+//                  and second gauge, whose 155 KB ring leaves the L1 fewer
+//                  lines than their copies hold; 377 against 365 for the three
+//                  fabrics' 15
 //   Args           kernel arguments, with `int N`
 //   State          per-thread state kept along the i walk
 //   load(args, st, idx)                first plane's global loads
@@ -38,7 +43,8 @@ namespace scp {
 template <class M, int TX, int TY>
 struct WalkLayout {
     static constexpr int NR = M::NR;
-    static constexpr int FS = (TX + 2) * (TY + 2);   // ring elements of one field
+    static constexpr int OFF = M::WIDE ? 2 : 1;      // columns before the tile's first
+    static constexpr int FS = (TX + 2 * OFF) * (TY + 2);   // ring elements of one field
     static constexpr int PLANE = NR * FS;
     static constexpr int NT = TX * TY;
     static constexpr int HPT = (2 * TX + 2 * TY + 2 + NT - 1) / NT;
@@ -51,7 +57,7 @@ struct WalkStage {
     using LY = WalkLayout<M, TX, TY>;
     double *xs;
     int tx, ty, pitch, c_s, own_g, h_s, h_g, h_f0;
-    bool act;
+    bool act, wide, chunk;
 
     struct View {
         const double *p;
@@ -64,24 +70,32 @@ struct WalkStage {
     __device__ __forceinline__ WalkStage(double *ring, int tw) : xs(ring) {
         ty = (int)threadIdx.x / tw;
         tx = (int)threadIdx.x - ty * tw;
-        pitch = tw + 2;
-        c_s = (ty + 1) * pitch + tx + 1;
+        pitch = tw + 2 * LY::OFF;
+        c_s = (ty + 1) * pitch + tx + LY::OFF;
     }
     // this thread's own site and its halo copy: rows j0-1 and j0+nj, columns
     // k0-1 and k0+nk, two corners (fields from h_f0 on; M::NR: no copy)
     __device__ __forceinline__ void begin(int N, int k0, int j0, int nk, int nj) {
         act = tx < nk && ty < nj;
         own_g = (j0 + ty) * N + k0 + tx;
-        const int h = threadIdx.x;
-        int r = 0, col = 0;
+        int h = threadIdx.x, r = 0, col = 0;
         h_f0 = M::NR;
-        if (h < nk) { r = 0; col = h + 1; h_f0 = 0; }
+        chunk = false;
+        // even edges and tiles, WIDE models: rows -1 .. nj in 16-byte chunks
+        wide = M::WIDE && ((N | pitch) & 1) == 0;
+        if (wide) {
+            const int nch = nk / 2, nc = nch * (nj + 2);
+            if (h < nc) { r = h / nch; col = 1 + 2 * (h - r * nch); h_f0 = 0; chunk = true; }
+            h += 2 * nk - nc;   // the columns and corners follow
+        } else if (h < nk) { r = 0; col = h + 1; h_f0 = 0; }
         else if (h < 2 * nk) { r = nj + 1; col = h - nk + 1; h_f0 = 0; }
-        else if (h < 2 * nk + nj) { r = h - 2 * nk + 1; col = 0; h_f0 = 0; }
-        else if (h < 2 * nk + 2 * nj) { r = h - 2 * nk - nj + 1; col = nk + 1; h_f0 = 0; }
-        else if (h == 2 * nk + 2 * nj) { r = nj + 1; col = 0; h_f0 = M::CF; }
-        else if (h == 2 * nk + 2 * nj + 1) { r = 0; col = nk + 1; h_f0 = M::CF; }
-        h_s = r * pitch + col;
+        if (!chunk && h >= 2 * nk) {
+            if (h < 2 * nk + nj) { r = h - 2 * nk + 1; col = 0; h_f0 = 0; }
+            else if (h < 2 * nk + 2 * nj) { r = h - 2 * nk - nj + 1; col = nk + 1; h_f0 = 0; }
+            else if (h == 2 * nk + 2 * nj) { r = nj + 1; col = 0; h_f0 = M::CF; }
+            else if (h == 2 * nk + 2 * nj + 1) { r = 0; col = nk + 1; h_f0 = M::CF; }
+        }
+        h_s = r * pitch + col + LY::OFF - 1;
         h_g = wrapi(j0 - 1 + r, N) * N + wrapi(k0 - 1 + col, N);
     }
     // f(the number of fields this launch stages, as a constant)
@@ -115,6 +129,21 @@ struct WalkStage {
                     for (int f = 0; f < NF; f++) sb[f * LY::FS + h_s] = v[f];
                 }
             });
+        } else if (M::WIDE && wide) {
+            with_staged(a, [&](auto nf) {
+                constexpr int NF = decltype(nf)::value;
+                if (chunk) {
+#pragma unroll
+                    for (int f = 0; f < NF; f++) cp_async16(sb + f * LY::FS + h_s, M::src(a, f, n3) + pb + h_g);
+                } else if (h_f0 == 0) {
+#pragma unroll
+                    for (int f = 0; f < NF; f++) cp_async8(sb + f * LY::FS + h_s, M::src(a, f, n3) + pb + h_g);
+                }
+            });
+            if (M::CF < M::NR && h_f0 == M::CF) {
+#pragma unroll
+                for (int f = M::CF; f < M::NR; f++) cp_async8(sb + f * LY::FS + h_s, M::src(a, f, n3) + pb + h_g);
+            }
         } else if constexpr (M::HALO_APART) {
             with_staged(a, [&](auto nf) {
                 constexpr int NF = decltype(nf)::value;

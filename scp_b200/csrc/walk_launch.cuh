@@ -21,7 +21,8 @@ int walk_plan_fn(const void *fn, int N, int nsm, ExtPlan *p) {
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, LY::NT, LY::smem_bytes) != cudaSuccess || occ < 1)
         return -1;
     int tw = kWalkX, th = kWalkY;
-    fit_tile(N, LY::NT, LY::FS, &tw, &th);
+    // (w + 2)(h + 2) <= 340 with h <= 16 keeps (w + 4)(h + 2) within 360 too
+    fit_tile(N, LY::NT, (kWalkX + 2) * (kWalkY + 2), &tw, &th);
     plan_tiles(N, tw, th, nsm * occ, &p->tg, &p->grid);
     p->tx = tw;
     p->ty = th;
