@@ -640,9 +640,10 @@ def main():
     params = seeds.params_for(seed, precision=prec, device=local, tile_variant=args.tile, **over,
                               **WORKLOAD_OVER.get(args.workload, {}))
     # kernels per step: one fused launch (the Higgs / second-gauge stepper
-    # too); with three fabrics one per moving fabric plus the link update
+    # too); with three fabrics one per moving fabric, the last with the
+    # links
     fab = params.complex_gauge and params.n_fabrics == 3
-    launches_per_step = ((3 if params.mf_lock_CQ else 4) if fab else 1)
+    launches_per_step = ((2 if params.mf_lock_CQ else 3) if fab else 1)
     st = workload_state(args.workload, params)
     cols = st.cols()
     n3 = params.N ** 3

@@ -99,7 +99,7 @@ typedef struct {
      * zero = the default terms): mass mode 1 (m_eff^2 = inv_alpha/(1+inv_beta|phi|^2))
      * or 3 (kappa_eff = kappa/(1+kappa_gamma|phi|^2)), Cosserat strain alpha_cs,
      * curl-squared hardening beta_h, chiral helicity kappa_h.  With any of them set the
-     * real mode runs on its own FP64 plane-ring kernels (FP32C refused). */
+     * real mode runs on its own FP64 kernel, one launch per step (FP32C refused). */
     int32_t mode;
     double  inv_alpha, inv_beta, kappa_gamma, alpha_cs, beta_h, kappa_h;
     /* Extensions of the gauged stepper (complex_gauge=1 and g_gauge != 0; ignored
@@ -109,7 +109,7 @@ typedef struct {
      * higgs_rvoid (scp_sim.c:2802-2817).  Second compact U(1) gauge (g_gauge2 != 0)
      * with per-component charges gauge2_q[3] (scp_config.h:97-103); its links and
      * field start at zero and are Gauss-projected at init.  Either runs on one fused
-     * FP64 plane-ring kernel per step. */
+     * FP64 kernel per step. */
     double  higgs_v, higgs_lam, higgs_kap, higgs_rvoid;
     double  g_gauge2;
     double  gauge2_q[3];
@@ -119,7 +119,8 @@ typedef struct {
      * q_fab[f] (q_C, q_Q, q_L); the Gauss law uses sum_f q_f rho_f.  mf_lock_CQ = 1
      * keeps Q equal to C at every step (the Q columns passed to init are then
      * ignored); 0 evolves Q on its own (scp_config.h:135-149).  A step is one FP64
-     * plane-ring kernel per fabric and one for the links. */
+     * kernel per moving fabric (two with Q locked), the last of which moves the
+     * links too. */
     int32_t n_fabrics;
     int32_t mf_lock_CQ;
     double  q_fab[3];

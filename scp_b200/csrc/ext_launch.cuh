@@ -1,6 +1,6 @@
-// ext_launch.cuh -- host-side launchers of the extension steppers' ring
-// kernels (higgs_u1.cuh, fabrics.cuh), instantiated in kern_ext.cu so they
-// compile in their own nvcc process.
+// ext_launch.cuh -- host-side launchers of the extension steppers' kernels
+// (higgs_u1.cuh in kern_higgs.cu, fabrics.cuh in kern_fabric.cu, real6.cuh in
+// kern_real.cu: each compiles in its own nvcc process).
 #pragma once
 #include <cuda_runtime.h>
 #include <stddef.h>
@@ -13,7 +13,7 @@ struct HuConsts;
 struct FabConsts;
 struct R6Consts;
 
-// Launch geometry of one ring kernel: tile shape, work items, CTAs.
+// Launch geometry of one such kernel: tile shape, work items, CTAs.
 struct ExtPlan {
     int tx = 0, ty = 0;
     TileGrid tg{};

@@ -2,7 +2,8 @@
 // steppers (higgs_u1.cuh, fabrics.cuh): the Higgs start value and energy, the
 // second Gauss law and its projection, the fabrics' EM charge density, Gauss
 // residual, charges and the view of fabric L for the energy reductions.
-// Host translation unit scp_gpu.cu only (the ring kernels live in kern_ext.cu).
+// Host translation unit scp_gpu.cu only (the step kernels live in
+// kern_higgs.cu, kern_fabric.cu and kern_real.cu).
 #pragma once
 #include "fabrics.cuh"
 #include "gauss.cuh"

@@ -1,7 +1,7 @@
 // higgs_u1.cuh -- the gauged stepper with the Higgs condensate and/or the
 // second compact U(1) (the reference's v71 extensions of the gauged force,
 // sfa/sim/scp_sim.c:1053-1263; its energy :1970-1975; the second Gauss
-// projection :2400-2458), as one fused ring kernel per time step.
+// projection :2400-2458), as one fused kernel per time step.
 //
 // Physics.  The Higgs field H is a real scalar with
 //     V_H = (lambda/4)(H^2 - v^2)^2 + (kappa_H/2) s H^2,   s = prod_a |Phi_a|^2,
