@@ -150,7 +150,8 @@ struct scp_gpu {
     int *flag = nullptr;
     unsigned *count = nullptr;   // last-CTA counter of the fused CG launches
     double h_small[64];          // host landing area of the small device-to-host reads
-    double *res = nullptr;       // page-locked: the folded values of a diagnostics call, written by the device
+    struct ResultSlot *slot = nullptr;
+    double *res = nullptr;       // slot's, page-locked: the folded values of a diagnostics call, written by the device
     void *stage = nullptr;       // snapshot down-conversion staging (N3 doubles)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // asynchronous snapshots: device staging of every column, copies on their own stream
@@ -336,8 +337,8 @@ static bool encode_mom_map(const double *W, int N, int nf, int tx, int ty, CUten
 // two tile rows along j, and are selected by SCP_STAGING in the environment:
 // tma (1: TMA tile loads of the positions) or cpm (2: the cp.async position
 // ring with TMA-staged momenta).  Both give the same bits as the default and
-// ran slower on B200 (0.282 and 0.296 against 0.227 ms per 128^3 gauged
-// step): the step is bound by shared-memory traffic and FP64 dependency
+// ran slower on B200 (0.233 and 0.271 against 0.198 ms per 128^3 gauged
+// step on 32 x 4 tiles): the step is bound by shared-memory traffic and FP64 dependency
 // chains, which the TMA forms do not shorten.
 static int staging_mode(const scp_gpu *h, int shape) {
     if (h->prec != SCP_PREC_FP64 || (shape != 1 && shape != 2)) return 0;
@@ -667,25 +668,59 @@ static thread_local int t_stream_priority = 0;
 // Page-locked slots of DF_N doubles for the results of diagnostics calls: a
 // block of 256 is pinned when none is free (pinning costs the better part of a
 // millisecond, and the server makes and frees handles at a high rate), a slot
-// returns to the free list with its handle.
+// returns to the free list with its handle.  A block dies with the context
+// that pinned it (cudaDeviceReset), so a slot is handed out only in that
+// context, told by its id; the list's nodes outlive it.
+struct ResultSlot {
+    double *p;
+    unsigned long long ctx;
+    ResultSlot *next;
+};
 static std::mutex g_res_mu;
-static std::vector<double *> g_res_free;
-static double *result_slot() {
-    constexpr int kBlock = 256;
-    std::lock_guard<std::mutex> lk(g_res_mu);
-    if (g_res_free.empty()) {
-        void *p = nullptr;
-        if (cudaHostAlloc(&p, sizeof(double) * DF_N * kBlock, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
-            return nullptr;
-        for (int q = kBlock - 1; q >= 0; q--) g_res_free.push_back((double *)p + (size_t)q * DF_N);
-    }
-    double *r = g_res_free.back();
-    g_res_free.pop_back();
-    return r;
+static ResultSlot *g_res_free = nullptr;
+
+static unsigned long long context_id() {
+    using IdFn = CUresult (*)(CUcontext, unsigned long long *);
+    static IdFn fn = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return (IdFn)f;
+    }();
+    unsigned long long id = 0;
+    if (fn && fn(nullptr, &id) != CUDA_SUCCESS) id = 0;   // of the current context
+    return id;
 }
-static void result_slot_free(double *r) {
+
+static ResultSlot *result_slot() {
+    constexpr int kBlock = 256;
+    const unsigned long long ctx = context_id();
     std::lock_guard<std::mutex> lk(g_res_mu);
-    g_res_free.push_back(r);
+    for (ResultSlot **at = &g_res_free; *at; at = &(*at)->next)
+        if ((*at)->ctx == ctx) {
+            ResultSlot *r = *at;
+            *at = r->next;
+            return r;
+        }
+    void *p = nullptr;
+    auto *n = (ResultSlot *)malloc(sizeof(ResultSlot) * kBlock);
+    if (!n) return nullptr;
+    if (cudaHostAlloc(&p, sizeof(double) * DF_N * kBlock, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+        free(n);
+        return nullptr;
+    }
+    for (int q = kBlock - 1; q >= 0; q--) {
+        n[q] = ResultSlot{(double *)p + (size_t)q * DF_N, ctx, g_res_free};
+        if (q) g_res_free = &n[q];
+    }
+    return n;
+}
+static void result_slot_free(ResultSlot *r) {
+    std::lock_guard<std::mutex> lk(g_res_mu);
+    r->next = g_res_free;
+    g_res_free = r;
 }
 
 static int alloc_common(scp_gpu *h) {
@@ -694,7 +729,8 @@ static int alloc_common(scp_gpu *h) {
     CK(cudaMallocAsync(&h->part, sizeof(double) * kRedMaxBlocks * 32, h->stream));
     CK(cudaMallocAsync(&h->fold, sizeof(double) * DF_N, h->stream));
     CK(cudaMemsetAsync(h->fold, 0, sizeof(double) * DF_N, h->stream));
-    if (!(h->res = result_slot())) return SCP_ENOMEM;
+    if (!(h->slot = result_slot())) return SCP_ENOMEM;
+    h->res = h->slot->p;
     CK(cudaMallocAsync(&h->cg, sizeof(double) * 16, h->stream));
     CK(cudaMallocAsync(&h->point, sizeof(double) * 8, h->stream));
     CK(cudaMallocAsync(&h->flag, sizeof(int), h->stream));
@@ -1746,7 +1782,7 @@ void scp_gpu_free(scp_gpu *h) {
             if (b) cudaFreeAsync(b, h->stream);
         cudaStreamSynchronize(h->stream);
     }
-    if (h->res) result_slot_free(h->res);
+    if (h->slot) result_slot_free(h->slot);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
     if (h->snap_ready) cudaEventDestroy(h->snap_ready);

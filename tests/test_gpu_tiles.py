@@ -3,6 +3,9 @@ real mode's fused terms, the packed frames and the diagnostics of compensated
 states, at the grid edges where a tile, a row or a launch mode changes."""
 import ctypes
 import dataclasses
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -149,3 +152,26 @@ def test_frames_into_any_columns(gpu, precision, dtype, npd):
                     sim.snapshot(dtype, out=cols)
                 for a, b in zip(cols, want):
                     assert np.array_equal(a, b)
+
+
+AFTER_RESET = """
+import ctypes, glob
+from scp_b200 import seeds
+from scp_b200.api import Simulation
+rt = ctypes.CDLL(glob.glob("/usr/local/cuda/lib64/libcudart.so*")[0])
+st = seeds.small_state(24, True, seed=3)
+got = []
+for _ in range(2):
+    with Simulation(st.params, st.cols()) as sim:
+        sim.step(3)
+        got.append(sim.diag())
+    assert rt.cudaDeviceReset() == 0
+assert got[0] == got[1]
+"""
+
+
+def test_diagnostics_after_a_device_reset(gpu):
+    """Page-locked result slots die with their context: a handle made after a
+    reset takes none of the old ones."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", AFTER_RESET], cwd=root, check=True, timeout=120)
