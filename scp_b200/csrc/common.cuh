@@ -108,10 +108,24 @@ __device__ __forceinline__ double link_wrap(double v) {
 }
 
 // A load that stays where it is written: the compiler does not move it down to
-// its first use, so its latency passes under what follows.
+// its first use, so its latency passes under what follows, nor above
+// griddep_wait.  An ordinary (coherent) load: a step reads momenta that it
+// overwrites itself and, as a dependent launch, that the launch before it may
+// still be writing while this one is already resident; the read-only path
+// (ld.global.nc, __ldg) promises nothing for such data.
 __device__ __forceinline__ double ld_early(const double *p) {
     double v;
-    asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_early(const float *p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint16_t ld_early(const uint16_t *p) {
+    uint16_t v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
     return v;
 }
 

@@ -56,7 +56,8 @@ struct DiagWalk {
     __device__ static __forceinline__ const double *src(const Args &a, int f, long long n3) {
         return f < TH ? a.x + f * n3 : f < EF ? a.th + (f - TH) * n3 : a.E + (f - EF) * n3;
     }
-    // staged field f of a compensated state
+    // staged field f of a compensated state (read-only loads: no launch in
+    // flight writes a state whose diagnostics are taken)
     __device__ static __forceinline__ double value(const Args &a, int f, long long n3, long long at) {
         if (f < TH) return (double)__ldg(a.x32 + f * n3 + at) + (double)bf16_to_f(__ldg(a.lo + f * n3 + at));
         if (f < EF) return (double)__ldg(a.x32 + f * n3 + at) + (double)__ldg(a.tlo + (f - TH) * n3 + at);

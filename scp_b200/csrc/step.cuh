@@ -109,9 +109,6 @@ struct StepLayout {
 __device__ __forceinline__ void cp_async_elem(double *s, const double *g) { cp_async8(s, g); }
 __device__ __forceinline__ void cp_async_elem(float *s, const float *g) { cp_async4(s, g); }
 
-__device__ __forceinline__ double ldg_t(const double *p) { return __ldg(p); }
-__device__ __forceinline__ float ldg_t(const float *p) { return __ldg(p); }
-
 __device__ __forceinline__ float bf16_to_f(uint16_t h) { return __uint_as_float((uint32_t)h << 16); }
 __device__ __forceinline__ uint16_t f_to_bf16(float f) {
     return __bfloat16_as_ushort(__float2bfloat16_rn(f));
@@ -279,8 +276,18 @@ __device__ __forceinline__ void step_sums(const StepSums &t, const C &c, DiagSum
 }
 
 // The site's momenta w_n, read one plane ahead: each is replaced by the next
-// plane's as soon as its kick has used it, so a load has a whole plane of
-// arithmetic to pass under.
+// plane's once its kick has used it, so a load has a whole plane of arithmetic
+// to pass under.
+//
+// Where the loads stand.  They are ordinary loads of memory that this launch
+// also stores to, so the compiler keeps them where they are written among the
+// stores, and the place matters (us a step, loads ahead of a component's stores
+// against the form taken): without links each between its component's two
+// stores (113^3 138 -> 123, 160^3 292 -> 281, 128^3 144 -> 145); with links
+// Phi's like that and Theta's as one batch once the triplet's stores are out
+// (128^3 190 -> 183, 192^3 582 -> 563, 113^3 187 -> 185; Theta's like Phi's
+// 128^3 189, 192^3 577, 113^3 172).  All of them at the end of the site: 197 at
+// 128^3 with links.
 template <bool GAUGED>
 struct Momenta {
     double v[GAUGED ? 15 : 12];
@@ -323,10 +330,10 @@ struct SiteUpdate {
     __device__ __forceinline__ double put(int f, double x, double a) {
         double wn;
         const double v = kick(mom(f), a, &wn);
-        ahead(f);
         const double xn = rfma(c.dt, wn, x);
-        st_cs(io.xout + f * c.N3 + site, xn);
         io.wout[f * c.N3 + site] = wn;
+        if (!GAUGED || f < FTU) ahead(f);
+        st_cs(io.xout + f * c.N3 + site, xn);
         if (SYNC && !FIRST) {
             st_cs(io.sout + f * c.N3 + site, v);
             bad |= !isfinite(xn) || !isfinite(v);
@@ -352,8 +359,12 @@ struct SiteUpdate {
             rho += q;
         }
     }
-    // potential terms: squared moduli of Phi, den = 1 + kappa s
+    // potential terms: squared moduli of Phi, den = 1 + kappa s; Theta is done
     __device__ __forceinline__ void moduli(const double (&s)[3], double den) {
+        if constexpr (GAUGED) {
+#pragma unroll
+            for (int f = 0; f < 6; f++) ahead(FTU + f);
+        }
         if constexpr (DIAG) {
             const double s3 = s[0] * s[1] * s[2];
             rho2 = s[0] + s[1] + s[2];
@@ -375,7 +386,6 @@ struct SiteUpdate {
     __device__ __forceinline__ void link(int d, double th0, double K) {
         double Eh;
         const double E = kick(mom(FTH + d), K, &Eh);
-        ahead(FTH + d);
         const double th = link_wrap(rfma(c.gad, Eh, th0));
         st_cs(io.xout + (FTH + d) * c.N3 + site, th);
         io.wout[(FTH + d) * c.N3 + site] = Eh;
@@ -383,6 +393,7 @@ struct SiteUpdate {
             st_cs(io.sout + (FTH + d) * c.N3 + site, E);
             bad |= !isfinite(E) || !isfinite(th);
         }
+        ahead(FTH + d);
         if constexpr (DIAG) sums->s[SS_EE] += E * E;
     }
 };
@@ -632,6 +643,9 @@ __device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepCo
 #pragma unroll
                 for (int f = 0; f < NF; f++) prefetch_line_l2(io.win + f * N3 + site + (long long)N * N);
             }
+            // momenta and low parts of this plane; without links kept at the top
+            // (113^3 115 us a step against 119, 151^3 224 against 233), with
+            // links where the compiler puts them (151^3 304 against 311)
             T w[NF];
             uint16_t lo[P::COMP ? 12 : 1];
             if (act) {
@@ -640,11 +654,11 @@ __device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepCo
                     for (int f = 0; f < NF; f++) w[f] = stg.mom((i - i0) & 1, f);
                 } else {
 #pragma unroll
-                    for (int f = 0; f < NF; f++) w[f] = ldg_t(io.win + f * N3 + site);
+                    for (int f = 0; f < NF; f++) w[f] = GAUGED ? io.win[f * N3 + site] : ld_early(io.win + f * N3 + site);
                 }
                 if constexpr (P::COMP) {
 #pragma unroll
-                    for (int f = 0; f < 12; f++) lo[f] = __ldg(io.loin + f * N3 + site);
+                    for (int f = 0; f < 12; f++) lo[f] = GAUGED ? io.loin[f * N3 + site] : ld_early(io.loin + f * N3 + site);
                 }
             }
             if (!act) continue;

@@ -265,10 +265,10 @@ __device__ __forceinline__ void duo_item(const StepIO<F64> &io, const StepConsts
         if (act) {
             if (role == 0) {
 #pragma unroll
-                for (int f = 0; f < 6; f++) w[f] = __ldg(io.win + (FU + f) * N3 + site);
+                for (int f = 0; f < 6; f++) w[f] = io.win[(FU + f) * N3 + site];
             } else {
 #pragma unroll
-                for (int f = 0; f < 9; f++) w[f] = __ldg(io.win + (FTU + f) * N3 + site);
+                for (int f = 0; f < 9; f++) w[f] = io.win[(FTU + f) * N3 + site];
             }
             double dmp = 1.0;
             if (DAMP && !FIRST) {
