@@ -75,13 +75,14 @@ __device__ __forceinline__ void fabric_current(const V &c, const V &p, int fth, 
 }
 
 // One fabric's matter step.  The force uses links of charge qf; the current
-// g qf J(qf) goes to the accumulator, preceded, with SECOND, by g qx J(qx)
+// g qf J(qf) goes to the accumulator, joined, with SECOND, by g qx J(qx)
 // over the same fields (the locked pair's C current), and with ACC added to
 // what the fabrics before left there.  With LINKS the launch
 // also steps the shared links with the accumulated currents.
 template <class MODE, bool SECOND, bool ACC, bool LINKS>
 struct FabricPass {
     static_assert(!LINKS || ACC, "the links come with the last fabric");
+    static_assert(!SECOND || !ACC, "the locked pair comes first");
     static constexpr int TH = 12;
     static constexpr int NR = 15, CF = LINKS ? 12 : 15;
     static constexpr int NM = LINKS ? 15 : 12;
@@ -125,7 +126,7 @@ struct FabricPass {
         const Args &A;
         State &st;
         LeapSite<MODE, NM> &leap;
-        double (&kx)[3];        // g qx J(qx) dx (SECOND)
+        double (&k0)[3];        // SECOND: J(qf), until J(qx) joins it
         __device__ __forceinline__ void theta(int a, double u, double v, double au, double av) {
             leap.put(FTU + a, u, au, leap.dmp);
             leap.put(FTV + a, v, av, leap.dmp);
@@ -138,8 +139,11 @@ struct FabricPass {
         __device__ __forceinline__ void angles(double, double, double) {}
         // the fabric's current on top of what the others left
         __device__ __forceinline__ double current(int d, double K) {
+            if (SECOND) {
+                k0[d] = K;
+                return K;
+            }
             double t = rmul(A.gqf, K);
-            if (SECOND) t = rfma(A.gqx, kx[d], t);
             if (ACC) t = radd(st.kin[d], t);
             if (ACC) st.kin[d] = ld_early(A.kacc + d * A.c.N3 + leap.site + leap.next);
             if (!LINKS) A.kacc[d * A.c.N3 + leap.site] = t;
@@ -157,11 +161,22 @@ struct FabricPass {
         const double dmp = (MODE::DAMP && !MODE::FIRST)
                                ? sponge_factor(i, j, k, fc.L, fc.dx, fc.damp_width, fc.damp_rate) : 1.0;
         LeapSite<MODE, NM> leap{A.io, st.w, fc.N3, idx, next, fc.hdt, fc.dt, dmp};
-        double kx[3];
-        if (SECOND) fabric_current(c, p, TH, A.qx, fc.cross, kx);
-        Out out{A, st, leap, kx};
+        double k0[3];
+        Out out{A, st, leap, k0};
         GaugedSums none;
         gauged_site<false, true, LINKS>(c, p, TH, st.cy, GaugedConsts(fc), out, none, A.qf);
+        if (SECOND) {
+            // The current under qx follows the force, behind a fence that keeps
+            // the compiler from holding the neighbours it reads in registers
+            // meanwhile: ahead of the force it spilled 256 bytes a thread
+            // (locked pair with q_C != 0, a step at 128^3 559 us against 378,
+            // at 113^3 498 against 381)
+            asm volatile("" ::: "memory");
+            double kx[3];
+            fabric_current(c, p, TH, A.qx, fc.cross, kx);
+#pragma unroll
+            for (int d = 0; d < 3; d++) A.kacc[d * fc.N3 + idx] = rfma(A.gqx, kx[d], rmul(A.gqf, k0[d]));
+        }
         if (MODE::SYNC && leap.bad) atomicOr(A.io.flag, 1);
     }
 };
