@@ -68,14 +68,20 @@ inline void plan_tiles(int N, int tw, int th, int slots, TileGrid *out, int *gri
 // odd N leaves every row unaligned anyway).  So 32-site rows stay except where
 // they pad: 16 x 16 takes 54 us at 80^3 against 62, 25 x 10 takes 107 us at
 // 97^3 (whose fourth column of 32-site tiles holds one site) against 123.
+// FP32C with one site a thread (odd N) pays more for leaving 32-site rows, which
+// are one line: with the sponge 27 x 4 tiles 59 against 56 us at 81^3, 22 x 5 76
+// against 69 at 85^3 and 19 x 6 168 against 155 at 113^3 with 16, 11 and 12 %
+// fewer padded sites, 17 x 7 106 against 111 at 97^3 (no sponge) with 22 %
+// fewer; 16 x 8 has no advantage there (52 against 46 us of 25 x 5 at 73^3).
+// All counted 1.25.
 // wide, wide_area: a second limit, for fields staged `wide` sites further out.
-inline void fit_tile(int N, int nt, int area, int *tw, int *th, int wide = 0, int wide_area = 0) {
+inline void fit_tile(int N, int nt, int area, int *tw, int *th, int wide = 0, int wide_area = 0, bool fp32 = false) {
     double best = 1e300;
     for (int w = 32; w >= 16; w--) {
         int h = nt / w;
         while (h > 1 && ((w + 2) * (h + 2) > area || (w + 2 + wide) * (h + 2 + wide) > (wide ? wide_area : 1 << 30))) h--;
         const double pad = (double)((N + w - 1) / w) * w * ((N + h - 1) / h) * h;
-        const double cost = pad * (w == 32 ? 1.0 : w == 16 ? 1.08 : (N & 1) ? 1.12 : 1.22);
+        const double cost = pad * (w == 32 ? 1.0 : fp32 ? 1.25 : w == 16 ? 1.08 : (N & 1) ? 1.12 : 1.22);
         if (cost < best - 1e-9) { best = cost; *tw = w; *th = h; }
     }
 }
