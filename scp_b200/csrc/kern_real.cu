@@ -21,7 +21,7 @@ int r6_plan_of(int N, int nsm, ExtPlan *p) {
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, LY::NT, LY::smem_bytes) != cudaSuccess || occ < 1)
         return -1;
     int tw = kR6X, th = kR6Y;
-    fit_tile(N, LY::NT, LY::TFS, &tw, &th, 2 * (LY::H - 1), LY::PFS);
+    fit_tile(N, LY::NT, LY::TFS, &tw, &th, {2 * (LY::H - 1), 2 * (LY::H - 1), LY::PFS});
     plan_tiles(N, tw, th, nsm * occ, &p->tg, &p->grid);
     p->tx = tw;
     p->ty = th;

@@ -74,12 +74,16 @@ inline void plan_tiles(int N, int tw, int th, int slots, TileGrid *out, int *gri
 // fewer padded sites, 17 x 7 106 against 111 at 97^3 (no sponge) with 22 %
 // fewer; 16 x 8 has no advantage there (52 against 46 us of 25 x 5 at 73^3).
 // All counted 1.25.
-// wide, wide_area: a second limit, for fields staged `wide` sites further out.
-inline void fit_tile(int N, int nt, int area, int *tw, int *th, int wide = 0, int wide_area = 0, bool fp32 = false) {
+// more: a second limit, for fields staged further out (or rows of more columns).
+struct WiderStage {
+    int cols = 0, rows = 0;   // staged beyond the tile's (w + 2) x (h + 2)
+    int area = 1 << 30;       // ring elements of one such field
+};
+inline void fit_tile(int N, int nt, int area, int *tw, int *th, const WiderStage &more = {}, bool fp32 = false) {
     double best = 1e300;
     for (int w = 32; w >= 16; w--) {
         int h = nt / w;
-        while (h > 1 && ((w + 2) * (h + 2) > area || (w + 2 + wide) * (h + 2 + wide) > (wide ? wide_area : 1 << 30))) h--;
+        while (h > 1 && ((w + 2) * (h + 2) > area || (w + 2 + more.cols) * (h + 2 + more.rows) > more.area)) h--;
         const double pad = (double)((N + w - 1) / w) * w * ((N + h - 1) / h) * h;
         const double cost = pad * (w == 32 ? 1.0 : fp32 ? 1.25 : w == 16 ? 1.08 : (N & 1) ? 1.12 : 1.22);
         if (cost < best - 1e-9) { best = cost; *tw = w; *th = h; }

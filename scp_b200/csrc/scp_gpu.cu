@@ -421,7 +421,7 @@ static int setup_launch(scp_gpu *h) {
     if (h->p.tile_variant == 0 && pairs)
         fit_pair_tile(h->N, &tw, &th);
     else if (h->p.tile_variant == 0 && h->tma == 0)
-        fit_tile(h->N, ts.tx * ts.ty, (ts.tx + 2) * (ts.ty + 2), &tw, &th, 0, 0, h->prec == SCP_PREC_FP32C);
+        fit_tile(h->N, ts.tx * ts.ty, (ts.tx + 2) * (ts.ty + 2), &tw, &th, {}, h->prec == SCP_PREC_FP32C);
     plan_tiles(h->N, tw, th, nsm * occ, &h->tg, &h->grid);
     h->tg_run = h->tg;
     h->grid_run = h->grid;

@@ -42,6 +42,7 @@ namespace scp {
 
 template <class M, int TX, int TY>
 struct WalkLayout {
+    static constexpr int TX_ = TX, TY_ = TY;
     static constexpr int NR = M::NR;
     static constexpr int OFF = M::WIDE ? 2 : 1;      // columns before the tile's first
     static constexpr int FS = (TX + 2 * OFF) * (TY + 2);   // ring elements of one field

@@ -12,6 +12,16 @@ namespace {
 // registers a thread, as the gauged FP64 step.
 constexpr int kWalkX = 32, kWalkY = 8;
 
+// the tile of a grid edge: its rows, with the columns its staging keeps on
+// either side, fit a ring field
+template <class LY>
+void walk_tile(int N, int *tw, int *th) {
+    constexpr int X = LY::TX_, Y = LY::TY_;
+    *tw = X;
+    *th = Y;
+    fit_tile(N, LY::NT, (X + 2) * (Y + 2), tw, th, {2 * (LY::OFF - 1), 0, LY::FS});
+}
+
 template <class M>
 int walk_plan_fn(const void *fn, int N, int nsm, ExtPlan *p) {
     using LY = WalkLayout<M, kWalkX, kWalkY>;
@@ -20,9 +30,8 @@ int walk_plan_fn(const void *fn, int N, int nsm, ExtPlan *p) {
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, LY::NT, LY::smem_bytes) != cudaSuccess || occ < 1)
         return -1;
-    int tw = kWalkX, th = kWalkY;
-    // (w + 2)(h + 2) <= 340 with h <= 16 keeps (w + 4)(h + 2) within 360 too
-    fit_tile(N, LY::NT, (kWalkX + 2) * (kWalkY + 2), &tw, &th);
+    int tw, th;
+    walk_tile<LY>(N, &tw, &th);
     plan_tiles(N, tw, th, nsm * occ, &p->tg, &p->grid);
     p->tx = tw;
     p->ty = th;
