@@ -21,6 +21,7 @@
 #include "diag_walk.cuh"
 #include "gauss.cuh"
 #include "reduce.cuh"
+#include "result_slots.h"
 #include "snapshot.cuh"
 #include "spectral.cuh"
 #include "launch.cuh"
@@ -150,7 +151,7 @@ struct scp_gpu {
     int *flag = nullptr;
     unsigned *count = nullptr;   // last-CTA counter of the fused CG launches
     double h_small[64];          // host landing area of the small device-to-host reads
-    struct ResultSlot *slot = nullptr;
+    ResultSlot *slot = nullptr;
     double *res = nullptr;       // slot's, page-locked: the folded values of a diagnostics call, written by the device
     void *stage = nullptr;       // snapshot down-conversion staging (N3 doubles)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -665,20 +666,19 @@ static void keep_pool(int dev) {
 // the running chunks instead of queueing behind them.
 static thread_local int t_stream_priority = 0;
 
-// Page-locked slots of DF_N doubles for the results of diagnostics calls: a
-// block of 256 is pinned when none is free (pinning costs the better part of a
-// millisecond, and the server makes and frees handles at a high rate), a slot
-// returns to the free list with its handle.  A block dies with the context
-// that pinned it (cudaDeviceReset), so a slot is handed out only in that
-// context, told by its id; the list's nodes outlive it.
-struct ResultSlot {
-    double *p;
-    unsigned long long ctx;
-    ResultSlot *next;
+// Page-locked slots of DF_N doubles for the results of diagnostics calls.
+struct PinnedMem {
+    static double *alloc(size_t bytes) {
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) return (double *)p;
+        cudaGetLastError();   // reported by the caller, not by the next launch's check
+        return nullptr;
+    }
+    static void free(double *p) { cudaFreeHost(p); }
 };
-static std::mutex g_res_mu;
-static ResultSlot *g_res_free = nullptr;
+static SlotPool<PinnedMem, DF_N> g_slots;
 
+// id of the current context (0 where the driver does not say)
 static unsigned long long context_id() {
     using IdFn = CUresult (*)(CUcontext, unsigned long long *);
     static IdFn fn = [] {
@@ -694,42 +694,13 @@ static unsigned long long context_id() {
     return id;
 }
 
-static ResultSlot *result_slot() {
-    constexpr int kBlock = 256;
-    const unsigned long long ctx = context_id();
-    std::lock_guard<std::mutex> lk(g_res_mu);
-    for (ResultSlot **at = &g_res_free; *at; at = &(*at)->next)
-        if ((*at)->ctx == ctx) {
-            ResultSlot *r = *at;
-            *at = r->next;
-            return r;
-        }
-    void *p = nullptr;
-    auto *n = (ResultSlot *)malloc(sizeof(ResultSlot) * kBlock);
-    if (!n) return nullptr;
-    if (cudaHostAlloc(&p, sizeof(double) * DF_N * kBlock, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-        free(n);
-        return nullptr;
-    }
-    for (int q = kBlock - 1; q >= 0; q--) {
-        n[q] = ResultSlot{(double *)p + (size_t)q * DF_N, ctx, g_res_free};
-        if (q) g_res_free = &n[q];
-    }
-    return n;
-}
-static void result_slot_free(ResultSlot *r) {
-    std::lock_guard<std::mutex> lk(g_res_mu);
-    r->next = g_res_free;
-    g_res_free = r;
-}
-
 static int alloc_common(scp_gpu *h) {
     keep_pool(h->device);
     CK(cudaStreamCreateWithPriority(&h->stream, cudaStreamNonBlocking, t_stream_priority));
     CK(cudaMallocAsync(&h->part, sizeof(double) * kRedMaxBlocks * 32, h->stream));
     CK(cudaMallocAsync(&h->fold, sizeof(double) * DF_N, h->stream));
     CK(cudaMemsetAsync(h->fold, 0, sizeof(double) * DF_N, h->stream));
-    if (!(h->slot = result_slot())) return SCP_ENOMEM;
+    if (!(h->slot = g_slots.take(context_id()))) return SCP_ENOMEM;
     h->res = h->slot->p;
     CK(cudaMallocAsync(&h->cg, sizeof(double) * 16, h->stream));
     CK(cudaMallocAsync(&h->point, sizeof(double) * 8, h->stream));
@@ -1782,7 +1753,7 @@ void scp_gpu_free(scp_gpu *h) {
             if (b) cudaFreeAsync(b, h->stream);
         cudaStreamSynchronize(h->stream);
     }
-    if (h->slot) result_slot_free(h->slot);
+    if (h->slot) g_slots.give(h->slot, context_id());
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
     if (h->snap_ready) cudaEventDestroy(h->snap_ready);
