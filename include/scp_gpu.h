@@ -217,6 +217,13 @@ int  scp_gpu_abi_version(void);
  * difference of sin and cos in FP64 and of sin and cos in FP32.  Synchronous;
  * allocates and frees its own device buffers. */
 int  scp_gpu_check_trig(int n, const double *x, double *err);
+/* The batched sines and cosines the step kernels use, for the n host angles
+ * x[]: sn[] and, for the kinds that give them, cs[].  kind 0: FP64, sine and
+ * cosine of five angles at a time, |x| < 2^20; 1: the same for any x; 2: FP64,
+ * sine of seven, |x| < 2^20; 3 and 4: FP32 pairs (angles rounded to float),
+ * sine and cosine of five pairs, sine of seven pairs, |x| <= 2^12.  Consecutive
+ * angles share a batch.  Synchronous; allocates and frees its own device buffer. */
+int  scp_gpu_trig_batch(int kind, int n, const double *x, double *sn, double *cs);
 
 /* Diagnostics for callers that must not allocate device memory.
  *

@@ -27,6 +27,7 @@
 #include "launch.cuh"
 #include "plan.cuh"
 #include "tma.cuh"
+#include "vec2.cuh"
 #include "ext_launch.cuh"
 #include "ext_startup.cuh"
 
@@ -1823,6 +1824,68 @@ extern "C" int scp_gpu_check_trig(int n, const double *x, double *err) {
     if (e == cudaSuccess) e = cudaMemcpy(err, de, sizeof(double) * 4, cudaMemcpyDeviceToHost);
     cudaFree(dx);
     cudaFree(de);
+    CK(e);
+    return SCP_OK;
+}
+
+// One batch routine over consecutive groups of angles: sines to sn, cosines
+// (where the routine gives them) to cs.
+enum : int { TRIG_BATCH = 0, TRIG_BATCH_ANY, TRIG_SIN, TRIG_PAIR, TRIG_PAIR_SIN, TRIG_KINDS };
+__global__ void trig_batch_kernel(int kind, const double *x, int n, double *sn, double *cs) {
+    constexpr int NB = 5, NS = 7;   // as many as a site's link phases and plaquettes
+    const bool pair = kind == TRIG_PAIR || kind == TRIG_PAIR_SIN, sine = kind == TRIG_SIN || kind == TRIG_PAIR_SIN;
+    const int group = (sine ? NS : NB) * (pair ? 2 : 1);
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g * group < n; g += gridDim.x * blockDim.x) {
+        double a[2 * NS], s[2 * NS], c[2 * NS];
+        for (int i = 0; i < 2 * NS; i++) {
+            a[i] = i < group && g * group + i < n ? x[g * group + i] : 0.0;
+            c[i] = 0.0;
+        }
+        if (pair) {
+            V2 v[NS], vs[NB], vc[NB], v5[NB];
+            for (int i = 0; i < NS; i++) v[i] = V2((float)a[2 * i], (float)a[2 * i + 1]);
+            if (sine) {
+                sin2_batch(v);
+                for (int i = 0; i < NS; i++) { s[2 * i] = v[i].v.x; s[2 * i + 1] = v[i].v.y; }
+            } else {
+                for (int i = 0; i < NB; i++) v5[i] = v[i];
+                sincos2_batch(v5, vs, vc);
+                for (int i = 0; i < NB; i++) {
+                    s[2 * i] = vs[i].v.x; s[2 * i + 1] = vs[i].v.y;
+                    c[2 * i] = vc[i].v.x; c[2 * i + 1] = vc[i].v.y;
+                }
+            }
+        } else if (sine) {
+            double v[NS];
+            for (int i = 0; i < NS; i++) v[i] = a[i];
+            sin_batch(v);
+            for (int i = 0; i < NS; i++) s[i] = v[i];
+        } else {
+            double v[NB], vs[NB], vc[NB];
+            for (int i = 0; i < NB; i++) v[i] = a[i];
+            if (kind == TRIG_BATCH_ANY) sincos_batch<NB, true>(v, vs, vc);
+            else sincos_batch(v, vs, vc);
+            for (int i = 0; i < NB; i++) { s[i] = vs[i]; c[i] = vc[i]; }
+        }
+        for (int i = 0; i < group && g * group + i < n; i++) {
+            sn[g * group + i] = s[i];
+            cs[g * group + i] = c[i];
+        }
+    }
+}
+
+extern "C" int scp_gpu_trig_batch(int kind, int n, const double *x, double *sn, double *cs) {
+    if (kind < 0 || kind >= TRIG_KINDS || n < 1 || n > (1 << 28) || !x || !sn || !cs) return SCP_EINVAL;
+    double *d = nullptr;
+    CK(cudaMalloc(&d, sizeof(double) * 3 * n));
+    cudaError_t e = cudaMemcpy(d, x, sizeof(double) * n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        trig_batch_kernel<<<64, 128>>>(kind, d, n, d + n, d + 2 * (size_t)n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(sn, d + n, sizeof(double) * n, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(cs, d + 2 * (size_t)n, sizeof(double) * n, cudaMemcpyDeviceToHost);
+    cudaFree(d);
     CK(e);
     return SCP_OK;
 }

@@ -7,6 +7,9 @@
 // the quadrant k mod 4 applied by selects.  FP64: terms through r^17 / r^16
 // (truncation below 1e-17); FP32: through r^11 / r^10.  Valid for |x| up to
 // about 2^20; tests/test_gpu_trig.py checks the result against CUDA's sin/cos.
+// The FP64 step and the plane walkers take the batches further down, the FP32C
+// pairs those of vec2.cuh: tests/test_gpu_trig_batch.py checks each against
+// extended-precision values, tests/test_trig_polynomials.py the coefficients.
 #pragma once
 #include "common.cuh"
 

@@ -20,7 +20,7 @@ EXPORTS = (
     "scp_gpu_snapshot", "scp_gpu_snapshot_async", "scp_gpu_snapshot_wait", "scp_gpu_host_alloc",
     "scp_gpu_host_free", "scp_gpu_get_info", "scp_gpu_time_steps", "scp_gpu_stream",
     "scp_gpu_free", "scp_gpu_errstr", "scp_gpu_last_cuda_error", "scp_gpu_abi_version",
-    "scp_gpu_diag_noalloc", "scp_gpu_check_trig",
+    "scp_gpu_diag_noalloc", "scp_gpu_check_trig", "scp_gpu_trig_batch",
     "scp_srv_create", "scp_srv_submit", "scp_srv_submit_borrowed", "scp_srv_poll", "scp_srv_status", "scp_srv_result",
     "scp_srv_stats", "scp_srv_free",
 )
@@ -137,6 +137,7 @@ def lib() -> ctypes.CDLL:
     L.scp_gpu_errstr.restype = ctypes.c_char_p
     L.scp_gpu_last_cuda_error.restype = ctypes.c_char_p
     L.scp_gpu_check_trig.argtypes = [ctypes.c_int, vp, vp]
+    L.scp_gpu_trig_batch.argtypes = [ctypes.c_int, ctypes.c_int, vp, vp, vp]
     ip = ctypes.POINTER(ctypes.c_int)
     L.scp_srv_create.argtypes = [ctypes.POINTER(SrvConfig), ctypes.POINTER(vp)]
     L.scp_srv_submit.argtypes = [vp, ctypes.POINTER(CParams), ctypes.POINTER(vp), ctypes.c_int64,
