@@ -1,7 +1,7 @@
 // ext_startup.cuh -- start-up and diagnostic kernels of the extension
 // steppers (higgs_u1.cuh, fabrics.cuh): the Higgs start value and energy, the
 // second Gauss law and its projection, the fabrics' EM charge density, Gauss
-// residual, charges and the view of fabric L for the energy reductions.
+// residual and charges, and the real mode's energies.
 // Host translation unit scp_gpu.cu only (the step kernels live in
 // kern_higgs.cu, kern_fabric.cu and kern_real.cu).
 #pragma once
@@ -203,16 +203,6 @@ __global__ void __launch_bounds__(kRedThreads) fabric_diag_kernel(FabView f, int
     }
     block_fold<FS_NSUM, 1>(S, M, scratch, part);
 }
-
-// Fabric L seen through the diagnostics' state view: its 12 matter fields
-// with C's links and E (the reference's energy of L uses the unit-charge
-// links, compute_energy_complex_gauge :1977-2028)
-struct ViewFabric {
-    const double *XF, *PF, *XC, *PC;
-    long long N3;
-    __device__ __forceinline__ double q(int f, long long i) const { return f < 12 ? XF[f * N3 + i] : XC[f * N3 + i]; }
-    __device__ __forceinline__ double p(int f, long long i) const { return f < 12 ? PF[f * N3 + i] : PC[f * N3 + i]; }
-};
 
 // ---- real mode with the optional terms
 // Energy terms of the real mode (compute_energy with the optional terms) and

@@ -3,7 +3,9 @@
 // Every reduction in the library is two-level with a fixed shape: each CTA of
 // a fixed-size grid folds its grid-stride share of sites in a fixed order,
 // then a warp-shuffle tree and a fixed cross-warp order produce one partial
-// per CTA, and a single finishing CTA folds the partials in index order.  The
+// per CTA, and a single finishing CTA folds the partials in a fixed order: a
+// stride of 32 partials per lane and a shuffle tree (fold_partials_*), or a
+// stride per warp and the warps in order (fold_rows_block).  The
 // result is bitwise reproducible from run to run and independent of timing
 // (the reference GPU code uses atomicAdd on doubles, sfa/sim/scp_sim.cu:2051-2087,
 // whose summation order varies between runs).

@@ -148,7 +148,7 @@ struct scp_gpu {
     float *W32 = nullptr, *S32 = nullptr;
     void *slab32 = nullptr;
     // scratch
-    double *part = nullptr, *fold = nullptr, *cg = nullptr, *point = nullptr;
+    double *part = nullptr, *fold = nullptr, *cg = nullptr;
     int *flag = nullptr;
     unsigned *count = nullptr;   // last-CTA counter of the fused CG launches
     double h_small[64];          // host landing area of the small device-to-host reads
@@ -340,8 +340,8 @@ static bool encode_mom_map(const double *W, int N, int nf, int tx, int ty, CUten
 // tma (1: TMA tile loads of the positions) or cpm (2: the cp.async position
 // ring with TMA-staged momenta).  Both give the same bits as the default and
 // ran slower on B200 (0.233 and 0.271 against 0.198 ms per 128^3 gauged
-// step on 32 x 4 tiles): the step is bound by shared-memory traffic and FP64 dependency
-// chains, which the TMA forms do not shorten.
+// step on 32 x 4 tiles): the step is bound by DRAM (step.cuh), whose traffic they
+// do not cut, and they add shared-memory traffic of their own.
 static int staging_mode(const scp_gpu *h, int shape) {
     if (h->prec != SCP_PREC_FP64 || (shape != 1 && shape != 2)) return 0;
     const char *e = getenv("SCP_STAGING");
@@ -704,14 +704,13 @@ static int alloc_common(scp_gpu *h) {
     if (!(h->slot = g_slots.take(context_id()))) return SCP_ENOMEM;
     h->res = h->slot->p;
     CK(cudaMallocAsync(&h->cg, sizeof(double) * 16, h->stream));
-    CK(cudaMallocAsync(&h->point, sizeof(double) * 8, h->stream));
     CK(cudaMallocAsync(&h->flag, sizeof(int), h->stream));
     CK(cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream));
     CK(cudaMallocAsync(&h->count, sizeof(unsigned), h->stream));
     CK(cudaMemsetAsync(h->count, 0, sizeof(unsigned), h->stream));
     CK(cudaEventCreate(&h->ev0));
     CK(cudaEventCreate(&h->ev1));
-    h->dev_bytes += sizeof(double) * (kRedMaxBlocks * 32 + DF_N + 16 + 8);
+    h->dev_bytes += sizeof(double) * (kRedMaxBlocks * 32 + DF_N + 16);
     return SCP_OK;
 }
 
@@ -1748,7 +1747,7 @@ void scp_gpu_free(scp_gpu *h) {
     if (h->snap_pending) cudaEventSynchronize(h->snap_done);
     if (h->copy_stream) cudaStreamSynchronize(h->copy_stream);
     if (h->stream) {
-        void *bufs[] = {h->slab32, h->slab, h->part, h->fold, h->cg, h->point, h->flag, h->count, h->stage,
+        void *bufs[] = {h->slab32, h->slab, h->part, h->fold, h->cg, h->flag, h->count, h->stage,
                         h->snap_dev, h->kacc, h->dpart, h->drho};
         for (void *b : bufs)
             if (b) cudaFreeAsync(b, h->stream);

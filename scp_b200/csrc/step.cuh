@@ -18,9 +18,9 @@
 //     [v_{n+1} *= damp(r)]                    (reference stage 5, bc_type 0)
 //     w_{n+1} = v_{n+1} + hdt*a_{n+1}         (next step's stage-1 kick)
 //     x_{n+2} = x_{n+1} + dt*w_{n+1}          (next step's drift)
-// with the reference's arithmetic in the reference's order, so no
-// acceleration array exists and each state word is read once and written
-// once per step.  Links follow the same pattern with E and the wrapped drift
+// so no acceleration array exists and each state word is read once and written
+// once per step.  (The terms are the reference's; in FP64 they are summed field
+// by field, gauged.cuh, to roundoff of the reference's order.)  Links follow the same pattern with E and the wrapped drift
 // th += -g*dx*dt*E.  The launch that starts a run (FIRST) reads v_0 instead
 // of w and skips the stage-4 kick; a SYNC launch also stores v_{n+1} and
 // E_{n+1} for diagnostics and snapshots.
@@ -558,10 +558,8 @@ template <int TX, int TY, bool GAUGED, bool FIRST>
 __device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepConsts &c, const TileGrid &tg,
                                             const Piece &pc, const bool SYNC, const bool DAMP,
                                             CpStage<F32C, TX, TY, GAUGED> &stg) {
-    using P = F32C;
     using T = float;
-    using Stage = CpStage<F32C, TX, TY, GAUGED>;
-    using LY = StepLayout<P, TX, TY, GAUGED>;
+    using LY = StepLayout<F32C, TX, TY, GAUGED>;
     constexpr int NF = LY::NF;
     constexpr int NR = LY::NR;
     const int N = c.N;
@@ -592,14 +590,11 @@ __device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepCo
             const int sb = (b == 0) ? sp : sc, rb = r + (b == 1 ? 1 : 0), cb = col + (b == 2 ? 1 : 0);
             const T tay = XS(sc, FTH + a, r, col), tby = XS(sc, FTH + b, r, col);
             const T tbya = XS(sa, FTH + b, ra, ca), tayb = XS(sb, FTH + a, rb, cb);
-            if constexpr (NR > NF) {   // FP32C: hi differences plus lo differences
-                const T hi = (tay - tayb) + (tbya - tby);
-                const T lo = (XS(sc, NF + a, r, col) - XS(sb, NF + a, rb, cb)) +
-                             (XS(sa, NF + b, ra, ca) - XS(sc, NF + b, r, col));
-                return sin_bounded(hi + lo);
-            } else {
-                return sin_bounded(tay + tbya - tayb - tby);
-            }
+            // hi differences plus lo differences
+            const T hi = (tay - tayb) + (tbya - tby);
+            const T lo = (XS(sc, NF + a, r, col) - XS(sb, NF + a, rb, cb)) +
+                         (XS(sa, NF + b, ra, ca) - XS(sc, NF + b, r, col));
+            return sin_bounded(hi + lo);
         };
 
         __syncthreads();   // previous item finished reading the ring
@@ -619,24 +614,15 @@ __device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepCo
             P0m = plaq_sin(0, 0, 1, ty + 1, tx + 1);
             P2m = plaq_sin(2, 0, 1, ty + 1, tx + 1);
         }
-        // planes i0+1 .. i0+NS-2 (NS ring slots: NS-2 planes ahead in flight)
-        constexpr int NS = Stage::NSLOT;
-#pragma unroll
-        for (int q = 1; q <= NS - 2; q++)
-            if (i0 + q <= i1) issue_plane(i0 + q, q + 1);
-        if constexpr (Stage::MOM) stg.issue_mom(i0, 0);   // momenta of the first plane
+        issue_plane(i0 + 1, 2);
         stg.commit();
 
         for (int i = i0; i < i1; i++) {
-            // plane p sits in slot (p - i0 + 1) mod NS; plane i + NS - 1 reuses the slot of i - 1
-            const int sc = (i - i0 + 1) % NS, sp = (i - i0 + 2) % NS, sn = (i - i0) % NS;
-            stg.template wait<NS - 3>(sp);   // the copies of planes beyond i+1 may stay in flight
-            if constexpr (Stage::MOM) stg.wait_mom((i - i0) & 1);
+            // plane p sits in slot (p - i0 + 1) mod 3; plane i + 2 reuses the slot of i - 1
+            const int sc = (i - i0 + 1) % 3, sp = (i - i0 + 2) % 3, sn = (i - i0) % 3;
+            stg.template wait<0>(sp);
             __syncthreads();
-            if (i + NS - 1 <= i1) issue_plane(i + NS - 1, sn);
-            if constexpr (Stage::MOM) {   // momenta of the next plane, into the slot plane i-1 used
-                if (i + 1 < i1) stg.issue_mom(i + 1, (i + 1 - i0) & 1);
-            }
+            if (i + 2 <= i1) issue_plane(i + 2, sn);
             stg.commit();
             const long long site = (long long)i * N * N + oc;
             if (c.prefetch && act && i + 1 < i1) {
@@ -647,19 +633,12 @@ __device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepCo
             // (113^3 115 us a step against 119, 151^3 224 against 233), with
             // links where the compiler puts them (151^3 304 against 311)
             T w[NF];
-            uint16_t lo[P::COMP ? 12 : 1];
+            uint16_t lo[12];
             if (act) {
-                if constexpr (Stage::MOM) {
 #pragma unroll
-                    for (int f = 0; f < NF; f++) w[f] = stg.mom((i - i0) & 1, f);
-                } else {
+                for (int f = 0; f < NF; f++) w[f] = GAUGED ? io.win[f * N3 + site] : ld_early(io.win + f * N3 + site);
 #pragma unroll
-                    for (int f = 0; f < NF; f++) w[f] = GAUGED ? io.win[f * N3 + site] : ld_early(io.win + f * N3 + site);
-                }
-                if constexpr (P::COMP) {
-#pragma unroll
-                    for (int f = 0; f < 12; f++) lo[f] = GAUGED ? io.loin[f * N3 + site] : ld_early(io.loin + f * N3 + site);
-                }
+                for (int f = 0; f < 12; f++) lo[f] = GAUGED ? io.loin[f * N3 + site] : ld_early(io.loin + f * N3 + site);
             }
             if (!act) continue;
             T acc[12];
@@ -689,14 +668,10 @@ __device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepCo
                         default: return XS(sc, f, ty + 1, tx);
                     }
                 };
-                auto lap = [&](int f) -> T {
-                    if constexpr (P::COMP) {   // neighbour differences: no cancellation against 6*centre
-                        const T x0 = ctr[f];
-                        return ((nb(f, 0) - x0) + (nb(f, 1) - x0) + (nb(f, 2) - x0) + (nb(f, 3) - x0) +
-                                (nb(f, 4) - x0) + (nb(f, 5) - x0)) * idx2;
-                    } else {
-                        return (nb(f, 0) + nb(f, 1) + nb(f, 2) + nb(f, 3) + nb(f, 4) + nb(f, 5) - T(6) * ctr[f]) * idx2;
-                    }
+                auto lap = [&](int f) -> T {   // neighbour differences: no cancellation against 6*centre
+                    const T x0 = ctr[f];
+                    return ((nb(f, 0) - x0) + (nb(f, 1) - x0) + (nb(f, 2) - x0) + (nb(f, 3) - x0) +
+                            (nb(f, 4) - x0) + (nb(f, 5) - x0)) * idx2;
                 };
                 auto curl = [&](int g0, int a) -> T {
                     if (a == 0) return (nb(g0 + 2, 2) - nb(g0 + 2, 3) - nb(g0 + 1, 4) + nb(g0 + 1, 5)) * idx1;
@@ -752,14 +727,9 @@ __device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepCo
                         }
                         const T TRp = cP * up - sP * vp, TIp = cP * vp + sP * up;
                         const T TRm = cM * um + sM * vm, TIm = cM * vm - sM * um;
-                        if constexpr (P::COMP) {   // accumulate (transported - centre) differences
-                            const T cu = fu[q], cv = fv[q];
-                            if (d == 0) { lapU[q] = (TRp - cu) + (TRm - cu); lapV[q] = (TIp - cv) + (TIm - cv); }
-                            else { lapU[q] = lapU[q] + (TRp - cu) + (TRm - cu); lapV[q] = lapV[q] + (TIp - cv) + (TIm - cv); }
-                        } else {
-                            if (d == 0) { lapU[q] = TRp + TRm; lapV[q] = TIp + TIm; }
-                            else { lapU[q] = lapU[q] + TRp + TRm; lapV[q] = lapV[q] + TIp + TIm; }
-                        }
+                        const T cu = fu[q], cv = fv[q];   // (transported - centre) differences
+                        if (d == 0) { lapU[q] = (TRp - cu) + (TRm - cu); lapV[q] = (TIp - cv) + (TIm - cv); }
+                        else { lapU[q] = lapU[q] + (TRp - cu) + (TRm - cu); lapV[q] = lapV[q] + (TIp - cv) + (TIm - cv); }
                         const int qa = q < 3 ? q : q - 3;
                         if (qa != d) {
                             const T DR = (TRp - TRm) * idx1, DI = (TIp - TIm) * idx1;
@@ -784,15 +754,10 @@ __device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepCo
                     for (int a = 0; a < 3; a++) {
                         const T TIt = cP * tvp[a] + sP * tup[a];
                         const T TRt = cP * tup[a] - sP * tvp[a];
-                        if constexpr (P::COMP) {
-                            // u*TI - v*TR = u*(TI - v) - v*(TR - u): differences of neighbouring
-                            // values instead of a difference of two O(|f|^2) products
-                            Jg += fu[a] * (TIpP[a] - fv[a]) - fv[a] * (TRpP[a] - fu[a]);
-                            Jg += fu[3 + a] * (TIt - fv[3 + a]) - fv[3 + a] * (TRt - fu[3 + a]);
-                        } else {
-                            Jg += fu[a] * TIpP[a] - fv[a] * TRpP[a];
-                            Jg += fu[3 + a] * TIt - fv[3 + a] * TRt;
-                        }
+                        // u*TI - v*TR = u*(TI - v) - v*(TR - u): differences of neighbouring
+                        // values instead of a difference of two O(|f|^2) products
+                        Jg += fu[a] * (TIpP[a] - fv[a]) - fv[a] * (TRpP[a] - fu[a]);
+                        Jg += fu[3 + a] * (TIt - fv[3 + a]) - fv[3 + a] * (TRt - fu[3 + a]);
                     }
                     const int d1 = (d + 1) % 3, d2 = (d + 2) % 3;
                     const T WpR1 = cP * fu[d2] + sP * fv[d2], WpI1 = cP * fv[d2] - sP * fu[d2];
@@ -818,11 +783,8 @@ __device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepCo
                 K[2] = stp * st2 + gg * K[2];
 #pragma unroll
                 for (int a = 0; a < 3; a++) {
-                    const T c6 = P::COMP ? T(0) : T(6);   // FP32C accumulated differences already
-                    const T lUP = (lapU[a] - c6 * fu[a]) * idx2;
-                    const T lVP = (lapV[a] - c6 * fv[a]) * idx2;
-                    const T lUT = (lapU[3 + a] - c6 * fu[3 + a]) * idx2;
-                    const T lVT = (lapV[3 + a] - c6 * fv[3 + a]) * idx2;
+                    const T lUP = lapU[a] * idx2, lVP = lapV[a] * idx2;
+                    const T lUT = lapU[3 + a] * idx2, lVT = lapV[3 + a] * idx2;
                     acc[FU + a] = lUP - m2 * fu[a] - T(2) * Vp * fu[a] * rest[a] + eta * crT[a];
                     acc[FV + a] = lVP - m2 * fv[a] - T(2) * Vp * fv[a] * rest[a] + eta * ciT[a];
                     acc[FTU + a] = lUT - mt2 * fu[3 + a] + eta * crP[a];
@@ -846,22 +808,20 @@ __device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepCo
 #pragma unroll
             for (int f = 0; f < 12; f++) {
                 T v, wn, xn;
-                if constexpr (P::COMP) {
-                    // kicks with dt and dt/2 as fp32 pairs: the increment h*a is formed
-                    // first (hi*a + lo*a), then added to the momentum in one rounding --
-                    // folding lo*a into the momentum first would lose it below half an
-                    // ulp and run the kick with fp32(dt), a systematic energy drift
-                    const float ha = fmaf(hdt, acc[f], hdt_lo * acc[f]);
-                    v = FIRST ? w[f] : w[f] + ha;
-                    if (DAMP && !FIRST) v *= dmp;
-                    if (DAMP || FIRST) wn = v + ha;
-                    else wn = w[f] + fmaf((float)c.dt, acc[f], dt_lo * acc[f]);   // w_n + dt*a, no damping
-                    // compensated drift (hi, lo) += dt*w_{n+1}
-                    const float y = fmaf((float)c.dt, wn, fmaf(dt_lo, wn, bf16_to_f(lo[f])));
-                    float e;
-                    two_sum(ctr[f], y, &xn, &e);
-                    io.loout[f * N3 + site] = f_to_bf16(e);
-                }
+                // kicks with dt and dt/2 as fp32 pairs: the increment h*a is formed
+                // first (hi*a + lo*a), then added to the momentum in one rounding --
+                // folding lo*a into the momentum first would lose it below half an
+                // ulp and run the kick with fp32(dt), a systematic energy drift
+                const float ha = fmaf(hdt, acc[f], hdt_lo * acc[f]);
+                v = FIRST ? w[f] : w[f] + ha;
+                if (DAMP && !FIRST) v *= dmp;
+                if (DAMP || FIRST) wn = v + ha;
+                else wn = w[f] + fmaf((float)c.dt, acc[f], dt_lo * acc[f]);   // w_n + dt*a, no damping
+                // compensated drift (hi, lo) += dt*w_{n+1}
+                const float y = fmaf((float)c.dt, wn, fmaf(dt_lo, wn, bf16_to_f(lo[f])));
+                float e;
+                two_sum(ctr[f], y, &xn, &e);
+                io.loout[f * N3 + site] = f_to_bf16(e);
                 st_cs(io.xout + f * N3 + site, xn);
                 io.wout[f * N3 + site] = wn;
                 if (SYNC && !FIRST) {
@@ -874,25 +834,23 @@ __device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepCo
 #pragma unroll
                 for (int d = 0; d < 3; d++) {
                     T E, Eh, th;
-                    if constexpr (P::COMP) {
-                        const float hK = fmaf(hdt, K[d], hdt_lo * K[d]);
-                        E = FIRST ? w[FTH + d] : w[FTH + d] + hK;
-                        if (DAMP && !FIRST) E *= dmp;
-                        if (DAMP || FIRST) Eh = E + hK;
-                        else Eh = w[FTH + d] + fmaf((float)c.dt, K[d], dt_lo * K[d]);
-                        const float gad_lo = (float)(c.gad - (double)(float)c.gad);
-                        const float y = fmaf(gad, Eh, fmaf(gad_lo, Eh, XS(sc, NR - 3 + d, ty + 1, tx + 1)));
-                        float lnew;
-                        two_sum(ctr[FTH + d], y, &th, &lnew);
-                        if (fabsf(th) > 3.0f) {   // wrap by 2 pi, carried as an fp32 pair
-                            const float kq = rintf(th * 0.159154943091895336f);
-                            float t1, e1;
-                            two_sum(th, -kq * 6.28318548202514648f, &t1, &e1);   // 2 pi (fp32) times |kq| <= 1
-                            lnew = lnew + e1 + kq * 1.74845553e-7f;              // 2 pi = 6.2831855f - 1.748e-7
-                            two_sum(t1, lnew, &th, &lnew);
-                        }
-                        io.tloout[d * N3 + site] = lnew;
+                    const float hK = fmaf(hdt, K[d], hdt_lo * K[d]);
+                    E = FIRST ? w[FTH + d] : w[FTH + d] + hK;
+                    if (DAMP && !FIRST) E *= dmp;
+                    if (DAMP || FIRST) Eh = E + hK;
+                    else Eh = w[FTH + d] + fmaf((float)c.dt, K[d], dt_lo * K[d]);
+                    const float gad_lo = (float)(c.gad - (double)(float)c.gad);
+                    const float y = fmaf(gad, Eh, fmaf(gad_lo, Eh, XS(sc, NR - 3 + d, ty + 1, tx + 1)));
+                    float lnew;
+                    two_sum(ctr[FTH + d], y, &th, &lnew);
+                    if (fabsf(th) > 3.0f) {   // wrap by 2 pi, carried as an fp32 pair
+                        const float kq = rintf(th * 0.159154943091895336f);
+                        float t1, e1;
+                        two_sum(th, -kq * 6.28318548202514648f, &t1, &e1);   // 2 pi (fp32) times |kq| <= 1
+                        lnew = lnew + e1 + kq * 1.74845553e-7f;              // 2 pi = 6.2831855f - 1.748e-7
+                        two_sum(t1, lnew, &th, &lnew);
                     }
+                    io.tloout[d * N3 + site] = lnew;
                     st_cs(io.xout + (FTH + d) * N3 + site, th);
                     io.wout[(FTH + d) * N3 + site] = Eh;
                     if (SYNC && !FIRST) {

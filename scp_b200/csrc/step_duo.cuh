@@ -18,8 +18,11 @@
 // plane, with a barrier over the two warps of one tile row (TX = 32: a warp
 // is a row).  Both threads evaluate the link cos/sin they transport with.
 //
-// Arithmetic is that of step_item's gauged F64 branch term by term; the
-// current J_d is summed in the same order (Phi_0, Theta_0, Phi_1, ...).
+// Arithmetic: the reference's terms direction by direction, the current J_d
+// summed as the reference visits it (Phi_0, Theta_0, Phi_1, ...), one-angle
+// sines, and the compiler's choice of fused operations.  The one-thread step
+// goes field by field in explicitly rounded operations, so the two agree to
+// roundoff (1e-11 after the tests' runs), not to the bit.
 // Staging, work plan and the fused leapfrog scheme are those of step.cuh.
 #pragma once
 #include "step.cuh"
