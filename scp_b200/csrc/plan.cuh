@@ -8,9 +8,12 @@ namespace scp {
 // Launch a step kernel of a grid of edge N; up to 112^3 as a programmatic
 // dependent of the launch before it on the stream: its CTAs take free slots and
 // set up while that launch drains, which hides the launch gap (gauged 32^3 6.7
-// against 8.2 us a step, 64^3 27.0 against 28.7, FP32C 95^3 77.5 against 79.9).
-// Larger grids fill every slot themselves and lose by it (128^3 181.0 against
-// 179.1 us, 256^3 1.40 against 1.39 ms).
+// against 8.2 us a step).  Never slower up to there on any stepper: gauged 5 %
+// at 64^3, 1 % at 96^3 and 112^3; without links 14, 2 and 2; FP32C 12 to 17, 3
+// to 4 and 2 to 4; Higgs and second gauge 5, 2 and 1; three fabrics 7, 2 and 1;
+// real mode with its terms 10, 3 and 3.  From 128^3 it depends on the stepper:
+// FP64 with links, without, and three fabrics lose 1 %, FP32C and the real mode
+// gain 1 to 2.
 constexpr int kDependentMaxN = 112;
 template <class... P, class... A>
 inline cudaError_t launch_step_kernel(void (*fn)(P...), int N, int grid, int threads, size_t smem, cudaStream_t st,

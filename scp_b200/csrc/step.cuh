@@ -629,16 +629,18 @@ __device__ __forceinline__ void step_item_c(const StepIO<F32C> &io, const StepCo
 #pragma unroll
                 for (int f = 0; f < NF; f++) prefetch_line_l2(io.win + f * N3 + site + (long long)N * N);
             }
-            // momenta and low parts of this plane; without links kept at the top
-            // (113^3 115 us a step against 119, 151^3 224 against 233), with
-            // links where the compiler puts them (151^3 304 against 311)
+            // momenta and low parts of this plane, kept at its top: where the
+            // compiler may place them it sinks some to their use (without links
+            // 113^3 119 us a step against 115, 151^3 233 against 224; with links
+            // 95^3 82.6 against 79.1, 111^3 156 against 147; only 97^3, 105
+            // against 109, and 127^3, 198 against 199, are the better for it)
             T w[NF];
             uint16_t lo[12];
             if (act) {
 #pragma unroll
-                for (int f = 0; f < NF; f++) w[f] = GAUGED ? io.win[f * N3 + site] : ld_early(io.win + f * N3 + site);
+                for (int f = 0; f < NF; f++) w[f] = ld_early(io.win + f * N3 + site);
 #pragma unroll
-                for (int f = 0; f < 12; f++) lo[f] = GAUGED ? io.loin[f * N3 + site] : ld_early(io.loin + f * N3 + site);
+                for (int f = 0; f < 12; f++) lo[f] = ld_early(io.loin + f * N3 + site);
             }
             if (!act) continue;
             T acc[12];
