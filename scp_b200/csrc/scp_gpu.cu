@@ -543,9 +543,13 @@ static int cg_solve(scp_gpu *h, int nb, double *b, double *x, double *r, double 
         // explicit residual of that chi restarts the iteration
         const int N = h->N, nc = spectral_ctas(N);
         const size_t sm = spectral_smem_bytes(N);
+        // the limit belongs to the kernel, not to this call: always the largest
+        // grid's, or a thread starting a smaller grid would lower it between
+        // another's setting and its launches
         CK(cudaFuncSetAttribute(is_pow2(N) ? (const void *)spectral_pass_kernel<true>
                                            : (const void *)spectral_pass_kernel<false>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)spectral_smem_bytes(is_pow2(N) ? kFftMaxN : kDftMaxN)));
         const double *in_re[5] = {b, r, r, r, r};
         const double *in_im[5] = {nullptr, p, p, p, p};
         double *out_re[5] = {r, r, r, r, x};
