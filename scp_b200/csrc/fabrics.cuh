@@ -22,8 +22,8 @@
 // is not locked.
 //
 // What bounds it: DRAM, 936 B per site with Q locked (432 for C, 504 for L
-// with the links) against 864 that no split can avoid; 370 us a step at 128^3
-// (0.76 of a plain copy's rate on the 864 B) against 524 with four resident
+// with the links) against 864 that no split can avoid; 363 us a step at 128^3
+// (0.77 of a plain copy's rate on the 864 B) against 524 with four resident
 // planes, momenta loaded at their own plane and a launch of its own for the
 // links.
 #pragma once
